@@ -113,6 +113,7 @@ extern "C" void psg_destroy(psg_context *ctx) {
 	free_tree(ctx);
 	if (ctx->d_ar) cudaFree(ctx->d_ar);
 	if (ctx->d_ar_ni) cudaFree(ctx->d_ar_ni);
+	if (ctx->d_ar_he) cudaFree(ctx->d_ar_he);
 	if (ctx->d_xs) cudaFree(ctx->d_xs);
 	if (ctx->d_kernel) cudaFree(ctx->d_kernel);
 	if (ctx->d_status) cudaFree(ctx->d_status);
@@ -258,12 +259,12 @@ extern "C" int psg_set_physics(psg_context *ctx, const psg_units *u, const psg_r
 	PSG_CUDA(cudaSetDevice(ctx->device));
 	if (ctx->d_ar) cudaFree(ctx->d_ar);
 	if (ctx->d_ar_ni) cudaFree(ctx->d_ar_ni);
-	if (ctx->d_ar_all) cudaFree(ctx->d_ar_all);
+	if (ctx->d_ar_he) cudaFree(ctx->d_ar_he);
 	if (ctx->d_xs) cudaFree(ctx->d_xs);
 	if (ctx->d_kernel) cudaFree(ctx->d_kernel);
 	ctx->d_ar = ctx->d_xs = ctx->d_kernel = nullptr;
 	ctx->d_ar_ni = nullptr;
-	ctx->d_ar_all = nullptr;
+	ctx->d_ar_he = nullptr;
 	// rows of 16 doubles (one 128-byte line): log T, then the 15 rate columns
 	const size_t nr = (size_t)ar->nrows;
 	static_assert(PSG_AR_NCOLS + 1 == 16, "one rate row is one 128-byte line");
@@ -311,25 +312,32 @@ extern "C" int psg_set_physics(psg_context *ctx, const psg_units *u, const psg_r
 		free(ni);
 		PSG_CUDA(e2);
 	}
-	// The helium right-hand side reads up to 15 columns: the same FP32 value
-	// and slope form, a (value, slope) pair per column, one 128-byte row.
+	// The helium right-hand side's columns in the same FP32 value and slope
+	// form: a (value, slope) pair per column, so a 16-byte load brings two
+	// columns and the 11 of case B take six loads (a 128-byte row).
 	{
-		float *all = (float *)calloc(nr * 32, sizeof(float));
-		if (!all) return psg_fail(ctx, PSG_E_NOMEM, "psg_set_physics: host allocation failed");
-		for (int c = 0; c < PSG_AR_NCOLS; c++) {
+		const bool ots = flags->on_the_spot != 0;
+		const int cols[PSG_HE_NCOLS] = {PSG_AR_HI_CI, ots ? PSG_AR_HII_RC_B : PSG_AR_HII_RC_A, PSG_AR_HEI_CI,
+				ots ? PSG_AR_HEII_RC_B : PSG_AR_HEII_RC_A, PSG_AR_HEII_CI, ots ? PSG_AR_HEIII_RC_B : PSG_AR_HEIII_RC_A,
+				ots ? PSG_AR_HII_RCC_B : PSG_AR_HII_RCC_A, PSG_AR_E_BREMC, PSG_AR_HI_CIC, PSG_AR_HI_CEC,
+				PSG_AR_E_COMPC, PSG_AR_HII_RC_B, PSG_AR_HEII_RC_B, PSG_AR_HEIII_RC_B};
+		float *he = (float *)calloc(nr * 32, sizeof(float));
+		if (!he) return psg_fail(ctx, PSG_E_NOMEM, "psg_set_physics: host allocation failed");
+		for (int c = 0; c < PSG_HE_NCOLS; c++) {
+			const double *col = ar->col[cols[c]];
 			double m = 0.0;
-			for (size_t j = 0; j < nr; j++) m = fmax(m, fabs(ar->col[c][j]));
-			ctx->ar_all_scale[c] = m > 0.0 ? m : 1.0;
+			for (size_t j = 0; j < nr; j++) m = fmax(m, fabs(col[j]));
+			ctx->ar_he_scale[c] = m > 0.0 ? m : 1.0;
 			for (size_t j = 0; j < nr; j++) {
-				const double v = ar->col[c][j] / ctx->ar_all_scale[c];
-				const double s = j + 1 < nr ? (ar->col[c][j + 1] / ctx->ar_all_scale[c] - v) * ar->step_inv : 0.0;
-				all[32 * j + 2 * c] = (float)v;
-				all[32 * j + 2 * c + 1] = (float)s;
+				const double v = col[j] / ctx->ar_he_scale[c];
+				const double s = j + 1 < nr ? (col[j + 1] / ctx->ar_he_scale[c] - v) * ar->step_inv : 0.0;
+				he[32 * j + 2 * c] = (float)v;
+				he[32 * j + 2 * c + 1] = (float)s;
 			}
 		}
-		cudaError_t e4 = cudaMalloc(&ctx->d_ar_all, sizeof(float) * nr * 32);
-		if (e4 == cudaSuccess) e4 = cudaMemcpy(ctx->d_ar_all, all, sizeof(float) * nr * 32, cudaMemcpyHostToDevice);
-		free(all);
+		cudaError_t e4 = cudaMalloc(&ctx->d_ar_he, sizeof(float) * nr * 32);
+		if (e4 == cudaSuccess) e4 = cudaMemcpy(ctx->d_ar_he, he, sizeof(float) * nr * 32, cudaMemcpyHostToDevice);
+		free(he);
 		PSG_CUDA(e4);
 	}
 	const size_t nx = (size_t)xs->nrows;

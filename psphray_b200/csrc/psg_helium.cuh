@@ -60,87 +60,95 @@ __device__ __forceinline__ double ye_he(const PhysParams &P, double lamH, double
 	return (1.0 - lamH) + P.hemf / P.hmf * 0.25 * (l2 + 2 * (1.0 - l2 - l1));
 }
 
-// The rate columns at one log T from the FP32 (value, slope) rows (each
-// column scaled by its largest magnitude): the two-point line of
-// tabfun_get() tabfun.c:38-58 written as value + slope * offset; a column
-// is one 8-byte load.
-struct RateRow {
-	const float2 *row;
-	double du;
-	const double *scale;
-	__device__ __forceinline__ double operator()(int c) const {
-		const float2 vs = row[c];
-		return __fma_rn((double)vs.y, du, (double)vs.x) * scale[c];
-	}
-};
-
-__device__ __forceinline__ RateRow rate_row(const PhysParams &P, double logT) {
-	long long idx = (long long)((logT - P.ar_min) * P.ar_step_inv);
-	RateRow R;
-	if (idx < 0) {
-		idx = 0;
-		R.du = 0.0;
-	} else if (idx >= P.ar_nrows - 1) {
-		idx = P.ar_nrows - 1;
-		R.du = 0.0;
-	} else {
-		R.du = logT - __fma_rn((double)idx, P.ar_step, P.ar_min);
-	}
-	R.row = P.ar_all + 16 * idx;
-	R.scale = P.ar_all_scale;
-	return R;
-}
-
 // One helium step: the Step fields the right-hand side reads.
 struct HeStep {
 	double yeMET, gHI, gHeI, gHeII, heat, time, nH, T;
 };
+
+// What the right-hand side needs of it, with what does not change along the
+// step taken out of it (the divisions by the step length).
+struct HeCtx {
+	double yeMET, g0, g1, g2, heat, nH, t, T;      // g, heat: per unit time, the photons negative
+};
+
+__device__ __forceinline__ HeCtx make_he_ctx(const HeStep &s) {
+	HeCtx c;
+	c.yeMET = s.yeMET;
+	c.g0 = -s.gHI / s.time;
+	c.g1 = -s.gHeI / s.time;
+	c.g2 = -s.gHeII / s.time;
+	c.heat = s.heat / s.time;
+	c.nH = s.nH;
+	c.t = s.time;
+	c.T = s.T;
+	return c;
+}
+
+// x / 3 correctly rounded (Markstein's theorem: the quotient by the rounded
+// reciprocal, corrected once by its exact remainder).
+__device__ __forceinline__ double div3(double x) {
+	const double y = 1.0 / 3.0, q = x * y;
+	return __fma_rn(__fma_rn(-3.0, q, x), y, q);
+}
 
 // function() solve.c:76-141 with helium (the rates of FETCH_VARS
 // solve.c:42-73); x = (lambdaH, lambdaHeI, lambdaHeII, ie), the derivative
 // per unit normalised time. On the spot (case B) the helium equations use
 // x_HI where solve.c:94-95 writes it; not on the spot (case A) rec[3]
 // receives the recombination photons' rates d(yGrecHII, yGrecHeII,
-// yGrecHeIII)/ds of solve.c:84-91.
-__device__ inline void rhs_he(const PhysParams &P, const HeStep &s, const double x[4], double dx[4],
+// yGrecHeIII)/ds of solve.c:84-91. The products and sums are those of
+// solve.c, each rounded; the rates come two columns to a 16-byte load from
+// the row of tabfun_get() tabfun.c:38-58 (clamped rows, a NaN temperature
+// included: offset 0), FP32 value + slope * offset in FP64.
+__device__ __forceinline__ void rhs_he(const PhysParams &P, const HeCtx &c, const double x[4], double dx[4],
 		double *rec = nullptr) {
 	const double xHI = x[0], xHII = 1.0 - x[0], xHeII = x[2];
 	const double xHeIII = 1.0 - x[2] - x[1];
-	const double ye = (xHII + P.hemf / P.hmf * 0.25 * (xHeII + 2 * xHeIII)) + s.yeMET;
-	const double T = P.isothermal ? s.T : ieye2T(P, x[3], ye);
-	const RateRow R = rate_row(P, log10(T));
-	const double nH = s.nH, t = s.time;
-	const double gamma_HI = R(PSG_AR_HI_CI) * nH;
-	const double gamma_HeI = R(PSG_AR_HEI_CI) * nH;
-	const double gamma_HeII = R(PSG_AR_HEII_CI) * nH;
-	const double aHII_B = R(PSG_AR_HII_RC_B) * nH, aHeII_B = R(PSG_AR_HEII_RC_B) * nH;
-	const double aHeIII_B = R(PSG_AR_HEIII_RC_B) * nH;
-	if (P.on_the_spot) {
-		dx[0] = (-s.gHI / t + (-gamma_HI * ye * xHI + aHII_B * ye * xHII)) * t;
-		dx[1] = (-s.gHeI / t + (-gamma_HeI * ye * xHI + aHeII_B * ye * xHeII)) * t;
-		dx[2] = (-s.gHeII / t + (-gamma_HeII * ye * xHI - aHeII_B * ye * xHeII + aHeIII_B * ye * xHeIII)) * t;
-	} else {
-		const double xHeI = x[1];
-		const double aHII_A = R(PSG_AR_HII_RC_A) * nH, aHeII_A = R(PSG_AR_HEII_RC_A) * nH;
-		const double aHeIII_A = R(PSG_AR_HEIII_RC_A) * nH;
-		dx[0] = (-s.gHI / t + (-gamma_HI * ye * xHI + aHII_A * ye * xHII)) * t;
-		dx[1] = (-s.gHeI / t + (-gamma_HeI * ye * xHeI + aHeII_A * ye * xHeII)) * t;
-		dx[2] = (-s.gHeII / t + (-gamma_HeII * ye * xHeII - aHeII_A * ye * xHeII + aHeIII_A * ye * xHeIII)) * t;
-		if (rec) {
-			rec[0] = fdim(aHII_A, aHII_B) * ye * xHII * t;
-			rec[1] = fdim(aHeII_A, aHeII_B) * ye * xHeII * t;
-			rec[2] = fdim(aHeIII_A, aHeIII_B) * ye * xHeIII * t;
+	const double ye = (xHII + P.he_f * (xHeII + 2 * xHeIII)) + c.yeMET;
+	const double T = P.isothermal ? c.T
+			: div3(rn_dmul(__ddiv_rn(rn_dmul(P.MPROTON_OVER_BOLTZMANN, x[3]), rn_dadd(P.T_den0, rn_dmul(P.hmf, ye))), 2.0));
+	const double logT = log10(T);
+	const double u = (logT - P.ar_min) * P.ar_step_inv;
+	int idx = 0;
+	double du = 0.0;
+	if (u > -1.0) {
+		idx = P.ar_nrows - 1;
+		if (u < (double)(P.ar_nrows - 1)) {
+			idx = (int)u;
+			du = logT - __fma_rn((double)idx, P.ar_step, P.ar_min);
 		}
+	}
+	const float4 *row = P.ar_he + 8 * (size_t)idx;
+	const float4 q0 = row[0], q1 = row[1], q2 = row[2];
+#define PSG_RATE(v, s, col) (__fma_rn((double)(s), du, (double)(v)) * P.ar_he_scale[col])
+	const double nH = c.nH, t = c.t;
+	const double ci0 = PSG_RATE(q0.x, q0.y, PSG_HE_CI0) * nH, rc0 = PSG_RATE(q0.z, q0.w, PSG_HE_RC0) * nH;
+	const double ci1 = PSG_RATE(q1.x, q1.y, PSG_HE_CI1) * nH, rc1 = PSG_RATE(q1.z, q1.w, PSG_HE_RC1) * nH;
+	const double ci2 = PSG_RATE(q2.x, q2.y, PSG_HE_CI2) * nH, rc2 = PSG_RATE(q2.z, q2.w, PSG_HE_RC2) * nH;
+	const bool ots = P.on_the_spot;
+	const double i1 = ots ? xHI : x[1], i2 = ots ? xHI : xHeII;      // what ionisation multiplies
+	dx[0] = (c.g0 + (-ci0 * ye * xHI + rc0 * ye * xHII)) * t;
+	dx[1] = (c.g1 + (-ci1 * ye * i1 + rc1 * ye * xHeII)) * t;
+	dx[2] = (c.g2 + (-ci2 * ye * i2 - rc1 * ye * xHeII + rc2 * ye * xHeIII)) * t;
+	if (!ots && rec) {
+		const float4 q5 = row[5], q6 = row[6];
+		const double b0 = PSG_RATE(q5.z, q5.w, PSG_HE_RCB0) * nH, b1 = PSG_RATE(q6.x, q6.y, PSG_HE_RCB1) * nH;
+		const double b2 = PSG_RATE(q6.z, q6.w, PSG_HE_RCB2) * nH;
+		rec[0] = fdim(rc0, b0) * ye * xHII * t;
+		rec[1] = fdim(rc1, b1) * ye * xHeII * t;
+		rec[2] = fdim(rc2, b2) * ye * xHeIII * t;
 	}
 	if (P.isothermal || P.adiabatic) {
 		dx[3] = 0.0;
 	} else {
-		const double eta = R(P.on_the_spot ? PSG_AR_HII_RCC_B : PSG_AR_HII_RCC_A) * nH;
-		const double psi = R(PSG_AR_HI_CEC) * nH, zeta = R(PSG_AR_HI_CIC) * nH;
-		const double beta = R(PSG_AR_E_BREMC) * nH, chi = R(PSG_AR_E_COMPC);
+		const float4 q3 = row[3], q4 = row[4], q5 = row[5];
+		const double eta = PSG_RATE(q3.x, q3.y, PSG_HE_RCC) * nH, beta = PSG_RATE(q3.z, q3.w, PSG_HE_BREM) * nH;
+		const double zeta = PSG_RATE(q4.x, q4.y, PSG_HE_CIC) * nH, psi = PSG_RATE(q4.z, q4.w, PSG_HE_CEC) * nH;
+		const double chi = PSG_RATE(q5.x, q5.y, PSG_HE_COMP);
 		const double L = P.H_PER_MASS * ((zeta + psi) * ye * xHI + (eta * ye * xHII) + beta * ye * xHII + chi * ye);
-		dx[3] = (s.heat / t - L) * t;
+		dx[3] = (c.heat - L) * t;
 	}
+#undef PSG_RATE
 }
 
 #define HE_SWITCH 32
@@ -155,106 +163,200 @@ __device__ __forceinline__ double he_err_norm(const double e[4], const double x[
 	return sqrt(0.25 * err);
 }
 
-// Rosenbrock ode23s over the four variables from (t, x) with step h. With
-// rec (not on the spot) the three recombination-photon counts are carried
-// as extra components whose Jacobian columns are zero: W's extra rows add
+// Rosenbrock ode23s over the four variables, a step at a time. With QUAD
+// four neighbouring lanes hold the same integration and evaluate a column of
+// the Jacobian each (a forward difference), the rest alike: a step is then
+// three right-hand sides long instead of six. The loops over W are unrolled
+// and its row swaps selected, so that it stays in registers. Not on the spot
+// (REC) the three recombination-photon counts are carried as extra
+// components whose Jacobian columns are zero: W's extra rows add
 // h*d*(J_r . k) to their stage values; they stay out of the error norm.
-__device__ inline bool rosenbrock_he(const PhysParams &P, const HeStep &s, double x[4], double t, double h,
-		int max_steps, double *rec = nullptr) {
-	const double d = 1.0 / (2.0 + 1.4142135623730951), e32 = 6.0 + 1.4142135623730951;
-	const double atol3 = DP_ATOL1_REL * fabs(x[3]) + 1e-300;
-	double F0[4], R0[3] = {0.0, 0.0, 0.0};
-	rhs_he(P, s, x, F0, rec ? R0 : nullptr);
-	h = fmin(fmax(h, 1e-10), 1.0);
-	for (int it = 0; it < max_steps; it++) {
-		if (t >= 1.0) return true;
-		if (t + h > 1.0) h = 1.0 - t;
-		double W[4][4], JR[3][4];
-		for (int j = 0; j < 4; j++) {
-			const double del = 1e-7 * fmax(fabs(x[j]), (j < 3 ? DP_ATOL0 : atol3) / RB_RTOL);
-			double y[4] = {x[0], x[1], x[2], x[3]}, Fj[4], Rj[3] = {0.0, 0.0, 0.0};
-			y[j] += del;
-			rhs_he(P, s, y, Fj, rec ? Rj : nullptr);
-			for (int i = 0; i < 4; i++) W[i][j] = (i == j ? 1.0 : 0.0) - h * d * (Fj[i] - F0[i]) / del;
-			for (int i = 0; i < 3; i++) JR[i][j] = (Rj[i] - R0[i]) / del;
-		}
-		// LU with partial pivoting, in place
-		int piv[4];
-		bool sing = false;
-		for (int k = 0; k < 4; k++) {
-			int m = k;
-			for (int i = k + 1; i < 4; i++)
-				if (fabs(W[i][k]) > fabs(W[m][k])) m = i;
-			piv[k] = m;
-			if (m != k)
-				for (int j = 0; j < 4; j++) {
-					const double tmp = W[k][j];
-					W[k][j] = W[m][j];
-					W[m][j] = tmp;
-				}
-			if (W[k][k] == 0.0) {
-				sing = true;
-				break;
-			}
-			for (int i = k + 1; i < 4; i++) {
-				W[i][k] /= W[k][k];
-				for (int j = k + 1; j < 4; j++) W[i][j] -= W[i][k] * W[k][j];
-			}
-		}
-		if (sing) return false;
-		auto solve = [&](const double b[4], double out[4]) {
-			double v[4] = {b[0], b[1], b[2], b[3]};
-			for (int k = 0; k < 4; k++) {
-				const double tmp = v[k];
-				v[k] = v[piv[k]];
-				v[piv[k]] = tmp;
-			}
-			for (int i = 1; i < 4; i++)
-				for (int j = 0; j < i; j++) v[i] -= W[i][j] * v[j];
-			for (int i = 3; i >= 0; i--) {
-				for (int j = i + 1; j < 4; j++) v[i] -= W[i][j] * v[j];
-				v[i] /= W[i][i];
-			}
-			for (int i = 0; i < 4; i++) out[i] = v[i];
-		};
-		double k1[4], k2[4], k3[4], F1[4], F2[4], y[4], yn[4], b[4], e[4];
-		double R1[3] = {0.0, 0.0, 0.0}, R2[3] = {0.0, 0.0, 0.0}, kr1[3], kr2[3];
-		solve(F0, k1);
-		for (int i = 0; i < 3; i++)
-			kr1[i] = R0[i] + h * d * (JR[i][0] * k1[0] + JR[i][1] * k1[1] + JR[i][2] * k1[2] + JR[i][3] * k1[3]);
-		for (int i = 0; i < 4; i++) y[i] = x[i] + 0.5 * h * k1[i];
-		rhs_he(P, s, y, F1, rec ? R1 : nullptr);
-		for (int i = 0; i < 4; i++) b[i] = F1[i] - k1[i];
-		solve(b, k2);
-		for (int i = 0; i < 3; i++)
-			kr2[i] = (R1[i] - kr1[i]) + h * d * (JR[i][0] * k2[0] + JR[i][1] * k2[1] + JR[i][2] * k2[2] +
-					JR[i][3] * k2[3]) + kr1[i];
-		for (int i = 0; i < 4; i++) {
-			k2[i] += k1[i];
-			yn[i] = x[i] + h * k2[i];
-		}
-		rhs_he(P, s, yn, F2, rec ? R2 : nullptr);
-		for (int i = 0; i < 4; i++) b[i] = F2[i] - e32 * (k2[i] - F1[i]) - 2.0 * (k1[i] - F0[i]);
-		solve(b, k3);
-		for (int i = 0; i < 4; i++) e[i] = h / 6.0 * (k1[i] - 2.0 * k2[i] + k3[i]);
-		const double err = he_err_norm(e, x, yn, atol3, RB_RTOL);
-		if (err <= 1.0 && isfinite(err)) {
-			t += h;
-			for (int i = 0; i < 4; i++) {
-				x[i] = yn[i];
-				F0[i] = F2[i];
-			}
-			if (rec)
-				for (int i = 0; i < 3; i++) {
-					rec[i] += h * kr2[i];
-					R0[i] = R2[i];
-				}
-		}
-		const double fac = (err > 0.0 && isfinite(err)) ? fmin(5.0, fmax(0.2, 0.9 * pow(err, -1.0 / 3.0)))
-				: (isfinite(err) ? 5.0 : 0.2);
-		h = fmax(h * fac, 1e-14);
+struct HeRbState {
+	double x[4], F0[4], t, h, atol3;
+	double rec[3], R0[3];
+};
+
+template <bool REC>
+__device__ __forceinline__ void he_rb_init(const PhysParams &P, const HeCtx &c, HeRbState &S, const double x[4],
+		double t, double h, const double *rec) {
+#pragma unroll
+	for (int i = 0; i < 4; i++) S.x[i] = x[i];
+	S.t = t;
+	S.h = fmin(fmax(h, 1e-10), 1.0);
+	S.atol3 = DP_ATOL1_REL * fabs(x[3]) + 1e-300;
+#pragma unroll
+	for (int i = 0; i < 3; i++) {
+		S.rec[i] = REC ? rec[i] : 0.0;
+		S.R0[i] = 0.0;
 	}
-	return t >= 1.0;
+	rhs_he(P, c, S.x, S.F0, REC ? S.R0 : nullptr);
+}
+
+// One attempted step from S.t < 1: 1 once s = 1 is reached, 0 before, -1
+// where W is singular. mask: the lanes that call (whole groups of four).
+template <bool REC, bool QUAD>
+__device__ __forceinline__ int he_rb_step(const PhysParams &P, const HeCtx &c, HeRbState &S, unsigned mask = 0) {
+	const double d = 1.0 / (2.0 + 1.4142135623730951), e32 = 6.0 + 1.4142135623730951;
+	double h = S.h;
+	if (S.t + h > 1.0) h = 1.0 - S.t;
+	double W[4][4], JR[3][4];
+	if (QUAD) {
+		const int q = threadIdx.x & 3;
+		double y[4], Fj[4], Rj[3] = {0.0, 0.0, 0.0}, wcol[4], jcol[3], del = 0.0;
+#pragma unroll
+		for (int j = 0; j < 4; j++) {
+			const double dj = 1e-7 * fmax(fabs(S.x[j]), (j < 3 ? DP_ATOL0 : S.atol3) / RB_RTOL);
+			y[j] = j == q ? S.x[j] + dj : S.x[j];
+			del = j == q ? dj : del;
+		}
+		rhs_he(P, c, y, Fj, REC ? Rj : nullptr);
+#pragma unroll
+		for (int i = 0; i < 4; i++) wcol[i] = (i == q ? 1.0 : 0.0) - h * d * (Fj[i] - S.F0[i]) / del;
+		if (REC)
+#pragma unroll
+			for (int i = 0; i < 3; i++) jcol[i] = (Rj[i] - S.R0[i]) / del;
+#pragma unroll
+		for (int j = 0; j < 4; j++) {
+			const int src = (threadIdx.x & 28) + j;
+#pragma unroll
+			for (int i = 0; i < 4; i++) W[i][j] = __shfl_sync(mask, wcol[i], src);
+			if (REC)
+#pragma unroll
+				for (int i = 0; i < 3; i++) JR[i][j] = __shfl_sync(mask, jcol[i], src);
+		}
+	} else {
+#pragma unroll
+		for (int j = 0; j < 4; j++) {
+			const double del = 1e-7 * fmax(fabs(S.x[j]), (j < 3 ? DP_ATOL0 : S.atol3) / RB_RTOL);
+			double y[4] = {S.x[0], S.x[1], S.x[2], S.x[3]}, Fj[4], Rj[3] = {0.0, 0.0, 0.0};
+			y[j] += del;
+			rhs_he(P, c, y, Fj, REC ? Rj : nullptr);
+#pragma unroll
+			for (int i = 0; i < 4; i++) W[i][j] = (i == j ? 1.0 : 0.0) - h * d * (Fj[i] - S.F0[i]) / del;
+			if (REC)
+#pragma unroll
+				for (int i = 0; i < 3; i++) JR[i][j] = (Rj[i] - S.R0[i]) / del;
+		}
+	}
+	// LU with partial pivoting, in place
+	int piv[4];
+	bool sing = false;
+#pragma unroll
+	for (int k = 0; k < 4; k++) {
+		int m = k;
+		double best = fabs(W[k][k]);
+#pragma unroll
+		for (int i = k + 1; i < 4; i++) {
+			const bool up = fabs(W[i][k]) > best;
+			m = up ? i : m;
+			best = up ? fabs(W[i][k]) : best;
+		}
+		piv[k] = m;
+#pragma unroll
+		for (int i = k + 1; i < 4; i++) {
+			const bool sw = m == i;
+#pragma unroll
+			for (int j = 0; j < 4; j++) {
+				const double a = W[k][j], b = W[i][j];
+				W[k][j] = sw ? b : a;
+				W[i][j] = sw ? a : b;
+			}
+		}
+		sing = sing || W[k][k] == 0.0;
+#pragma unroll
+		for (int i = k + 1; i < 4; i++) {
+			W[i][k] /= W[k][k];
+#pragma unroll
+			for (int j = k + 1; j < 4; j++) W[i][j] -= W[i][k] * W[k][j];
+		}
+	}
+	if (sing) return -1;
+	auto solve = [&](const double b[4], double v[4]) {
+#pragma unroll
+		for (int i = 0; i < 4; i++) v[i] = b[i];
+#pragma unroll
+		for (int k = 0; k < 3; k++)
+#pragma unroll
+			for (int i = k + 1; i < 4; i++) {
+				const bool sw = piv[k] == i;
+				const double a = v[k], q = v[i];
+				v[k] = sw ? q : a;
+				v[i] = sw ? a : q;
+			}
+#pragma unroll
+		for (int i = 1; i < 4; i++)
+#pragma unroll
+			for (int j = 0; j < i; j++) v[i] -= W[i][j] * v[j];
+#pragma unroll
+		for (int i = 3; i >= 0; i--) {
+#pragma unroll
+			for (int j = i + 1; j < 4; j++) v[i] -= W[i][j] * v[j];
+			v[i] /= W[i][i];
+		}
+	};
+	auto rdot = [&](int i, const double k[4]) {
+		return JR[i][0] * k[0] + JR[i][1] * k[1] + JR[i][2] * k[2] + JR[i][3] * k[3];
+	};
+	double k1[4], k2[4], k3[4], F1[4], F2[4], y[4], yn[4], b[4], e[4];
+	double R1[3] = {0.0, 0.0, 0.0}, R2[3] = {0.0, 0.0, 0.0}, kr1[3], kr2[3];
+	solve(S.F0, k1);
+	if (REC)
+#pragma unroll
+		for (int i = 0; i < 3; i++) kr1[i] = S.R0[i] + h * d * rdot(i, k1);
+#pragma unroll
+	for (int i = 0; i < 4; i++) y[i] = S.x[i] + 0.5 * h * k1[i];
+	rhs_he(P, c, y, F1, REC ? R1 : nullptr);
+#pragma unroll
+	for (int i = 0; i < 4; i++) b[i] = F1[i] - k1[i];
+	solve(b, k2);
+	if (REC)
+#pragma unroll
+		for (int i = 0; i < 3; i++) kr2[i] = (R1[i] - kr1[i]) + h * d * rdot(i, k2) + kr1[i];
+#pragma unroll
+	for (int i = 0; i < 4; i++) {
+		k2[i] += k1[i];
+		yn[i] = S.x[i] + h * k2[i];
+	}
+	rhs_he(P, c, yn, F2, REC ? R2 : nullptr);
+#pragma unroll
+	for (int i = 0; i < 4; i++) b[i] = F2[i] - e32 * (k2[i] - F1[i]) - 2.0 * (k1[i] - S.F0[i]);
+	solve(b, k3);
+#pragma unroll
+	for (int i = 0; i < 4; i++) e[i] = h / 6.0 * (k1[i] - 2.0 * k2[i] + k3[i]);
+	const double err = he_err_norm(e, S.x, yn, S.atol3, RB_RTOL);
+	if (err <= 1.0 && isfinite(err)) {
+		S.t += h;
+#pragma unroll
+		for (int i = 0; i < 4; i++) {
+			S.x[i] = yn[i];
+			S.F0[i] = F2[i];
+		}
+		if (REC)
+#pragma unroll
+			for (int i = 0; i < 3; i++) {
+				S.rec[i] += h * kr2[i];
+				S.R0[i] = R2[i];
+			}
+	}
+	const double fac = (err > 0.0 && isfinite(err)) ? fmin(5.0, fmax(0.2, 0.9 * pow(err, -1.0 / 3.0)))
+			: (isfinite(err) ? 5.0 : 0.2);
+	S.h = fmax(h * fac, 1e-14);
+	return S.t >= 1.0 ? 1 : 0;
+}
+
+// The whole finish on one thread; false if the step limit is reached or W
+// is singular.
+template <bool REC>
+__device__ inline bool rosenbrock_he(const PhysParams &P, const HeCtx &c, double x[4], double t, double h,
+		int max_steps, double *rec) {
+	HeRbState S;
+	he_rb_init<REC>(P, c, S, x, t, h, rec);
+	int done = t >= 1.0;
+	for (int it = 0; it < max_steps && done == 0; it++) done = he_rb_step<REC, false>(P, c, S);
+	for (int i = 0; i < 4; i++) x[i] = S.x[i];
+	if (REC)
+		for (int i = 0; i < 3; i++) rec[i] = S.rec[i];
+	return done == 1;
 }
 
 // Up to HE_SWITCH Dormand-Prince 5(4) steps over the four variables from
@@ -263,7 +365,7 @@ __device__ inline bool rosenbrock_he(const PhysParams &P, const HeStep &s, doubl
 // rec[3] accumulates the recombination photons as a quadrature over the
 // same stages.
 template <bool REC>
-__device__ inline bool dopri_he_explicit(const PhysParams &P, const HeStep &s, double x[4], double *rec,
+__device__ inline bool dopri_he_explicit(const PhysParams &P, const HeCtx &s, double x[4], double *rec,
 		double *t_out, double *h_out) {
 	const double a21 = 1. / 5, a31 = 3. / 40, a32 = 9. / 40, a41 = 44. / 45, a42 = -56. / 15, a43 = 32. / 9;
 	const double a51 = 19372. / 6561, a52 = -25360. / 2187, a53 = 64448. / 6561, a54 = -212. / 729;
@@ -325,12 +427,12 @@ __device__ inline bool dopri_he_explicit(const PhysParams &P, const HeStep &s, d
 }
 
 // Dormand-Prince 5(4) over the four variables, then the Rosenbrock finish.
-__device__ inline bool dopri_he(const PhysParams &P, const HeStep &s, double x[4], int max_steps,
+__device__ inline bool dopri_he(const PhysParams &P, const HeCtx &s, double x[4], int max_steps,
 		double *rec = nullptr) {
 	double t = 0.0, h = 0.0;
-	const bool done = rec ? dopri_he_explicit<true>(P, s, x, rec, &t, &h) : dopri_he_explicit<false>(P, s, x, rec, &t, &h);
-	if (done) return true;
-	return rosenbrock_he(P, s, x, t, h, max_steps, rec);
+	if (rec)
+		return dopri_he_explicit<true>(P, s, x, rec, &t, &h) || rosenbrock_he<true>(P, s, x, t, h, max_steps, rec);
+	return dopri_he_explicit<false>(P, s, x, rec, &t, &h) || rosenbrock_he<false>(P, s, x, t, h, max_steps, rec);
 }
 
 // step_evolve_euler() solve.c:225-316 with helium: the internal step a
@@ -355,11 +457,12 @@ __device__ inline uint32_t euler_he(const PhysParams &P, const HeStep &s, double
 	if (nsteps < 1) nsteps = 1;
 	const double h = 1.0 / nsteps;
 	refined = nsteps > 1;
+	const HeCtx cx = make_he_ctx(s);
 	uint32_t st = 0;
 	int k;
 	for (k = 0; k < nsteps; k++) {
 		double dx[4], r[3] = {0.0, 0.0, 0.0};
-		rhs_he(P, s, x, dx, rec ? r : nullptr);
+		rhs_he(P, cx, x, dx, rec ? r : nullptr);
 		if (!(x[3] + dx[3] >= 0.0)) st |= PSG_ST_IE_NEG;
 		for (int i = 0; i < 4; i++) x[i] += dx[i] * h;
 		if (rec)
@@ -395,7 +498,7 @@ __device__ inline uint32_t solve_step_he(const PhysParams &P, const HeStep &s, d
 		double *rec = nullptr) {
 	uint32_t st = 0;
 	double gain[3] = {0.0, 0.0, 0.0};
-	if (!dopri_he(P, s, x, 200000, rec ? gain : nullptr)) st |= PSG_ST_SOLVER;
+	if (!dopri_he(P, make_he_ctx(s), x, 200000, rec ? gain : nullptr)) st |= PSG_ST_SOLVER;
 	if (rec)
 		for (int i = 0; i < 3; i++) rec[i] = fmax(0.0, rec[i] + gain[i]);
 	if (!(x[3] >= 0.0)) st |= PSG_ST_IE_NEG;

@@ -18,6 +18,14 @@
 // take the library segmented sort.
 #define PSG_SORT_MAX 8192
 
+// Columns of the helium right-hand side's rate rows, two to a 16-byte load:
+// what case B (on the spot) reads comes first, case A's further ones after it.
+enum {
+	PSG_HE_CI0 = 0, PSG_HE_RC0, PSG_HE_CI1, PSG_HE_RC1, PSG_HE_CI2, PSG_HE_RC2,      // ionisation, recombination (B or A)
+	PSG_HE_RCC, PSG_HE_BREM, PSG_HE_CIC, PSG_HE_CEC, PSG_HE_COMP, PSG_HE_RCB0,       // cooling; case B beside case A
+	PSG_HE_RCB1, PSG_HE_RCB2, PSG_HE_NCOLS
+};
+
 // Bits of the device status word.
 #define PSG_ST_NAN 1u          // NaN/inf reached a particle state
 #define PSG_ST_SOLVER 2u       // the general integrator hit its step limit
@@ -65,8 +73,8 @@ struct psg_context {
 	                             // right-hand side, values then slopes per log T
 	double ar_step = 0;
 	double ar_ni_scale[8] = {};  // each d_ar_ni column is stored divided by this
-	float2 *d_ar_all = nullptr;  // [ar_nrows][16]: (value, slope) of all 15 rate columns (helium)
-	double ar_all_scale[PSG_AR_NCOLS] = {};
+	float4 *d_ar_he = nullptr;   // [ar_nrows][8]: the helium right-hand side's columns (PSG_HE_*), (value, slope) pairs
+	double ar_he_scale[PSG_HE_NCOLS] = {};
 	int ar_nrows = 0;
 	double ar_min = 0, ar_step_inv = 0;
 	double *d_xs = nullptr;      // [4][xs_nrows]: energy, sigma_HI, sigma_HeI, sigma_HeII

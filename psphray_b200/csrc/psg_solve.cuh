@@ -35,8 +35,8 @@ struct PhysParams {
 	const float4 *ar_ni;   // [ar_nrows][4]: the right-hand side's 7 rates (+ alpha_B when not
 	                       // on the spot), values and slopes
 	double ar_ni_scale[8]; // ... each column divided by its largest magnitude
-	const float2 *ar_all;  // [ar_nrows][16]: (value, slope) of all 15 columns (helium)
-	double ar_all_scale[PSG_AR_NCOLS];
+	const float4 *ar_he;   // [ar_nrows][8]: the helium right-hand side's columns, (value, slope) pairs
+	double ar_he_scale[PSG_HE_NCOLS];   // ... each column divided by its largest magnitude
 	int ar_nrows;
 	double ar_min, ar_step_inv, ar_step;
 	float ar_min_f, ar_step_inv_f, ar_step_f;   // the same in FP32 (the explicit stages' lookups)
@@ -47,6 +47,8 @@ struct PhysParams {
 	int kernel_n;
 	double H_PER_MASS, HI_ENERGY, MPROTON_OVER_BOLTZMANN, BOLTZMANN_OVER_MPROTON, hmf, hemf;
 	double he_e;           // helium electrons per H, helium frozen (psystem.h:134-137)
+	double T_num, T_den0;  // T = T_num*ie/(T_den0 + hmf*ye): MPROTON_OVER_BOLTZMANN*2/3, hemf/4 + hmf
+	double he_f;           // helium nuclei per H: hemf/hmf/4
 	int isothermal, on_the_spot, adiabatic, euler;
 	float *ygrec;          // yGrecHII per particle (leaf order), when not on the spot
 	// helium (h_only = 0) and secondary ionisation
@@ -178,8 +180,6 @@ struct RhsCtx {
 	double yeMET, g, heat, time, nH, T;
 	double nHt;                  // nH*time: rates per unit normalised time
 	double hpt;                  // H_PER_MASS*time
-	double T_num;                // MPROTON_OVER_BOLTZMANN*2/3: T = T_num*ie/(T_den0 + hmf*ye)
-	double T_den0;               // hemf/4 + hmf
 };
 
 __device__ __forceinline__ RhsCtx make_rhs_ctx(const PhysParams &P, double yeMET, double g, double heat,
@@ -188,8 +188,6 @@ __device__ __forceinline__ RhsCtx make_rhs_ctx(const PhysParams &P, double yeMET
 	c.yeMET = yeMET; c.g = g; c.heat = heat; c.time = time; c.nH = nH; c.T = T;
 	c.nHt = nH * time;
 	c.hpt = P.H_PER_MASS * time;
-	c.T_num = P.MPROTON_OVER_BOLTZMANN * 2.0 / 3.0;
-	c.T_den0 = P.hemf * 0.25 + P.hmf;
 	return c;
 }
 
@@ -219,7 +217,7 @@ __device__ __forceinline__ void rhs(const PhysParams &P, const RhsCtx &cx, const
 	float duf = 0.0f;
 	if (T32) {
 		const float Tf = P.isothermal ? (float)cx.T
-				: __fdividef((float)cx.T_num * (float)x[1], (float)__fma_rn(P.hmf, ye, cx.T_den0));
+				: __fdividef((float)P.T_num * (float)x[1], (float)__fma_rn(P.hmf, ye, P.T_den0));
 		const float lT = __log10f(Tf);
 		const float uf = (lT - P.ar_min_f) * P.ar_step_inv_f;
 		const int i = (int)uf;       // truncation; a NaN converts to 0, caught by uf == uf
@@ -232,7 +230,7 @@ __device__ __forceinline__ void rhs(const PhysParams &P, const RhsCtx &cx, const
 			duf = lT - __fmaf_rn((float)i, P.ar_step_f, P.ar_min_f);
 		}
 	} else {
-		const double logT = log10(P.isothermal ? cx.T : cx.T_num * x[1] / __fma_rn(P.hmf, ye, cx.T_den0));
+		const double logT = log10(P.isothermal ? cx.T : P.T_num * x[1] / __fma_rn(P.hmf, ye, P.T_den0));
 		idx = (long long)((logT - P.ar_min) * P.ar_step_inv);
 		if (idx < 0) {
 			idx = 0;
@@ -371,26 +369,64 @@ __device__ __forceinline__ bool dp_step(const PhysParams &P, const RhsCtx &cx, D
 // explicit method crawl. After DP_SWITCH steps such a particle continues
 // with a Rosenbrock method (the L-stable second-order W-method with
 // third-order error estimate of Shampine & Reichelt's ode23s), Jacobian by
-// finite differences, rtol RB_RTOL.
+// finite differences, rtol RB_RTOL. The state of one integration is an
+// RbState, so that a warp can step 32 of them and refill its lanes.
 #define DP_SWITCH 32
 #define RB_RTOL 1e-5
 
-// With REC, *rec accumulates yGrecHII: the third component of the augmented
+// With REC, rec accumulates yGrecHII: the third component of the augmented
 // system, whose Jacobian column is zero, so W's last row only adds
 // h*d*(J20*k0 + J21*k1) to its stage values; it stays out of the error norm.
-template <bool REC = false>
-__device__ inline bool rosenbrock(const PhysParams &P, const RhsCtx &cx, double x[2], double t, double h,
-		int max_steps, double *rec = nullptr) {
+struct RbState {
+	double x[2], F0[2], t, h, atol1;
+	double rec, R0;
+};
+
+template <bool REC>
+__device__ __forceinline__ void rb_init(const PhysParams &P, const RhsCtx &cx, RbState &S, double x0, double x1,
+		double t, double h, double rec) {
+	S.x[0] = x0;
+	S.x[1] = x1;
+	S.t = t;
+	S.h = fmin(fmax(h, 1e-10), 1.0);
+	S.atol1 = DP_ATOL1_REL * fabs(x1) + 1e-300;
+	S.rec = rec;
+	S.R0 = 0.0;
+	rhs<REC>(P, cx, S.x, S.F0, &S.R0);
+}
+
+// One attempted step from S.t < 1; returns true once s = 1 is reached. With
+// PAIR two neighbouring lanes hold the same integration and evaluate a
+// column of the Jacobian each, the rest alike: a step is then three
+// right-hand sides long instead of four. mask: the lanes that call (pairs).
+template <bool REC, bool PAIR>
+__device__ __forceinline__ bool rb_step(const PhysParams &P, const RhsCtx &cx, RbState &S, unsigned mask = 0) {
 	const double d = 1.0 / (2.0 + 1.4142135623730951), e32 = 6.0 + 1.4142135623730951;
-	const double atol[2] = {DP_ATOL0, DP_ATOL1_REL * fabs(x[1]) + 1e-300};
-	double F0[2], R0 = 0.0;
-	rhs<REC>(P, cx, x, F0, &R0);
-	h = fmin(fmax(h, 1e-10), 1.0);
-	for (int it = 0; it < max_steps; it++) {
-		if (t >= 1.0) return true;
-		if (t + h > 1.0) h = 1.0 - t;
-		// Jacobian by forward differences
-		double J[2][2], JR[2] = {0.0, 0.0};
+	const double atol[2] = {DP_ATOL0, S.atol1};
+	double *x = S.x, *F0 = S.F0;
+	double h = S.h;
+	if (S.t + h > 1.0) h = 1.0 - S.t;
+	// Jacobian by forward differences
+	double J[2][2], JR[2] = {0.0, 0.0};
+	if (PAIR) {
+		const bool odd = threadIdx.x & 1;
+		const double xj = odd ? x[1] : x[0];
+		const double del = 1e-7 * fmax(fabs(xj), (odd ? atol[1] : atol[0]) / RB_RTOL);
+		const double y[2] = {odd ? x[0] : x[0] + del, odd ? x[1] + del : x[1]};
+		double Fj[2], Rj = 0.0;
+		rhs<REC>(P, cx, y, Fj, &Rj);
+		const double c0 = (Fj[0] - F0[0]) / del, c1 = (Fj[1] - F0[1]) / del;
+		const double o0 = __shfl_xor_sync(mask, c0, 1), o1 = __shfl_xor_sync(mask, c1, 1);
+		J[0][0] = odd ? o0 : c0;
+		J[1][0] = odd ? o1 : c1;
+		J[0][1] = odd ? c0 : o0;
+		J[1][1] = odd ? c1 : o1;
+		if (REC) {
+			const double cr = (Rj - S.R0) / del, co = __shfl_xor_sync(mask, cr, 1);
+			JR[0] = odd ? co : cr;
+			JR[1] = odd ? cr : co;
+		}
+	} else {
 		for (int j = 0; j < 2; j++) {
 			const double del = 1e-7 * fmax(fabs(x[j]), atol[j] / RB_RTOL);
 			double y[2] = {x[0], x[1]}, Fj[2], Rj = 0.0;
@@ -398,56 +434,70 @@ __device__ inline bool rosenbrock(const PhysParams &P, const RhsCtx &cx, double 
 			rhs<REC>(P, cx, y, Fj, &Rj);
 			J[0][j] = (Fj[0] - F0[0]) / del;
 			J[1][j] = (Fj[1] - F0[1]) / del;
-			if (REC) JR[j] = (Rj - R0) / del;
+			if (REC) JR[j] = (Rj - S.R0) / del;
 		}
-		const double a00 = 1.0 - h * d * J[0][0], a01 = -h * d * J[0][1];
-		const double a10 = -h * d * J[1][0], a11 = 1.0 - h * d * J[1][1];
-		const double det = a00 * a11 - a01 * a10;
-		auto solve = [&](const double b[2], double out[2]) {
-			out[0] = (a11 * b[0] - a01 * b[1]) / det;
-			out[1] = (a00 * b[1] - a10 * b[0]) / det;
-		};
-		double k1[2], k2[2], k3[2], F1[2], F2[2], y[2], yn[2], b[2], R1 = 0.0, R2 = 0.0;
-		solve(F0, k1);
-		const double kr1 = REC ? R0 + h * d * (JR[0] * k1[0] + JR[1] * k1[1]) : 0.0;
-		y[0] = x[0] + 0.5 * h * k1[0];
-		y[1] = x[1] + 0.5 * h * k1[1];
-		rhs<REC>(P, cx, y, F1, &R1);
-		b[0] = F1[0] - k1[0];
-		b[1] = F1[1] - k1[1];
-		solve(b, k2);
-		const double kr2 = REC ? (R1 - kr1) + h * d * (JR[0] * k2[0] + JR[1] * k2[1]) + kr1 : 0.0;
-		k2[0] += k1[0];
-		k2[1] += k1[1];
-		yn[0] = x[0] + h * k2[0];
-		yn[1] = x[1] + h * k2[1];
-		rhs<REC>(P, cx, yn, F2, &R2);
-		b[0] = F2[0] - e32 * (k2[0] - F1[0]) - 2.0 * (k1[0] - F0[0]);
-		b[1] = F2[1] - e32 * (k2[1] - F1[1]) - 2.0 * (k1[1] - F0[1]);
-		solve(b, k3);
-		double err = 0.0;
-		for (int i = 0; i < 2; i++) {
-			const double e = h / 6.0 * (k1[i] - 2.0 * k2[i] + k3[i]);
-			const double sc = atol[i] + RB_RTOL * fmax(fabs(x[i]), fabs(yn[i]));
-			err += (e / sc) * (e / sc);
-		}
-		err = sqrt(0.5 * err);
-		if (err <= 1.0 && isfinite(err)) {
-			t += h;
-			x[0] = yn[0];
-			x[1] = yn[1];
-			F0[0] = F2[0];
-			F0[1] = F2[1];
-			if (REC) {
-				*rec += h * kr2;
-				R0 = R2;
-			}
-		}
-		const float fac = (err > 0.0 && isfinite(err))
-				? fminf(5.0f, fmaxf(0.2f, 0.9f * __powf((float)err, -1.0f / 3.0f))) : (isfinite(err) ? 5.0f : 0.2f);
-		h = fmax(h * (double)fac, 1e-14);
 	}
-	return t >= 1.0;
+	const double a00 = 1.0 - h * d * J[0][0], a01 = -h * d * J[0][1];
+	const double a10 = -h * d * J[1][0], a11 = 1.0 - h * d * J[1][1];
+	const double det = a00 * a11 - a01 * a10;
+	auto solve = [&](const double b[2], double out[2]) {
+		out[0] = (a11 * b[0] - a01 * b[1]) / det;
+		out[1] = (a00 * b[1] - a10 * b[0]) / det;
+	};
+	double k1[2], k2[2], k3[2], F1[2], F2[2], y[2], yn[2], b[2], R1 = 0.0, R2 = 0.0;
+	solve(F0, k1);
+	const double kr1 = REC ? S.R0 + h * d * (JR[0] * k1[0] + JR[1] * k1[1]) : 0.0;
+	y[0] = x[0] + 0.5 * h * k1[0];
+	y[1] = x[1] + 0.5 * h * k1[1];
+	rhs<REC>(P, cx, y, F1, &R1);
+	b[0] = F1[0] - k1[0];
+	b[1] = F1[1] - k1[1];
+	solve(b, k2);
+	const double kr2 = REC ? (R1 - kr1) + h * d * (JR[0] * k2[0] + JR[1] * k2[1]) + kr1 : 0.0;
+	k2[0] += k1[0];
+	k2[1] += k1[1];
+	yn[0] = x[0] + h * k2[0];
+	yn[1] = x[1] + h * k2[1];
+	rhs<REC>(P, cx, yn, F2, &R2);
+	b[0] = F2[0] - e32 * (k2[0] - F1[0]) - 2.0 * (k1[0] - F0[0]);
+	b[1] = F2[1] - e32 * (k2[1] - F1[1]) - 2.0 * (k1[1] - F0[1]);
+	solve(b, k3);
+	double err = 0.0;
+	for (int i = 0; i < 2; i++) {
+		const double e = h / 6.0 * (k1[i] - 2.0 * k2[i] + k3[i]);
+		const double sc = atol[i] + RB_RTOL * fmax(fabs(x[i]), fabs(yn[i]));
+		err += (e / sc) * (e / sc);
+	}
+	err = sqrt(0.5 * err);
+	if (err <= 1.0 && isfinite(err)) {
+		S.t += h;
+		x[0] = yn[0];
+		x[1] = yn[1];
+		F0[0] = F2[0];
+		F0[1] = F2[1];
+		if (REC) {
+			S.rec += h * kr2;
+			S.R0 = R2;
+		}
+	}
+	const float fac = (err > 0.0 && isfinite(err))
+			? fminf(5.0f, fmaxf(0.2f, 0.9f * __powf((float)err, -1.0f / 3.0f))) : (isfinite(err) ? 5.0f : 0.2f);
+	S.h = fmax(h * (double)fac, 1e-14);
+	return S.t >= 1.0;
+}
+
+// The whole finish on one thread; false if the step limit is reached.
+template <bool REC = false>
+__device__ inline bool rosenbrock(const PhysParams &P, const RhsCtx &cx, double x[2], double t, double h,
+		int max_steps, double *rec = nullptr) {
+	RbState S;
+	rb_init<REC>(P, cx, S, x[0], x[1], t, h, REC ? *rec : 0.0);
+	bool done = t >= 1.0;
+	for (int it = 0; it < max_steps && !done; it++) done = rb_step<REC, false>(P, cx, S);
+	x[0] = S.x[0];
+	x[1] = S.x[1];
+	if (REC) *rec = S.rec;
+	return done;
 }
 
 // Whole integration on one thread; returns false if the step limit is

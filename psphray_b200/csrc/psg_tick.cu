@@ -34,8 +34,8 @@ PhysParams psg_phys_params(const psg_context *ctx) {
 	P.ar = ctx->d_ar;
 	P.ar_ni = ctx->d_ar_ni;
 	for (int c = 0; c < 8; c++) P.ar_ni_scale[c] = ctx->ar_ni_scale[c];
-	P.ar_all = ctx->d_ar_all;
-	for (int c = 0; c < PSG_AR_NCOLS; c++) P.ar_all_scale[c] = ctx->ar_all_scale[c];
+	P.ar_he = ctx->d_ar_he;
+	for (int c = 0; c < PSG_HE_NCOLS; c++) P.ar_he_scale[c] = ctx->ar_he_scale[c];
 	P.ar_step = ctx->ar_step;
 	P.ar_nrows = ctx->ar_nrows;
 	P.ar_min = ctx->ar_min;
@@ -58,6 +58,9 @@ PhysParams psg_phys_params(const psg_context *ctx) {
 	P.hemf = ctx->u.hemf;
 	// lambda_to_ye() psystem.h:134-138 with lambdaHeI = lambdaHeII = 0
 	P.he_e = ctx->u.hemf / ctx->u.hmf * 0.25 * (0.0 + 2 * (1.0 - 0.0 - 0.0));
+	P.T_num = ctx->u.MPROTON_OVER_BOLTZMANN * 2.0 / 3.0;
+	P.T_den0 = ctx->u.hemf * 0.25 + ctx->u.hmf;
+	P.he_f = ctx->u.hemf / ctx->u.hmf * 0.25;
 	P.isothermal = ctx->flags.isothermal;
 	P.on_the_spot = ctx->flags.on_the_spot;
 	P.adiabatic = ctx->flags.adiabatic;
@@ -1347,28 +1350,89 @@ __global__ void __launch_bounds__(32 * UPD_WARPS, MINB) k_update_queue(int t, co
 	if (st) atomicOr(status, st);
 }
 
-// The stiff particles of a tick, one thread each (their number is read on
-// the device): Rosenbrock from where the explicit steps stopped.
+// The stiff particles of a tick, Rosenbrock from where the explicit steps
+// stopped. One particle's steps are a serial chain, up to several hundred of
+// them, each a few right-hand sides of FP64 divisions and a logarithm long;
+// the longest chain bounds the kernel. So a particle takes a group of lanes
+// (two here, four with helium) that evaluate the Jacobian's columns side by
+// side, the first particles are dealt out over all warps, and a group whose
+// particle is done takes the next one from the tick's cursor (once a quarter
+// of the warp is idle: a refill costs the warp a right-hand side). On the
+// 16.8 M-particle field (2e5 stiff particles a tick, 10 steps each on average
+// and 800 at most) a tick went from 33.3 to 25.8 ms; before, 9472 threads
+// took the particles in a fixed stride and each warp waited for its longest.
+#define STIFF_THREADS 64
+// groups of a warp that take part: all, or as many as the first deal fills
+template <int G>
+__device__ __forceinline__ int stiff_groups(unsigned n, unsigned nwarp) {
+	return (int)min((unsigned)(32 / G), (n + nwarp - 1) / nwarp);
+}
+// the next item of each group of `need` (n and above: none left): the first
+// round dealt from the warp's index, later ones from the cursor, which
+// counts from behind that round
+template <int G>
+__device__ __forceinline__ unsigned stiff_next(unsigned need, bool first, int groups, unsigned warp, unsigned nwarp,
+		unsigned *__restrict__ cursor, int lane) {
+	if (first) return warp + nwarp * (unsigned)(lane / G);
+	unsigned base = 0;
+	const int leader = __ffs(need) - 1;
+	if (lane == leader) base = atomicAdd(cursor, (unsigned)__popc(need) / G);
+	base = __shfl_sync(0xffffffffu, base, leader);
+	return nwarp * (unsigned)groups + base + (unsigned)__popc(need & ((1u << (lane & ~(G - 1))) - 1u)) / G;
+}
+
 template <bool REC>
-__global__ void __launch_bounds__(64) k_update_stiff(const StiffItem *__restrict__ stiff,
-		const unsigned *__restrict__ nstiff, double *__restrict__ lambdaH, float *__restrict__ ie,
-		int64_t *__restrict__ lasthit, PhysParams P, const PsgBatchDev *__restrict__ B, int t,
+__global__ void __launch_bounds__(STIFF_THREADS) k_update_stiff(const StiffItem *__restrict__ stiff,
+		const unsigned *__restrict__ nstiff, unsigned *__restrict__ cursor, double *__restrict__ lambdaH,
+		float *__restrict__ ie, int64_t *__restrict__ lasthit, PhysParams P, const PsgBatchDev *__restrict__ B, int t,
 		uint32_t *__restrict__ status) {
-	const int64_t tick = B->tick0 + t;
+	constexpr int G = 2;
 	const unsigned n = *nstiff;
-	uint32_t st = 0;
-	for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-		const StiffItem it = stiff[i];
-		const RhsCtx cx = make_rhs_ctx(P, it.yeMET, it.g, it.heat, it.time, it.nH, it.T);
-		double x[2] = {it.x0, it.x1};
-		double rec = it.rec;
-		if (!rosenbrock<REC>(P, cx, x, it.t, it.h, UPD_MAX_STEPS, &rec)) st |= PSG_ST_SOLVER;
-		if (REC) P.ygrec[it.p] = (float)fmax(0.0, (double)P.ygrec[it.p] + rec);
-		if (!(x[1] >= 0.0)) st |= PSG_ST_IE_NEG;
-		if (!isfinite(x[0]) || !isfinite(x[1])) st |= PSG_ST_NAN;
-		lambdaH[it.p] = fmin(1.0, fmax(0.0, x[0]));
-		if (!P.adiabatic) ie[it.p] = (float)x[1];
-		lasthit[it.p] = tick;
+	const unsigned nwarp = gridDim.x * (STIFF_THREADS / 32), warp = blockIdx.x + gridDim.x * (threadIdx.x >> 5);
+	if (warp >= n) return;
+	const int64_t tick = B->tick0 + t;
+	const int lane = threadIdx.x & 31, groups = stiff_groups<G>(n, nwarp);
+	uint32_t st = 0, p = 0;
+	bool have = false, dry = lane / G >= groups, first = true;
+	int steps = 0;
+	RbState S;
+	RhsCtx cx;
+	for (;;) {
+		const unsigned need = __ballot_sync(0xffffffffu, !have && !dry), busy = __ballot_sync(0xffffffffu, have);
+		if (need && (__popc(need) >= 8 || !busy)) {
+			const unsigned i = stiff_next<G>(need, first, groups, warp, nwarp, cursor, lane);
+			first = false;
+			if (!have && !dry) {
+				if (i < n) {
+					const StiffItem it = stiff[i];
+					p = it.p;
+					cx = make_rhs_ctx(P, it.yeMET, it.g, it.heat, it.time, it.nH, it.T);
+					rb_init<REC>(P, cx, S, it.x0, it.x1, it.t, it.h, it.rec);
+					steps = 0;
+					have = true;
+				} else {
+					dry = true;
+				}
+			}
+		} else if (!busy) {
+			break;
+		}
+		const unsigned all = __ballot_sync(0xffffffffu, have);
+		if (have) {
+			const bool done = rb_step<REC, true>(P, cx, S, all);
+			if (done || ++steps >= UPD_MAX_STEPS) {
+				if (!done) st |= PSG_ST_SOLVER;
+				if (!(S.x[1] >= 0.0)) st |= PSG_ST_IE_NEG;
+				if (!isfinite(S.x[0]) || !isfinite(S.x[1])) st |= PSG_ST_NAN;
+				if (lane % G == 0) {
+					if (REC) P.ygrec[p] = (float)fmax(0.0, (double)P.ygrec[p] + S.rec);
+					lambdaH[p] = fmin(1.0, fmax(0.0, S.x[0]));
+					if (!P.adiabatic) ie[p] = (float)S.x[1];
+					lasthit[p] = tick;
+				}
+				have = false;
+			}
+		}
 	}
 	if (st) atomicOr(status, st);
 }
@@ -1560,7 +1624,7 @@ __global__ void __launch_bounds__(128, 4) k_update_he(int t, const int32_t *__re
 		P.gcarryHe2[p] = g2 * remain;
 	} else {
 		double gain[3] = {0.0, 0.0, 0.0}, tt = 0.0, hh = 0.0;
-		if (!dopri_he_explicit<REC>(P, s, x, gain, &tt, &hh)) {
+		if (!dopri_he_explicit<REC>(P, make_he_ctx(s), x, gain, &tt, &hh)) {
 			HeStiffItem it;
 			it.s = s;
 			for (int k = 0; k < 4; k++) it.x[k] = x[k];
@@ -1583,27 +1647,62 @@ __global__ void __launch_bounds__(128, 4) k_update_he(int t, const int32_t *__re
 	}
 }
 
-// The stiff helium particles of a tick, one thread each (their number is
-// read on the device): the Rosenbrock finish from where the explicit steps
-// stopped.
-__global__ void __launch_bounds__(64) k_update_he_stiff(const HeStiffItem *__restrict__ stiff,
-		const unsigned *__restrict__ nstiff, double *__restrict__ lambdaH, float *__restrict__ ie,
-		int64_t *__restrict__ lasthit, PhysParams P, const PsgBatchDev *__restrict__ B, int t,
+// The stiff helium particles of a tick (as k_update_stiff): the Rosenbrock
+// finish from where the explicit steps stopped.
+template <bool REC>
+__global__ void __launch_bounds__(STIFF_THREADS) k_update_he_stiff(const HeStiffItem *__restrict__ stiff,
+		const unsigned *__restrict__ nstiff, unsigned *__restrict__ cursor, double *__restrict__ lambdaH,
+		float *__restrict__ ie, int64_t *__restrict__ lasthit, PhysParams P, const PsgBatchDev *__restrict__ B, int t,
 		uint32_t *__restrict__ status) {
-	const int64_t tick = B->tick0 + t;
+	constexpr int G = 4;
 	const unsigned n = *nstiff;
+	const unsigned nwarp = gridDim.x * (STIFF_THREADS / 32), warp = blockIdx.x + gridDim.x * (threadIdx.x >> 5);
+	if (warp >= n) return;
+	const int64_t tick = B->tick0 + t;
+	const int lane = threadIdx.x & 31, groups = stiff_groups<G>(n, nwarp);
 	uint32_t st = 0;
-	for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-		const HeStiffItem &it = stiff[i];
-		double x[4] = {it.x[0], it.x[1], it.x[2], it.x[3]};
-		double gain[3] = {0.0, 0.0, 0.0}, rec[3];
-		if (!rosenbrock_he(P, it.s, x, it.t, it.h, UPD_MAX_STEPS, P.ygrec ? gain : nullptr)) st |= PSG_ST_SOLVER;
-		if (!(x[3] >= 0.0)) st |= PSG_ST_IE_NEG;
-		for (int k = 0; k < 4; k++)
-			if (!isfinite(x[k])) st |= PSG_ST_NAN;
-		clamp_he(x);
-		for (int k = 0; k < 3; k++) rec[k] = fmax(0.0, it.rec[k] + gain[k]);
-		he_write(P, it.p, x, rec, it.s.T, tick, lambdaH, ie, lasthit);
+	unsigned item = 0;
+	bool have = false, dry = lane / G >= groups, first = true;
+	int steps = 0;
+	HeRbState S;
+	HeCtx cx;
+	for (;;) {
+		const unsigned need = __ballot_sync(0xffffffffu, !have && !dry), busy = __ballot_sync(0xffffffffu, have);
+		if (need && (__popc(need) >= 8 || !busy)) {
+			const unsigned i = stiff_next<G>(need, first, groups, warp, nwarp, cursor, lane);
+			first = false;
+			if (!have && !dry) {
+				if (i < n) {
+					const HeStiffItem &it = stiff[i];
+					const double zero[3] = {0.0, 0.0, 0.0};
+					cx = make_he_ctx(it.s);
+					he_rb_init<REC>(P, cx, S, it.x, it.t, it.h, zero);
+					item = i;
+					steps = 0;
+					have = true;
+				} else {
+					dry = true;
+				}
+			}
+		} else if (!busy) {
+			break;
+		}
+		const unsigned all = __ballot_sync(0xffffffffu, have);
+		if (have) {
+			const int done = he_rb_step<REC, true>(P, cx, S, all);
+			if (done || ++steps >= UPD_MAX_STEPS) {
+				const HeStiffItem &it = stiff[item];
+				double rec[3];
+				if (done != 1) st |= PSG_ST_SOLVER;
+				if (!(S.x[3] >= 0.0)) st |= PSG_ST_IE_NEG;
+				for (int k = 0; k < 4; k++)
+					if (!isfinite(S.x[k])) st |= PSG_ST_NAN;
+				clamp_he(S.x);
+				for (int k = 0; k < 3; k++) rec[k] = fmax(0.0, it.rec[k] + (REC ? S.rec[k] : 0.0));
+				if (lane % G == 0) he_write(P, it.p, S.x, rec, it.s.T, tick, lambdaH, ie, lasthit);
+				have = false;
+			}
+		}
 	}
 	if (st) atomicOr(status, st);
 }
@@ -1767,7 +1866,7 @@ struct BatchPlan {
 	bool gen = false, helium = false, iso = false, euler = false, surr = false, aff = false, feat_on = false;
 
 	// grids
-	unsigned dep_grid = 0, red_grid = 0, queue_grid = 0, he_grid = 0, euler_grid = 0, log_grid = 0;
+	unsigned dep_grid = 0, red_grid = 0, queue_grid = 0, he_grid = 0, euler_grid = 0, log_grid = 0, stiff_grid = 0;
 	int queue_minb = 1;         // the integrator's register limit: resident blocks per SM
 	size_t src_R = 0;           // > 0: a recombination tick whose first src_R rays come traced and sorted (S_SRCHIT)
 };
@@ -1851,7 +1950,7 @@ size_t long_lists_bytes(const BatchPlan &pl) {
 }
 struct UpdView {
 	double *act_g, *act_heat;
-	unsigned *cursors, *nstiff, *nrej, *dep_ctr, *cursors2;
+	unsigned *cursors, *nstiff, *nrej, *dep_ctr, *cursors2, *stiff_ctr;
 	TickRays *tick_rays;
 	StiffItem *stiff;
 	uint32_t *rej;
@@ -1868,14 +1967,15 @@ UpdView upd_view(psg_context *ctx, const BatchPlan &pl) {
 	v.nrej = v.nstiff + (pl.K + 1);
 	v.dep_ctr = v.nrej + (pl.K + 1);
 	v.cursors2 = v.dep_ctr + (pl.K + 1);       // the integrator's second pass (update_order)
-	v.tick_rays = (TickRays *)(((uintptr_t)(v.cursors2 + pl.K + 1) + 31) & ~(uintptr_t)31);
+	v.stiff_ctr = v.cursors2 + (pl.K + 1);     // the stiff finish's
+	v.tick_rays = (TickRays *)(((uintptr_t)(v.stiff_ctr + pl.K + 1) + 31) & ~(uintptr_t)31);
 	v.stiff = (StiffItem *)(((uintptr_t)(v.tick_rays + pl.K) + 15) & ~(uintptr_t)15);
 	v.rej = (uint32_t *)(v.stiff + (pl.iso ? 0 : pl.pcap));
 	v.act_slow = (uint8_t *)(v.rej + (pl.surr ? pl.pcap : 0));
 	return v;
 }
 size_t upd_bytes(const BatchPlan &pl) {
-	return sizeof(double) * (pl.helium ? 4 : 2) * pl.cap + sizeof(unsigned) * 5 * (pl.K + 1) + sizeof(TickRays) * pl.K +
+	return sizeof(double) * (pl.helium ? 4 : 2) * pl.cap + sizeof(unsigned) * 6 * (pl.K + 1) + sizeof(TickRays) * pl.K +
 			(pl.iso ? 0 : sizeof(StiffItem) * pl.pcap + pl.cap) + (pl.surr ? sizeof(uint32_t) * pl.pcap : 0) + 512;
 }
 
@@ -1957,6 +2057,8 @@ int plan_batch(psg_context *ctx, size_t R, size_t K, const PsgTraceFill &tf, Bat
 			: pl.queue_minb == 3 ? occ_grid(ctx, k_update_queue<false, 3>, 32 * UPD_WARPS)
 			: occ_grid(ctx, k_update_queue<false, 1>, 32 * UPD_WARPS);
 	pl.he_grid = occ_grid(ctx, k_update_he<false>, 128);
+	pl.stiff_grid = pl.helium ? (ctx->flags.on_the_spot ? occ_grid(ctx, k_update_he_stiff<false>, STIFF_THREADS)
+			: occ_grid(ctx, k_update_he_stiff<true>, STIFF_THREADS)) : occ_grid(ctx, k_update_stiff<true>, STIFF_THREADS);
 	pl.euler_grid = occ_grid(ctx, k_update_euler, 128);
 	pl.log_grid = (unsigned)(ctx->sms * 8);
 	if (pl.surr) {
@@ -2024,7 +2126,7 @@ int enqueue_batch(psg_context *ctx, const BatchPlan &pl, const PsgBatchDev *B) {
 
 	// the long-segment lists and (not isothermal) the integrator's work
 	// cursors, stiff lists and the deposit's unit counters
-	PSG_CUDA(cudaMemsetAsync(uv.cursors, 0, sizeof(unsigned) * 5 * (K + 1), st));
+	PSG_CUDA(cudaMemsetAsync(uv.cursors, 0, sizeof(unsigned) * 6 * (K + 1), st));
 	if (pl.surr) PSG_CUDA(cudaMemsetAsync(ctx->d_counters + 8, 0, sizeof(unsigned long long), st));
 	UpdRec *urec = (!pl.helium && pl.euler) ? (UpdRec *)ctx->scratch[S_REC].p : nullptr;
 	HeStiffItem *hstiff = pl.helium ? (HeStiffItem *)ctx->scratch[S_REC].p : nullptr;
@@ -2095,8 +2197,12 @@ int enqueue_batch(psg_context *ctx, const BatchPlan &pl, const PsgBatchDev *B) {
 						uv.act_heat, ctx->d_lambdaH, ctx->d_ie, ctx->d_lasthit, ctx->d_rho,
 						ctx->d_yeMET, P, B, hstiff, uv.nstiff + t, ctx->d_status);
 			PSG_CHECK_LAUNCH();
-			k_update_he_stiff<<<sms, 64, 0, st>>>(hstiff, uv.nstiff + t, ctx->d_lambdaH, ctx->d_ie, ctx->d_lasthit,
-					P, B, (int)t, ctx->d_status);
+			if (P.ygrec)
+				k_update_he_stiff<true><<<pl.stiff_grid, STIFF_THREADS, 0, st>>>(hstiff, uv.nstiff + t, uv.stiff_ctr + t,
+						ctx->d_lambdaH, ctx->d_ie, ctx->d_lasthit, P, B, (int)t, ctx->d_status);
+			else
+				k_update_he_stiff<false><<<pl.stiff_grid, STIFF_THREADS, 0, st>>>(hstiff, uv.nstiff + t, uv.stiff_ctr + t,
+						ctx->d_lambdaH, ctx->d_ie, ctx->d_lasthit, P, B, (int)t, ctx->d_status);
 			PSG_CHECK_LAUNCH();
 			ctx->launches += 2;
 		} else {
@@ -2155,8 +2261,8 @@ int enqueue_batch(psg_context *ctx, const BatchPlan &pl, const PsgBatchDev *B) {
 							ctx->d_lambdaH, ctx->d_ie, ctx->d_lasthit, ctx->d_hstep, P, B, uv.cursors + t, cur2,
 							uv.stiff, uv.nstiff + t, nullptr, nullptr, ctx->d_status);
 					PSG_CHECK_LAUNCH();
-					k_update_stiff<true><<<sms, 64, 0, st>>>(uv.stiff, uv.nstiff + t, ctx->d_lambdaH, ctx->d_ie,
-							ctx->d_lasthit, P, B, (int)t, ctx->d_status);
+					k_update_stiff<true><<<pl.stiff_grid, STIFF_THREADS, 0, st>>>(uv.stiff, uv.nstiff + t,
+							uv.stiff_ctr + t, ctx->d_lambdaH, ctx->d_ie, ctx->d_lasthit, P, B, (int)t, ctx->d_status);
 				} else {
 #define PSG_QUEUE(MINB_)                                                                                       \
 	k_update_queue<false, MINB_><<<pl.queue_grid, 32 * UPD_WARPS, 0, st>>>((int)t, av.tick_act, us,          \
@@ -2167,8 +2273,8 @@ int enqueue_batch(psg_context *ctx, const BatchPlan &pl, const PsgBatchDev *B) {
 					else PSG_QUEUE(1);
 #undef PSG_QUEUE
 					PSG_CHECK_LAUNCH();
-					k_update_stiff<false><<<sms, 64, 0, st>>>(uv.stiff, uv.nstiff + t, ctx->d_lambdaH, ctx->d_ie,
-							ctx->d_lasthit, P, B, (int)t, ctx->d_status);
+					k_update_stiff<false><<<pl.stiff_grid, STIFF_THREADS, 0, st>>>(uv.stiff, uv.nstiff + t,
+							uv.stiff_ctr + t, ctx->d_lambdaH, ctx->d_ie, ctx->d_lasthit, P, B, (int)t, ctx->d_status);
 				}
 				PSG_CHECK_LAUNCH();
 				ctx->launches += 2;
