@@ -359,71 +359,144 @@ __device__ inline bool rosenbrock_he(const PhysParams &P, const HeCtx &c, double
 	return done == 1;
 }
 
-// Up to HE_SWITCH Dormand-Prince 5(4) steps over the four variables from
-// s = 0; returns true once s = 1 is reached, else leaves the time reached
-// and the next step size in *t_out, *h_out. With rec (not on the spot),
-// rec[3] accumulates the recombination photons as a quadrature over the
-// same stages.
+// Dormand-Prince 5(4) over the four variables: the coefficients of the
+// stages' arguments, row 5 those of the solution, and of the error (the
+// second stage enters neither).
+static __constant__ double kHeA[6][6] = {{1. / 5, 0, 0, 0, 0, 0}, {3. / 40, 9. / 40, 0, 0, 0, 0},
+	{44. / 45, -56. / 15, 32. / 9, 0, 0, 0}, {19372. / 6561, -25360. / 2187, 64448. / 6561, -212. / 729, 0, 0},
+	{9017. / 3168, -355. / 33, 46732. / 5247, 49. / 176, -5103. / 18656, 0},
+	{35. / 384, 0, 500. / 1113, 125. / 192, -2187. / 6784, 11. / 84}};
+static __constant__ double kHeE[6] = {71. / 57600, 0, -71. / 16695, 71. / 1920, -17253. / 339200, 22. / 525};
+
+// One integration; its stages' slopes live in k (a thread's own column of
+// 6 x 4 doubles, stride apart): a step then loops over its stages with one
+// copy of the right-hand side, which needs half the registers and a seventh
+// of the instructions that the unrolled form took. With REC (not on the
+// spot) the recombination photons are a quadrature over the same stages.
+struct HeDp {
+	double x[4], t, h, atol3;
+	double gain[3], r1[3];
+	int steps;
+};
+
+// Starts the integration at x: the first slope and step. Evaluates nothing
+// but the right-hand side at x.
 template <bool REC>
-__device__ inline bool dopri_he_explicit(const PhysParams &P, const HeCtx &s, double x[4], double *rec,
-		double *t_out, double *h_out) {
-	const double a21 = 1. / 5, a31 = 3. / 40, a32 = 9. / 40, a41 = 44. / 45, a42 = -56. / 15, a43 = 32. / 9;
-	const double a51 = 19372. / 6561, a52 = -25360. / 2187, a53 = 64448. / 6561, a54 = -212. / 729;
-	const double a61 = 9017. / 3168, a62 = -355. / 33, a63 = 46732. / 5247, a64 = 49. / 176, a65 = -5103. / 18656;
-	const double b1 = 35. / 384, b3 = 500. / 1113, b4 = 125. / 192, b5 = -2187. / 6784, b6 = 11. / 84;
-	const double e1 = 71. / 57600, e3 = -71. / 16695, e4 = 71. / 1920, e5 = -17253. / 339200, e6 = 22. / 525,
-			e7 = -1. / 40;
-	const double atol3 = DP_ATOL1_REL * fabs(x[3]) + 1e-300;
-	double k1[4], r1[3] = {0.0, 0.0, 0.0};
-	rhs_he(P, s, x, k1, REC ? r1 : nullptr);
+__device__ __forceinline__ void he_dp_start(HeDp &S, const double k1[4], const double r1[3], double *k, int stride) {
+	S.t = 0.0;
+	S.steps = 0;
+	S.atol3 = DP_ATOL1_REL * fabs(S.x[3]) + 1e-300;
 	double h = 1.0;
+#pragma unroll
 	for (int i = 0; i < 4; i++) {
-		const double scale = fabs(x[i]) + (i < 3 ? DP_ATOL0 : atol3) / DP_RTOL;
+		const double scale = fabs(S.x[i]) + (i < 3 ? DP_ATOL0 : S.atol3) / DP_RTOL;
 		if (fabs(k1[i]) > 0.0) h = fmin(h, 0.01 * scale / fabs(k1[i]));
+		k[i * stride] = k1[i];
 	}
-	h = fmax(h, 1e-8);
-	double t = 0.0;
-	for (int it = 0; it < HE_SWITCH; it++) {
-		if (t >= 1.0) return true;
-		if (t + h > 1.0) h = 1.0 - t;
-		double k2[4], k3[4], k4[4], k5[4], k6[4], k7[4], y[4], yn[4], e[4];
-		double r2[3], r3[3], r4[3], r5[3], r6[3], r7[3];
-		double *q2 = REC ? r2 : nullptr, *q3 = REC ? r3 : nullptr, *q4 = REC ? r4 : nullptr;
-		double *q5 = REC ? r5 : nullptr, *q6 = REC ? r6 : nullptr, *q7 = REC ? r7 : nullptr;
-		for (int i = 0; i < 4; i++) y[i] = x[i] + h * (a21 * k1[i]);
-		rhs_he(P, s, y, k2, q2);
-		for (int i = 0; i < 4; i++) y[i] = x[i] + h * (a31 * k1[i] + a32 * k2[i]);
-		rhs_he(P, s, y, k3, q3);
-		for (int i = 0; i < 4; i++) y[i] = x[i] + h * (a41 * k1[i] + a42 * k2[i] + a43 * k3[i]);
-		rhs_he(P, s, y, k4, q4);
-		for (int i = 0; i < 4; i++) y[i] = x[i] + h * (a51 * k1[i] + a52 * k2[i] + a53 * k3[i] + a54 * k4[i]);
-		rhs_he(P, s, y, k5, q5);
-		for (int i = 0; i < 4; i++)
-			y[i] = x[i] + h * (a61 * k1[i] + a62 * k2[i] + a63 * k3[i] + a64 * k4[i] + a65 * k5[i]);
-		rhs_he(P, s, y, k6, q6);
-		for (int i = 0; i < 4; i++) yn[i] = x[i] + h * (b1 * k1[i] + b3 * k3[i] + b4 * k4[i] + b5 * k5[i] + b6 * k6[i]);
-		rhs_he(P, s, yn, k7, q7);
-		for (int i = 0; i < 4; i++)
-			e[i] = h * (e1 * k1[i] + e3 * k3[i] + e4 * k4[i] + e5 * k5[i] + e6 * k6[i] + e7 * k7[i]);
-		const double err = he_err_norm(e, x, yn, atol3, DP_RTOL);
-		if (err <= 1.0) {
-			t += h;
-			for (int i = 0; i < 4; i++) {
-				x[i] = yn[i];
-				k1[i] = k7[i];
-			}
-			if (REC)
-				for (int i = 0; i < 3; i++) {
-					rec[i] += h * (b1 * r1[i] + b3 * r3[i] + b4 * r4[i] + b5 * r5[i] + b6 * r6[i]);
-					r1[i] = r7[i];
-				}
+	S.h = fmax(h, 1e-8);
+	if (REC)
+#pragma unroll
+		for (int i = 0; i < 3; i++) {
+			S.gain[i] = 0.0;
+			S.r1[i] = r1[i];
 		}
-		const double fac = err > 0.0 ? fmin(5.0, fmax(0.2, 0.9 * pow(err, -0.2))) : 5.0;
-		h = fmax(h * fac, 1e-14);
+}
+
+// One pass over the lanes' next work: for fresh lanes the slope at x first,
+// then for all lanes one attempted step. fresh must be the warp's when other
+// lanes call too: anyfresh says whether any lane's is set.
+template <bool REC>
+__device__ __forceinline__ void he_dp_step(const PhysParams &P, const HeCtx &c, HeDp &S, bool fresh, bool anyfresh,
+		double *k, int stride) {
+	double e[4], y[4], q[3], h = 0.0;
+#pragma unroll 1
+	for (int st = anyfresh ? -1 : 0; st < 6; st++) {
+		if (st < 0 && !fresh) continue;
+		if (st <= 0) {
+			if (st == 0) {
+				if (S.t + S.h > 1.0) S.h = 1.0 - S.t;
+				h = S.h;
+			}
+#pragma unroll
+			for (int i = 0; i < 4; i++) y[i] = S.x[i];
+			if (REC)
+#pragma unroll
+				for (int i = 0; i < 3; i++) q[i] = kHeA[5][0] * S.r1[i];
+		}
+		if (st >= 0) {
+#pragma unroll
+			for (int i = 0; i < 4; i++) {
+				const double k1 = k[i * stride];
+				double s = kHeA[st][0] * k1;
+				if (st == 5) e[i] = kHeE[0] * k1;
+#pragma unroll
+				for (int j = 1; j < 6; j++)
+					if (j <= st && (st < 5 || j != 1)) {
+						const double kj = k[(4 * j + i) * stride];
+						s += kHeA[st][j] * kj;
+						if (st == 5) e[i] += kHeE[j] * kj;
+					}
+				y[i] = S.x[i] + h * s;
+			}
+		}
+		double dx[4], r[3];
+		rhs_he(P, c, y, dx, REC ? r : nullptr);
+		if (st < 0) {
+			he_dp_start<REC>(S, dx, r, k, stride);
+		} else if (st < 5) {
+#pragma unroll
+			for (int i = 0; i < 4; i++) k[(4 * (st + 1) + i) * stride] = dx[i];
+			if (REC && st > 0)
+#pragma unroll
+				for (int i = 0; i < 3; i++) q[i] += kHeA[5][st + 1] * r[i];
+		} else {
+#pragma unroll
+			for (int i = 0; i < 4; i++) e[i] = h * (e[i] + (-1. / 40) * dx[i]);
+			const double err = he_err_norm(e, S.x, y, S.atol3, DP_RTOL);
+			if (err <= 1.0) {
+				S.t += h;
+#pragma unroll
+				for (int i = 0; i < 4; i++) {
+					S.x[i] = y[i];
+					k[i * stride] = dx[i];
+				}
+				if (REC)
+#pragma unroll
+					for (int i = 0; i < 3; i++) {
+						S.gain[i] += h * q[i];
+						S.r1[i] = r[i];
+					}
+			}
+			const double fac = err > 0.0 ? fmin(5.0, fmax(0.2, 0.9 * pow(err, -0.2))) : 5.0;
+			S.h = fmax(h * fac, 1e-14);
+			S.steps++;
+		}
 	}
-	*t_out = t;
-	*h_out = h;
-	return t >= 1.0;
+}
+
+// Up to HE_SWITCH steps from s = 0 on one thread; returns true once s = 1
+// is reached, else leaves the time reached and the next step size in *t_out,
+// *h_out. With rec, rec[3] accumulates the recombination photons.
+template <bool REC>
+__device__ inline bool dopri_he_explicit(const PhysParams &P, const HeCtx &c, double x[4], double *rec,
+		double *t_out, double *h_out) {
+	double k[24];
+	HeDp S;
+#pragma unroll
+	for (int i = 0; i < 4; i++) S.x[i] = x[i];
+	bool fresh = true;
+	do {
+		he_dp_step<REC>(P, c, S, fresh, fresh, k, 1);
+		fresh = false;
+	} while (S.t < 1.0 && S.steps < HE_SWITCH);
+#pragma unroll
+	for (int i = 0; i < 4; i++) x[i] = S.x[i];
+	if (REC)
+#pragma unroll
+		for (int i = 0; i < 3; i++) rec[i] += S.gain[i];
+	*t_out = S.t;
+	*h_out = S.h;
+	return S.t >= 1.0;
 }
 
 // Dormand-Prince 5(4) over the four variables, then the Rosenbrock finish.

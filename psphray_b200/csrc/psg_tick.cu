@@ -1569,82 +1569,148 @@ __global__ void __launch_bounds__(256) k_sum_he(int t, const int32_t *__restrict
 	}
 }
 
+// The step of active pair a (particle p) from its sums and the particle's
+// state; x the four variables at its start.
+struct HeSrc {
+	const uint32_t *act_ipar;
+	const double *g0, *g1, *g2, *heat;
+	const double *lambdaH;
+	const float *ie, *rho, *yeMET;
+	const int64_t *lasthit;
+};
+__device__ __forceinline__ HeStep load_he_step(const PhysParams &P, const HeSrc &src, int a, uint32_t p, int64_t tick,
+		double tick_time, double x[4]) {
+	HeStep s;
+	s.yeMET = (double)src.yeMET[p];
+	s.gHI = src.g0[a];
+	s.gHeI = src.g1[a];
+	s.gHeII = src.g2[a];
+	s.heat = src.heat[a];
+	s.time = (double)(tick - src.lasthit[p]) * tick_time;
+	s.nH = P.H_PER_MASS * (double)src.rho[p];
+	x[0] = src.lambdaH[p];
+	x[1] = P.lamHeI[p];
+	x[2] = P.lamHeII[p];
+	x[3] = (double)src.ie[p];
+	s.T = ieye2T(P, x[3], ye_he(P, x[0], x[1], x[2]));     // psys_T()
+	return s;
+}
+
+// update_pars() with helium: explicit steps, one attempted step per
+// iteration and lane. A lane whose particle is done takes the next one of
+// the tick, so that the warp stays full (particles take 1 to 32 steps, 1.7
+// on average on the 2M-particle field: a thread per particle kept half the
+// lanes waiting for the warp's slowest), and the stages' slopes live in
+// shared memory (see HeDp). A particle still unfinished after the explicit
+// steps goes to k_update_he_stiff.
+#define HEQ_THREADS 128
+#define HEQ_BLOCKS 5
 template <bool REC>
-__global__ void __launch_bounds__(128, 4) k_update_he(int t, const int32_t *__restrict__ tick_act,
-		const uint32_t *__restrict__ act_ipar, const double *__restrict__ sum_g0, const double *__restrict__ sum_g1,
-		const double *__restrict__ sum_g2, const double *__restrict__ sum_heat, double *__restrict__ lambdaH,
-		float *__restrict__ ie,
-		int64_t *__restrict__ lasthit, const float *__restrict__ rho, const float *__restrict__ yeMET, PhysParams P,
-		const PsgBatchDev *__restrict__ B, HeStiffItem *__restrict__ stiff, unsigned *__restrict__ nstiff,
-		uint32_t *__restrict__ status) {
+__global__ void __launch_bounds__(HEQ_THREADS, HEQ_BLOCKS) k_update_he(int t, const int32_t *__restrict__ tick_act,
+		const HeSrc src, double *__restrict__ lambdaH, float *__restrict__ ie, int64_t *__restrict__ lasthit,
+		PhysParams P, const PsgBatchDev *__restrict__ B, unsigned *__restrict__ cursor,
+		HeStiffItem *__restrict__ stiff, unsigned *__restrict__ nstiff, uint32_t *__restrict__ status) {
+	__shared__ double slopes[24 * HEQ_THREADS];
+	double *k = slopes + threadIdx.x;
+	const int64_t tick = B->tick0 + t;
+	const double tick_time = B->tick_time;
+	const int lo = tick_act[t], n = tick_act[t + 1] - lo;
+	const int lane = threadIdx.x & 31;
+	bool have = false, dry = false;
+	int a = 0;
+	uint32_t p = 0, st = 0;
+	HeDp S;
+	HeCtx cx;
+	for (;;) {
+		const unsigned need = __ballot_sync(0xffffffffu, !have && !dry);
+		bool fresh = false;
+		if (need) {
+			unsigned base = 0;
+			if (lane == __ffs(need) - 1) base = atomicAdd(cursor, (unsigned)__popc(need));
+			base = __shfl_sync(0xffffffffu, base, __ffs(need) - 1);
+			if (!have && !dry) {
+				const unsigned i = base + (unsigned)__popc(need & ((1u << lane) - 1u));
+				if (i < (unsigned)n) {
+					a = lo + (int)i;
+					p = src.act_ipar[a];
+					cx = make_he_ctx(load_he_step(P, src, a, p, tick, tick_time, S.x));
+					have = fresh = true;
+				} else {
+					dry = true;
+				}
+			}
+		}
+		if (!__any_sync(0xffffffffu, have)) break;
+		const bool anyfresh = __any_sync(0xffffffffu, fresh);
+		if (have) {
+			he_dp_step<REC>(P, cx, S, fresh, anyfresh, k, HEQ_THREADS);
+			double rec[3] = {0.0, 0.0, 0.0};
+			if (S.t >= 1.0 || S.steps >= HE_SWITCH) {
+				have = false;
+				if (REC) {
+					rec[0] = (double)P.ygrec[p] + S.gain[0];
+					rec[1] = (double)P.ygrecHe1[p] + S.gain[1];
+					rec[2] = (double)P.ygrecHe2[p] + S.gain[2];
+				}
+				if (S.t >= 1.0) {
+					if (!(S.x[3] >= 0.0)) st |= PSG_ST_IE_NEG;
+					for (int i = 0; i < 4; i++)
+						if (!isfinite(S.x[i])) st |= PSG_ST_NAN;
+					clamp_he(S.x);
+					for (int i = 0; i < 3; i++) rec[i] = fmax(0.0, rec[i]);
+					he_write(P, p, S.x, rec, cx.T, tick, lambdaH, ie, lasthit);
+				} else {
+					double x0[4];
+					HeStiffItem it;
+					it.s = load_he_step(P, src, a, p, tick, tick_time, x0);
+					for (int i = 0; i < 4; i++) it.x[i] = S.x[i];
+					for (int i = 0; i < 3; i++) it.rec[i] = rec[i];
+					it.t = S.t;
+					it.h = S.h;
+					it.p = p;
+					stiff[atomicAdd(nstiff, 1u)] = it;
+				}
+			}
+		}
+	}
+	if (st) atomicOr(status, st);
+}
+
+// update_pars() with helium and step_evolve_euler(), a thread per active
+// particle: no clamps there; update_pars() clamps (loop.c:759-761) and keeps
+// the unused photons (loop.c:745-747).
+__global__ void __launch_bounds__(128) k_update_he_euler(int t, const int32_t *__restrict__ tick_act, const HeSrc src,
+		double *__restrict__ lambdaH, float *__restrict__ ie, int64_t *__restrict__ lasthit, PhysParams P,
+		const PsgBatchDev *__restrict__ B, uint32_t *__restrict__ status) {
 	const int64_t tick = B->tick0 + t;
 	const double tick_time = B->tick_time;
 	const int hi = tick_act[t + 1];
+	uint32_t st = 0;
 	for (int a = tick_act[t] + (int)(blockIdx.x * blockDim.x + threadIdx.x); a < hi;
 			a += (int)(gridDim.x * blockDim.x)) {
-	double g0 = sum_g0[a], g1 = sum_g1[a], g2 = sum_g2[a];
-	const double heat = sum_heat[a];
-	const uint32_t p = act_ipar[a];
-	if (P.euler) {      // photons left over by an earlier explicit step (loop.c:745-747)
-		g0 += P.gcarry[p];
-		g1 += P.gcarryHe1[p];
-		g2 += P.gcarryHe2[p];
-	}
-	HeStep s;
-	s.yeMET = (double)yeMET[p];
-	s.gHI = g0;
-	s.gHeI = g1;
-	s.gHeII = g2;
-	s.heat = heat;
-	s.time = (double)(tick - lasthit[p]) * tick_time;
-	s.nH = P.H_PER_MASS * (double)rho[p];
-	const double ie0 = (double)ie[p];
-	s.T = ieye2T(P, ie0, ye_he(P, lambdaH[p], P.lamHeI[p], P.lamHeII[p]));     // psys_T()
-	double x[4] = {lambdaH[p], P.lamHeI[p], P.lamHeII[p], ie0};
-	double rec[3] = {0.0, 0.0, 0.0};
-	if (P.ygrec) {
-		rec[0] = (double)P.ygrec[p];
-		rec[1] = (double)P.ygrecHe1[p];
-		rec[2] = (double)P.ygrecHe2[p];
-	}
-	uint32_t st = 0;
-	if (P.euler) {
-		// step_evolve_euler(): no clamps there; update_pars() clamps
-		// (loop.c:759-761) and keeps the unused photons (loop.c:745-747)
-		double remain = 0.0, gain[3] = {0.0, 0.0, 0.0};
+		const uint32_t p = src.act_ipar[a];
+		double x[4];
+		HeStep s = load_he_step(P, src, a, p, tick, tick_time, x);
+		s.gHI += P.gcarry[p];      // photons left over by an earlier explicit step
+		s.gHeI += P.gcarryHe1[p];
+		s.gHeII += P.gcarryHe2[p];
+		double rec[3] = {0.0, 0.0, 0.0}, remain = 0.0, gain[3] = {0.0, 0.0, 0.0};
 		int refined = 0;
-		st = euler_he(P, s, x, remain, refined, P.ygrec ? gain : nullptr);
-		if (P.ygrec)
-			for (int k = 0; k < 3; k++) rec[k] += gain[k];
+		st |= euler_he(P, s, x, remain, refined, P.ygrec ? gain : nullptr);
+		if (P.ygrec) {
+			rec[0] = (double)P.ygrec[p] + gain[0];
+			rec[1] = (double)P.ygrecHe1[p] + gain[1];
+			rec[2] = (double)P.ygrecHe2[p] + gain[2];
+		}
 		x[0] = fmax(0.0, fmin(1.0, x[0]));
 		x[1] = fmax(0.0, fmin(1.0, x[1]));
 		x[2] = fmax(0.0, fmin(1.0 - x[1], x[2]));
-		P.gcarry[p] = g0 * remain;
-		P.gcarryHe1[p] = g1 * remain;
-		P.gcarryHe2[p] = g2 * remain;
-	} else {
-		double gain[3] = {0.0, 0.0, 0.0}, tt = 0.0, hh = 0.0;
-		if (!dopri_he_explicit<REC>(P, make_he_ctx(s), x, gain, &tt, &hh)) {
-			HeStiffItem it;
-			it.s = s;
-			for (int k = 0; k < 4; k++) it.x[k] = x[k];
-			for (int k = 0; k < 3; k++) it.rec[k] = rec[k] + gain[k];
-			it.t = tt;
-			it.h = hh;
-			it.p = p;
-			stiff[atomicAdd(nstiff, 1u)] = it;
-			continue;
-		}
-		if (!(x[3] >= 0.0)) st |= PSG_ST_IE_NEG;
-		for (int k = 0; k < 4; k++)
-			if (!isfinite(x[k])) st |= PSG_ST_NAN;
-		clamp_he(x);
-		if (P.ygrec)
-			for (int k = 0; k < 3; k++) rec[k] = fmax(0.0, rec[k] + gain[k]);
+		P.gcarry[p] = s.gHI * remain;
+		P.gcarryHe1[p] = s.gHeI * remain;
+		P.gcarryHe2[p] = s.gHeII * remain;
+		he_write(P, p, x, rec, s.T, tick, lambdaH, ie, lasthit);
 	}
-	he_write(P, p, x, rec, s.T, tick, lambdaH, ie, lasthit);
 	if (st) atomicOr(status, st);
-	}
 }
 
 // The stiff helium particles of a tick (as k_update_stiff): the Rosenbrock
@@ -2056,7 +2122,8 @@ int plan_batch(psg_context *ctx, size_t R, size_t K, const PsgTraceFill &tf, Bat
 	pl.queue_grid = pl.queue_minb == 4 ? occ_grid(ctx, k_update_queue<false, 4>, 32 * UPD_WARPS)
 			: pl.queue_minb == 3 ? occ_grid(ctx, k_update_queue<false, 3>, 32 * UPD_WARPS)
 			: occ_grid(ctx, k_update_queue<false, 1>, 32 * UPD_WARPS);
-	pl.he_grid = occ_grid(ctx, k_update_he<false>, 128);
+	pl.he_grid = pl.euler ? occ_grid(ctx, k_update_he_euler, 128) : ctx->flags.on_the_spot
+			? occ_grid(ctx, k_update_he<false>, HEQ_THREADS) : occ_grid(ctx, k_update_he<true>, HEQ_THREADS);
 	pl.stiff_grid = pl.helium ? (ctx->flags.on_the_spot ? occ_grid(ctx, k_update_he_stiff<false>, STIFF_THREADS)
 			: occ_grid(ctx, k_update_he_stiff<true>, STIFF_THREADS)) : occ_grid(ctx, k_update_stiff<true>, STIFF_THREADS);
 	pl.euler_grid = occ_grid(ctx, k_update_euler, 128);
@@ -2188,14 +2255,22 @@ int enqueue_batch(psg_context *ctx, const BatchPlan &pl, const PsgBatchDev *B) {
 					(uint32_t)ctx->tune.run_short, pl.want_heat, long_act, tick_long, ctx->d_hits, uv.act_g, g1, g2, uv.act_heat);
 			PSG_CHECK_LAUNCH();
 			ctx->launches++;
+			const HeSrc hs{av.act_ipar, uv.act_g, g1, g2, uv.act_heat, ctx->d_lambdaH, ctx->d_ie, ctx->d_rho,
+					ctx->d_yeMET, ctx->d_lasthit};
+			if (pl.euler) {
+				k_update_he_euler<<<pl.he_grid, 128, 0, st>>>((int)t, av.tick_act, hs, ctx->d_lambdaH, ctx->d_ie,
+						ctx->d_lasthit, P, B, ctx->d_status);
+				PSG_CHECK_LAUNCH();
+				ctx->launches++;
+				psg_mark_end(ctx);
+				continue;
+			}
 			if (P.ygrec)
-				k_update_he<true><<<pl.he_grid, 128, 0, st>>>((int)t, av.tick_act, av.act_ipar, uv.act_g, g1, g2,
-						uv.act_heat, ctx->d_lambdaH, ctx->d_ie, ctx->d_lasthit, ctx->d_rho,
-						ctx->d_yeMET, P, B, hstiff, uv.nstiff + t, ctx->d_status);
+				k_update_he<true><<<pl.he_grid, HEQ_THREADS, 0, st>>>((int)t, av.tick_act, hs, ctx->d_lambdaH, ctx->d_ie,
+						ctx->d_lasthit, P, B, uv.cursors + t, hstiff, uv.nstiff + t, ctx->d_status);
 			else
-				k_update_he<false><<<pl.he_grid, 128, 0, st>>>((int)t, av.tick_act, av.act_ipar, uv.act_g, g1, g2,
-						uv.act_heat, ctx->d_lambdaH, ctx->d_ie, ctx->d_lasthit, ctx->d_rho,
-						ctx->d_yeMET, P, B, hstiff, uv.nstiff + t, ctx->d_status);
+				k_update_he<false><<<pl.he_grid, HEQ_THREADS, 0, st>>>((int)t, av.tick_act, hs, ctx->d_lambdaH, ctx->d_ie,
+						ctx->d_lasthit, P, B, uv.cursors + t, hstiff, uv.nstiff + t, ctx->d_status);
 			PSG_CHECK_LAUNCH();
 			if (P.ygrec)
 				k_update_he_stiff<true><<<pl.stiff_grid, STIFF_THREADS, 0, st>>>(hstiff, uv.nstiff + t, uv.stiff_ctr + t,
