@@ -235,8 +235,8 @@ typedef struct {
 	int trace_warps;        /* warps per traversal block, 1-16 (default 4) */
 	int deposit_long;       /* rays with more hits than this take a 128-thread group (default 96) ... */
 	int deposit_mid;        /* ... more than this a 512-thread block (default 384); fewer take a warp */
-	int update_minblocks;   /* 3 or 4: the integrator's registers capped for that many resident
-	                         * blocks per multiprocessor (spilling the rest); 1: uncapped (default) */
+	int update_minblocks;   /* 1 (default), 3 or 4, accepted and kept; the integrator has one register
+	                         * budget (a block per multiprocessor) and runs the same for each */
 	int leaf_size;          /* particles per octree leaf: the reference's CFG_OCTTREE_PPC, 8; the hit
 	                         * lists are bit-exact only with the reference's leaves, so it is reported,
 	                         * never searched */
@@ -252,8 +252,8 @@ int psg_set_tune(psg_context *ctx, const psg_tune *tune);
 int psg_get_tune(psg_context *ctx, psg_tune *tune);
 /* Times candidate shapes on one batch of the caller's device rays (R rays
  * per tick, K ticks, as psg_run_ticks_device), each `reps` times, one
- * dimension after another (traversal warps, deposit thresholds, integrator
- * registers, short-run threshold, integrator order), and keeps the fastest. The particle state is restored after
+ * dimension after another (traversal warps, deposit thresholds, short-run
+ * threshold, integrator order), and keeps the fastest. The particle state is restored after
  * every trial, so the call does not advance the run. The result becomes the
  * context's shapes and the device's cached shapes, which contexts created
  * later on that device start from. *best_ms: the kept shape's batch time. */

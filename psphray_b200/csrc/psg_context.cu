@@ -113,6 +113,7 @@ extern "C" void psg_destroy(psg_context *ctx) {
 	free_tree(ctx);
 	if (ctx->d_ar) cudaFree(ctx->d_ar);
 	if (ctx->d_ar_ni) cudaFree(ctx->d_ar_ni);
+	if (ctx->d_ar_win) cudaFree(ctx->d_ar_win);
 	if (ctx->d_ar_he) cudaFree(ctx->d_ar_he);
 	if (ctx->d_xs) cudaFree(ctx->d_xs);
 	if (ctx->d_kernel) cudaFree(ctx->d_kernel);
@@ -259,11 +260,13 @@ extern "C" int psg_set_physics(psg_context *ctx, const psg_units *u, const psg_r
 	PSG_CUDA(cudaSetDevice(ctx->device));
 	if (ctx->d_ar) cudaFree(ctx->d_ar);
 	if (ctx->d_ar_ni) cudaFree(ctx->d_ar_ni);
+	if (ctx->d_ar_win) cudaFree(ctx->d_ar_win);
 	if (ctx->d_ar_he) cudaFree(ctx->d_ar_he);
 	if (ctx->d_xs) cudaFree(ctx->d_xs);
 	if (ctx->d_kernel) cudaFree(ctx->d_kernel);
 	ctx->d_ar = ctx->d_xs = ctx->d_kernel = nullptr;
 	ctx->d_ar_ni = nullptr;
+	ctx->d_ar_win = nullptr;
 	ctx->d_ar_he = nullptr;
 	// rows of 16 doubles (one 128-byte line): log T, then the 15 rate columns
 	const size_t nr = (size_t)ar->nrows;
@@ -309,8 +312,22 @@ extern "C" int psg_set_physics(psg_context *ctx, const psg_units *u, const psg_r
 			}
 		cudaError_t e2 = cudaMalloc(&ctx->d_ar_ni, sizeof(float) * nr * 16);
 		if (e2 == cudaSuccess) e2 = cudaMemcpy(ctx->d_ar_ni, ni, sizeof(float) * nr * 16, cudaMemcpyHostToDevice);
+		// the integrator's window of them, a row every 80 bytes
+		const double w0 = (PSG_WIN_LOGT - ar->min) * ar->step_inv;
+		const int lo = w0 > 0.0 ? (int)fmin(w0, (double)(nr - 1)) : 0, nwin = (int)std::min<size_t>(PSG_WIN_ROWS, nr - lo);
+		float *win = (float *)calloc((size_t)nwin * 20, sizeof(float));
+		if (e2 == cudaSuccess && win) {
+			for (int j = 0; j < nwin; j++) memcpy(win + 20 * (size_t)j, ni + 16 * (size_t)(lo + j), 16 * sizeof(float));
+			e2 = cudaMalloc(&ctx->d_ar_win, sizeof(float) * 20 * nwin);
+			if (e2 == cudaSuccess) e2 = cudaMemcpy(ctx->d_ar_win, win, sizeof(float) * 20 * nwin, cudaMemcpyHostToDevice);
+		}
+		const bool host_ok = win != nullptr;
+		free(win);
 		free(ni);
 		PSG_CUDA(e2);
+		if (!host_ok) return psg_fail(ctx, PSG_E_NOMEM, "psg_set_physics: host allocation failed");
+		ctx->ar_win_lo = lo;
+		ctx->ar_win_n = nwin;
 	}
 	// The helium right-hand side's columns in the same FP32 value and slope
 	// form: a (value, slope) pair per column, so a 16-byte load brings two

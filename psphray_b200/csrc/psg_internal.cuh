@@ -18,6 +18,11 @@
 // take the library segmented sort.
 #define PSG_SORT_MAX 8192
 
+// The rate rows the integrator keeps in shared memory: those from this log T
+// on, so many of them (up to log T = 8 with the reference's table; 100 KB).
+#define PSG_WIN_LOGT 3.0
+#define PSG_WIN_ROWS 1250
+
 // Columns of the helium right-hand side's rate rows, two to a 16-byte load:
 // what case B (on the spot) reads comes first, case A's further ones after it.
 enum {
@@ -32,6 +37,7 @@ enum {
 #define PSG_ST_IE_NEG 4u       // internal energy would turn negative (solve.c:137-139)
 #define PSG_ST_STACK 8u        // traversal stack overflow
 #define PSG_ST_SURR 16u        // a surrogate tile's tensor-core step did not complete
+#define PSG_ST_COPY 64u        // a block's copy of the rate rows did not end
 #define PSG_ST_SLAB 32u        // a hit list outgrew its slab in a call without host reads (redone)
 
 // scratch slots
@@ -71,6 +77,8 @@ struct psg_context {
 	double *d_ar = nullptr;      // [ar_nrows][16]: logT, then the PSG_AR_* columns
 	float4 *d_ar_ni = nullptr;   // [ar_nrows][4]: the 7 rates of the non-isothermal
 	                             // right-hand side, values then slopes per log T
+	float4 *d_ar_win = nullptr;  // [ar_win_n][5]: the rows from log T = 3 on that the integrator copies to shared memory
+	int ar_win_lo = 0, ar_win_n = 0;
 	double ar_step = 0;
 	double ar_ni_scale[8] = {};  // each d_ar_ni column is stored divided by this
 	float4 *d_ar_he = nullptr;   // [ar_nrows][8]: the helium right-hand side's columns (PSG_HE_*), (value, slope) pairs

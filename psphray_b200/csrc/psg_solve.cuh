@@ -35,6 +35,8 @@ struct PhysParams {
 	const float4 *ar_ni;   // [ar_nrows][4]: the right-hand side's 7 rates (+ alpha_B when not
 	                       // on the spot), values and slopes
 	double ar_ni_scale[8]; // ... each column divided by its largest magnitude
+	const float4 *ar_win;  // [ar_win_n][5]: rows [ar_win_lo, ar_win_lo + ar_win_n) of ar_ni, spaced for shared memory
+	int ar_win_lo, ar_win_n;
 	const float4 *ar_he;   // [ar_nrows][8]: the helium right-hand side's columns, (value, slope) pairs
 	double ar_he_scale[PSG_HE_NCOLS];   // ... each column divided by its largest magnitude
 	int ar_nrows;
@@ -191,6 +193,66 @@ __device__ __forceinline__ RhsCtx make_rhs_ctx(const PhysParams &P, double yeMET
 	return c;
 }
 
+// Where the right-hand side's rate rows come from: device memory, or a copy
+// of the rows around the usual temperatures in shared memory. The lanes of a
+// warp read rows of their own, and L1 looks up one 128-byte line a cycle:
+// from device memory a row costs a warp four loads of up to 32 lines each.
+// Shared memory serves eight lanes at a time from 16-byte banks; rows spaced
+// five of them apart spread over all eight.
+struct RateRows {
+	__device__ __forceinline__ void get(const PhysParams &P, int idx, float4 v[4]) const {
+		const float4 *row = P.ar_ni + 4 * (size_t)idx;
+#pragma unroll
+		for (int c = 0; c < 4; c++) v[c] = row[c];
+	}
+};
+struct RateWindow {
+	const float4 *sm;
+	int lo, n;
+	// One thread starts the copy (P.ar_win holds the rows as spaced here)
+	// into buf and arms bar; every thread waits for it before its first row.
+	__device__ __forceinline__ void start(const PhysParams &P, float4 *buf, uint64_t *bar) {
+		sm = buf;
+		lo = P.ar_win_lo;
+		n = P.ar_win_n;
+		if (threadIdx.x == 0) {
+			const uint32_t b = (uint32_t)__cvta_generic_to_shared(bar), d = (uint32_t)__cvta_generic_to_shared(buf);
+			const uint32_t bytes = (uint32_t)n * (5 * sizeof(float4));
+			asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(b) : "memory");
+			asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+			asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"(bytes) : "memory");
+			if (bytes)
+				asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(d),
+						"l"(P.ar_win), "r"(bytes), "r"(b)
+						: "memory");
+		}
+		__syncthreads();      // (the barrier is armed before anyone waits on it)
+	}
+	// false if the copy did not end within the limit (it takes microseconds)
+	__device__ __forceinline__ bool wait(uint64_t *bar) const {
+		const uint32_t b = (uint32_t)__cvta_generic_to_shared(bar);
+		for (int i = 0; i < (1 << 22); i++) {
+			uint32_t done;
+			asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n\t"
+						 "selp.u32 %0, 1, 0, p;\n\t}\n"
+						 : "=r"(done)
+						 : "r"(b)
+						 : "memory");
+			if (done) return true;
+		}
+		return false;
+	}
+	__device__ __forceinline__ void get(const PhysParams &P, int idx, float4 v[4]) const {
+		const unsigned w = (unsigned)(idx - lo);
+		if (w < (unsigned)n) {
+#pragma unroll
+			for (int c = 0; c < 4; c++) v[c] = sm[5 * w + c];
+		} else {
+			RateRows().get(P, idx, v);
+		}
+	}
+};
+
 // function() solve.c:76-141, hydrogen-only branch, for the integrators (not
 // isothermal): the same equations with the step length folded into the
 // rates, and fused multiply-adds (the last bits of an integrator's stage do
@@ -205,9 +267,9 @@ __device__ __forceinline__ RhsCtx make_rhs_ctx(const PhysParams &P, double yeMET
 // is then scaled and combined in FP64, and the state and its derivatives
 // stay FP64. Without it (finite-difference Jacobians, residual checks, the
 // explicit build's steps) the lookup is FP64.
-template <bool REC = false, bool T32 = false>
+template <bool REC = false, bool T32 = false, typename ROWS = RateRows>
 __device__ __forceinline__ void rhs(const PhysParams &P, const RhsCtx &cx, const double x[2], double dx[2],
-		double *rec = nullptr) {
+		double *rec = nullptr, const ROWS &rows = ROWS()) {
 	const double xHI = x[0], xHII = 1.0 - x[0];
 	const double ye = xHII + P.he_e + cx.yeMET;
 	// the row of tabfun_get() and the offset into it (clamped rows, a NaN
@@ -240,7 +302,8 @@ __device__ __forceinline__ void rhs(const PhysParams &P, const RhsCtx &cx, const
 			du = logT - __fma_rn((double)idx, P.ar_step, P.ar_min);
 		}
 	}
-	const float4 *row = P.ar_ni + 4 * idx;
+	float4 row[4];
+	rows.get(P, (int)idx, row);
 	const float4 v0 = row[0], v1 = row[1], s0 = row[2], s1 = row[3];
 #define PSG_LIN(v, s, c)                                                                                  \
 	((T32 ? (double)__fmaf_rn((s), duf, (v)) : __fma_rn((double)(s), du, (double)(v))) * P.ar_ni_scale[c])
@@ -264,57 +327,47 @@ __device__ __forceinline__ void rhs(const PhysParams &P, const RhsCtx &cx, const
 }
 
 // Adaptive Dormand-Prince 5(4) over s in [0,1]. LSODA runs the reference at
-// rtol 1e-4 (solve.c:151-152); 1e-6 here. The state of one integration is a
-// DPState; dp_init() evaluates the first derivative and picks the first step
-// (about a 1% change of each component, components near zero measured
-// against atol/rtol), dp_step() attempts one step.
-struct DPState {
-	double x[2], k1[2];
-	double rec, krec;   // REC: yGrecHII gained so far, and its derivative at x
-	double t, h;
-	float hnext;     // proposal for a step beyond s = 1 (the interval end truncates h)
-	int steps;
-};
-
+// rtol 1e-4 (solve.c:151-152); 1e-6 here.
 #define DP_RTOL 1e-6
 #define DP_ATOL0 1e-10
 #define DP_ATOL1_REL 1e-8
 
-// First step from the derivative S.k1 = f(S.x), already evaluated.
-__device__ __forceinline__ void dp_init_k1(DPState &S) {
-	S.t = 0.0;
-	S.steps = 0;
-	double h = 1.0;
-	const double atol1 = DP_ATOL1_REL * fabs(S.x[1]) + 1e-300;
-	for (int i = 0; i < 2; i++) {
-		const double scale = fabs(S.x[i]) + (i == 0 ? DP_ATOL0 : atol1) / DP_RTOL;
-		const double f = fabs(S.k1[i]);
-		if (f > 0.0) h = fmin(h, 0.01 * scale / f);
-	}
-	S.h = fmax(h, 1e-8);
-	S.hnext = 0.0f;
-}
+// One integration: its state between attempted steps.
+struct DPState {
+	double x[2], k1[2];
+	double rec, krec;   // REC: yGrecHII gained so far, and its derivative at x
+	double t, h, atol1;
+	float hnext;     // proposal for a step beyond s = 1 (the interval end truncates h)
+	int steps;
+};
 
-template <bool REC = false>
-__device__ __forceinline__ void dp_init(const PhysParams &P, const RhsCtx &cx, DPState &S) {
-	S.rec = 0.0;
-	rhs<REC, true>(P, cx, S.x, S.k1, &S.krec);
+// The integration's start: the slope at x and the first step (h0 if
+// positive, else about a 1% change of each component, components near zero
+// measured against atol/rtol).
+template <bool REC, typename ROWS>
+__device__ __forceinline__ void dp_start(const PhysParams &P, const RhsCtx &cx, DPState &S, double h0, const ROWS &rows) {
 	S.t = 0.0;
 	S.steps = 0;
+	S.rec = 0.0;
+	S.hnext = 0.0f;
+	S.atol1 = DP_ATOL1_REL * fabs(S.x[1]) + 1e-300;
+	rhs<REC, true>(P, cx, S.x, S.k1, &S.krec, rows);
+	if (h0 > 0.0) {
+		S.h = fmin(1.0, fmax(h0, 1e-8));
+		return;
+	}
 	double h = 1.0;
-	const double atol1 = DP_ATOL1_REL * fabs(S.x[1]) + 1e-300;
 	for (int i = 0; i < 2; i++) {
-		const double scale = fabs(S.x[i]) + (i == 0 ? DP_ATOL0 : atol1) / DP_RTOL;
+		const double scale = fabs(S.x[i]) + (i == 0 ? DP_ATOL0 : S.atol1) / DP_RTOL;
 		const double f = fabs(S.k1[i]);
 		if (f > 0.0) h = fmin(h, 0.01 * scale / f);
 	}
 	S.h = fmax(h, 1e-8);
-	S.hnext = 0.0f;
 }
 
 // One attempted step; returns true once s = 1 is reached.
-template <bool REC = false>
-__device__ __forceinline__ bool dp_step(const PhysParams &P, const RhsCtx &cx, DPState &S, double atol1) {
+template <bool REC, typename ROWS>
+__device__ __forceinline__ bool dp_step(const PhysParams &P, const RhsCtx &cx, DPState &S, const ROWS &rows) {
 	const double a21 = 1. / 5, a31 = 3. / 40, a32 = 9. / 40, a41 = 44. / 45, a42 = -56. / 15, a43 = 32. / 9;
 	const double a51 = 19372. / 6561, a52 = -25360. / 2187, a53 = 64448. / 6561, a54 = -212. / 729;
 	const double a61 = 9017. / 3168, a62 = -355. / 33, a63 = 46732. / 5247, a64 = 49. / 176, a65 = -5103. / 18656;
@@ -328,22 +381,22 @@ __device__ __forceinline__ bool dp_step(const PhysParams &P, const RhsCtx &cx, D
 	const double *x = S.x, *k1 = S.k1;
 #define F __fma_rn
 	for (int i = 0; i < 2; i++) y[i] = F(h, a21 * k1[i], x[i]);
-	rhs<REC, true>(P, cx, y, k2, &r2);
+	rhs<REC, true>(P, cx, y, k2, &r2, rows);
 	for (int i = 0; i < 2; i++) y[i] = F(h, F(a32, k2[i], a31 * k1[i]), x[i]);
-	rhs<REC, true>(P, cx, y, k3, &r3);
+	rhs<REC, true>(P, cx, y, k3, &r3, rows);
 	for (int i = 0; i < 2; i++) y[i] = F(h, F(a43, k3[i], F(a42, k2[i], a41 * k1[i])), x[i]);
-	rhs<REC, true>(P, cx, y, k4, &r4);
+	rhs<REC, true>(P, cx, y, k4, &r4, rows);
 	for (int i = 0; i < 2; i++) y[i] = F(h, F(a54, k4[i], F(a53, k3[i], F(a52, k2[i], a51 * k1[i]))), x[i]);
-	rhs<REC, true>(P, cx, y, k5, &r5);
+	rhs<REC, true>(P, cx, y, k5, &r5, rows);
 	for (int i = 0; i < 2; i++)
 		y[i] = F(h, F(a65, k5[i], F(a64, k4[i], F(a63, k3[i], F(a62, k2[i], a61 * k1[i])))), x[i]);
-	rhs<REC, true>(P, cx, y, k6, &r6);
+	rhs<REC, true>(P, cx, y, k6, &r6, rows);
 	for (int i = 0; i < 2; i++) yn[i] = F(h, F(b6, k6[i], F(b5, k5[i], F(b4, k4[i], F(b3, k3[i], b1 * k1[i])))), x[i]);
-	rhs<REC, true>(P, cx, yn, k7, &r7);
+	rhs<REC, true>(P, cx, yn, k7, &r7, rows);
 	double err = 0.0;
 	for (int i = 0; i < 2; i++) {
 		const double e = h * F(e7, k7[i], F(e6, k6[i], F(e5, k5[i], F(e4, k4[i], F(e3, k3[i], e1 * k1[i])))));
-		const double sc = (i == 0 ? DP_ATOL0 : atol1) + DP_RTOL * fmax(fabs(x[i]), fabs(yn[i]));
+		const double sc = (i == 0 ? DP_ATOL0 : S.atol1) + DP_RTOL * fmax(fabs(x[i]), fabs(yn[i]));
 		err += (e / sc) * (e / sc);
 	}
 #undef F
@@ -508,10 +561,9 @@ __device__ inline bool dopri(const PhysParams &P, const RhsCtx &cx, double x[2],
 	DPState S;
 	S.x[0] = x[0];
 	S.x[1] = x[1];
-	const double atol1 = DP_ATOL1_REL * fabs(x[1]) + 1e-300;
-	dp_init<REC>(P, cx, S);
+	dp_start<REC>(P, cx, S, 0.0, RateRows());
 	bool done = false;
-	while (!done && S.steps < DP_SWITCH) done = dp_step<REC>(P, cx, S, atol1);
+	while (!done && S.steps < DP_SWITCH) done = dp_step<REC>(P, cx, S, RateRows());
 	x[0] = S.x[0];
 	x[1] = S.x[1];
 	if (REC) *rec = S.rec;

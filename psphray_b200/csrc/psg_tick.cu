@@ -34,6 +34,9 @@ PhysParams psg_phys_params(const psg_context *ctx) {
 	P.ar = ctx->d_ar;
 	P.ar_ni = ctx->d_ar_ni;
 	for (int c = 0; c < 8; c++) P.ar_ni_scale[c] = ctx->ar_ni_scale[c];
+	P.ar_win = ctx->d_ar_win;
+	P.ar_win_lo = ctx->ar_win_lo;
+	P.ar_win_n = ctx->ar_win_n;
 	P.ar_he = ctx->d_ar_he;
 	for (int c = 0; c < PSG_HE_NCOLS; c++) P.ar_he_scale[c] = ctx->ar_he_scale[c];
 	P.ar_step = ctx->ar_step;
@@ -932,18 +935,14 @@ __global__ void k_long_place(const int32_t *__restrict__ tick_act, int K, const 
 	}
 }
 
-// One active particle's non-isothermal update, prepared by k_reduce<false>
-// so that the integrator reads one contiguous record instead of gathering
-// the particle's state: the inputs of the step and f(x0) (with the
-// recombination photons' rate when not on the spot). 80 bytes, a multiple
-// of 16 for cp.async.
+// One active particle's explicit-build step, prepared by k_reduce<false> so
+// that k_update_euler reads one contiguous record instead of gathering the
+// particle's state.
 struct __align__(16) UpdRec {
-	double time, lam0, g, heat, k0, k1;
-	float ie0, rho, yeMET, hstep;
-	uint32_t p, pad0;
-	double krec;
+	double time, lam0, g, heat;
+	float ie0, rho, yeMET;
+	uint32_t p;
 };
-static_assert(sizeof(UpdRec) == 80, "UpdRec layout");
 
 // An integration that looks long (the integrator queue claims these first):
 // no step proposal carried over, a proposal under a quarter of the step, or
@@ -982,18 +981,7 @@ __device__ __forceinline__ void finish_particle(int a, double g, double heat, in
 		r.ie0 = ie[p];
 		r.rho = rho[p];
 		r.yeMET = yeMET[p];
-		r.hstep = hstep[p];
 		r.p = p;
-		r.pad0 = 0u;
-		r.krec = 0.0;
-		const double ie0 = (double)r.ie0;
-		const double T = ieye2T(P, ie0, rn_dadd(rn_dsub(1.0, r.lam0), P.he_e));
-		const RhsCtx cx = make_rhs_ctx(P, (double)r.yeMET, g, heat, r.time, rn_dmul(P.H_PER_MASS, (double)r.rho), T);
-		const double x0[2] = {r.lam0, ie0};
-		double f0[2];
-		rhs<REC, true>(P, cx, x0, f0, &r.krec);
-		r.k0 = f0[0];
-		r.k1 = f0[1];
 		rec[a - lo] = r;    // records of one tick, from its first active particle
 		return;
 	}
@@ -1134,7 +1122,7 @@ __device__ __forceinline__ void warp_segment_sum(const double *__restrict__ acc,
 // read in order, shorter ones put in hit order by visit_run). The grid is
 // persistent (both loops stride over the tick's ranges, read on the device).
 template <bool ISO, bool REC>
-__global__ void __launch_bounds__(256) k_reduce(int t, const int32_t *__restrict__ tick_act,
+__global__ void __launch_bounds__(256, ISO && !REC ? 5 : 4) k_reduce(int t, const int32_t *__restrict__ tick_act,
 		const uint32_t *__restrict__ act_ipar, const uint32_t *__restrict__ act_seg,
 		const double *__restrict__ acc, const uint32_t *__restrict__ vals, uint32_t short_max, int want_heat,
 		const uint32_t *__restrict__ long_act, const int32_t *__restrict__ tick_long,
@@ -1187,8 +1175,7 @@ struct StiffItem {
 	double t, h, x0, x1, yeMET, g, heat, time, nH, T, rec;
 	uint32_t p;
 };
-#define UPD_WARPS 8
-// Where the integrator's records come from: the tick's active particles,
+// Where the integrator's inputs come from: the tick's active particles,
 // their summed deposits (act_g, act_heat, from k_reduce) and the particle
 // state.
 struct UpdSrc {
@@ -1198,13 +1185,22 @@ struct UpdSrc {
 	const uint8_t *slow;      // per active pair: claim in the first pass (with cursor2)
 };
 
-// Every warp owns two buffers of 32 records in shared memory: it claims
-// chunks of 32 particles from the tick's cursor and builds their records
-// (the summed deposits, the state, the step length) one chunk ahead, so a
-// lane whose particle is done takes the next one from shared memory; the
-// gathers of a chunk are paid once per 32 particles, not per integrator
-// step, and no record goes through device memory. MINB caps the registers
-// for that many resident blocks per multiprocessor (psg_tune).
+// A warp claims chunks of 32 particles from the tick's cursor; a lane whose
+// particle is done takes the next one of the chunk, and each iteration is
+// one attempted step of every lane (dp_pass).
+//
+// What bounds it: the latency of a right-hand side (an FP64 chain with a
+// logarithm, a division and a rate row in it) at 16 warps per
+// multiprocessor, and before the rate rows came from shared memory L1's line
+// lookups of them (66% of its peak). So one block fills the multiprocessor,
+// at 104 registers (128 with REC), and copies the rate rows of log T 3 to 8
+// beside it once per launch (RateWindow, 100 KB from L2, one bulk copy that
+// the first particles' gathers overlap); a temperature outside reads device
+// memory. Measured, update group per call, rows from device memory -> from
+// shared memory: 2M particles 3.44 -> 2.83 ms (8 ticks), 16.8M 34.5 -> 24.9
+// ms (4 ticks), 1M not on the spot 2.15 -> 1.42 ms (6 ticks). The stages in a
+// loop over slopes in shared memory (64 or 80 registers, 32 or 24 warps)
+// measured slower: 3.58 and 3.22 ms on the 2M field.
 //
 // With cursor2 (psg_tune.update_order) the tick's particles are claimed in
 // two passes: first, from cursor, those that look slow (src.slow, set by
@@ -1215,14 +1211,21 @@ struct UpdSrc {
 // chunk's particles of the pass. Long integrations then start early instead
 // of trailing the kernel on a few lanes. Which lane integrates a particle
 // changes, not its result.
-template <bool REC, int MINB>
-__global__ void __launch_bounds__(32 * UPD_WARPS, MINB) k_update_queue(int t, const int32_t *__restrict__ tick_act,
+#define UPD_THREADS 512
+#define UPD_SMEM (PSG_WIN_ROWS * 5 * 16 + UPD_THREADS + 16)
+template <bool REC>
+__global__ void __launch_bounds__(UPD_THREADS, 1) k_update_queue(int t, const int32_t *__restrict__ tick_act,
 		const UpdSrc src, double *__restrict__ lambdaH, float *__restrict__ ie,
 		int64_t *__restrict__ lasthit, float *__restrict__ hstep, PhysParams P, const PsgBatchDev *__restrict__ B,
 		unsigned *__restrict__ cursor, unsigned *__restrict__ cursor2, StiffItem *__restrict__ stiff,
 		unsigned *__restrict__ nstiff, const uint32_t *__restrict__ alist, const unsigned *__restrict__ nalist,
 		uint32_t *__restrict__ status) {
-	__shared__ UpdRec buf[UPD_WARPS][2][32];
+	extern __shared__ __align__(16) char upd_smem[];
+	uint8_t *chunk = reinterpret_cast<uint8_t *>(upd_smem + PSG_WIN_ROWS * 5 * 16) + (threadIdx.x & ~31);
+	uint64_t *bar = reinterpret_cast<uint64_t *>(upd_smem + PSG_WIN_ROWS * 5 * 16 + UPD_THREADS);
+	RateWindow rows;
+	rows.start(P, reinterpret_cast<float4 *>(upd_smem), bar);
+	bool rows_here = false;
 	const int64_t tick = B->tick0 + t;
 	const double tick_time = B->tick_time;
 	// the tick's particles, or only those listed in alist (the surrogate's rejects)
@@ -1230,111 +1233,71 @@ __global__ void __launch_bounds__(32 * UPD_WARPS, MINB) k_update_queue(int t, co
 	const unsigned n = alist ? *nalist : (unsigned)(hi - lo);
 	const int lane = threadIdx.x & 31;
 	const unsigned lt_mask = (1u << lane) - 1u;
-	UpdRec (*WB)[32] = buf[threadIdx.x >> 5];
-	int pass = 0;        // warp-uniform: 0 the slow-looking particles (or all), 1 the others
-	// fills WB[b] with the next particles of the pass, packed from slot 0;
-	// returns how many (0: none left)
-	auto fetch = [&](int b) -> int {
-		for (;;) {
-			unsigned base = 0;
-			if (lane == 0) base = atomicAdd(pass ? cursor2 : cursor, 32u);
-			base = __shfl_sync(0xffffffffu, base, 0);
-			if (base >= n) {
-				if (cursor2 && pass == 0) {
-					pass = 1;
-					continue;
-				}
-				return 0;
-			}
-			const int cnt = (int)min(32u, n - base);
-			bool keep = false;
-			UpdRec r;
-			if (lane < cnt) {
-				const unsigned k = base + lane;
-				const int a = alist ? (int)alist[k] : lo + (int)k;
-				keep = !cursor2 || (src.slow[a] != 0) == (pass == 0);
-				if (keep) {
-					const uint32_t p = src.act_ipar[a];
-					r.time = rn_dmul((double)(tick - lasthit[p]), tick_time);
-					r.lam0 = lambdaH[p];
-					r.g = src.act_g[a];
-					r.heat = src.act_heat[a];
-					r.ie0 = ie[p];
-					r.rho = src.rho[p];
-					r.yeMET = src.yeMET[p];
-					r.hstep = hstep[p];
-					r.p = p;
-					r.pad0 = 0u;
-					r.k0 = r.k1 = r.krec = 0.0;
-				}
-			}
-			const unsigned km = __ballot_sync(0xffffffffu, keep);
-			if (keep) WB[b][__popc(km & lt_mask)] = r;
-			__syncwarp();
-			if (km) return __popc(km);
-		}
-	};
-	int avail[2];
-	avail[0] = fetch(0);
-	avail[1] = fetch(1);
-	int cur = 0, used = 0;
-	bool exhausted = false;
+	int pass = 0;             // warp-uniform: 0 the slow-looking particles (or all), 1 the others
+	unsigned base = 0;        // the chunk's first particle; its places yet to be taken are chunk[used..left)
+	int used = 0, left = 0;
+	bool dry = false;
 	DPState S;
 	RhsCtx cx;
-	double atol1 = 0.0;
+	int a = 0;
 	uint32_t p = 0;
 	bool have = false;
 	uint32_t st = 0;
 	for (;;) {
+		bool fresh = false;
+		double h0 = 0.0;
 		unsigned need = __ballot_sync(0xffffffffu, !have);
-		while (need && !exhausted) {
-			const int left = avail[cur] - used;
-			if (left <= 0) {
-				if (avail[cur ^ 1] == 0) {
-					exhausted = true;
-					break;
+		while (need && !dry) {
+			if (used == left) {      // the next chunk
+				if (lane == 0) base = atomicAdd(pass ? cursor2 : cursor, 32u);
+				base = __shfl_sync(0xffffffffu, base, 0);
+				if (base >= n) {
+					if (cursor2 && pass == 0) pass = 1;
+					else dry = true;
+					continue;
 				}
-				cur ^= 1;
+				const unsigned i = base + lane;
+				const bool keep = i < n && (!cursor2 || (src.slow[lo + (int)i] != 0) == (pass == 0));
+				const unsigned km = __ballot_sync(0xffffffffu, keep);
+				if (keep) chunk[__popc(km & lt_mask)] = (uint8_t)lane;
+				__syncwarp();
 				used = 0;
-				avail[cur ^ 1] = fetch(cur ^ 1);
+				left = __popc(km);
 				continue;
 			}
 			const int rank = __popc(need & lt_mask);
-			const int take = min(__popc(need), left);
-			if (!have && rank < take) {
-				const UpdRec &r = WB[cur][used + rank];
-				p = r.p;
-				const double ie0 = (double)r.ie0;
-				const double T = ieye2T(P, ie0, rn_dadd(rn_dsub(1.0, r.lam0), P.he_e));
-				cx = make_rhs_ctx(P, (double)r.yeMET, r.g, r.heat, r.time, rn_dmul(P.H_PER_MASS, (double)r.rho), T);
-				S.x[0] = r.lam0;
-				S.x[1] = ie0;
-				S.rec = 0.0;
-				rhs<REC, true>(P, cx, S.x, S.k1, &S.krec);
-				atol1 = DP_ATOL1_REL * fabs(ie0) + 1e-300;
-				dp_init_k1(S);
+			if (!have && used + rank < left) {
+				const unsigned i = base + chunk[used + rank];
+				a = alist ? (int)alist[i] : lo + (int)i;
+				p = src.act_ipar[a];
+				const double time = rn_dmul((double)(tick - lasthit[p]), tick_time);
+				const float hs = hstep[p];
+				S.x[0] = lambdaH[p];
+				S.x[1] = (double)ie[p];
+				cx = make_rhs_ctx(P, (double)src.yeMET[p], src.act_g[a], src.act_heat[a], time,
+						rn_dmul(P.H_PER_MASS, (double)src.rho[p]), 0.0);
 				// the particle's last step proposal is a better first
 				// step than the derivative estimate
-				if (r.hstep > 0.0f) S.h = fmin(1.0, fmax((double)r.hstep / r.time, 1e-8));
-				have = true;
+				if (hs > 0.0f) h0 = fmax((double)hs / time, 1e-8);
+				have = fresh = true;
 			}
-			used += take;
+			used = min(left, used + __popc(need));
+			__syncwarp();
 			need = __ballot_sync(0xffffffffu, !have);
 		}
 		if (!__any_sync(0xffffffffu, have)) break;
+		if (!rows_here) {
+			rows_here = rows.wait(bar);
+			if (!rows_here) {      // (never seen: fall back on device memory, and say so)
+				rows.n = 0;
+				st |= PSG_ST_COPY;
+				rows_here = true;
+			}
+		}
+		if (fresh) dp_start<REC>(P, cx, S, h0, rows);
 		if (have) {
-			const bool done = dp_step<REC>(P, cx, S, atol1);
-			if (!done && S.steps >= DP_SWITCH) {
-				// stiff: hand the particle to k_update_stiff and free the lane
-				const unsigned q = atomicAdd(nstiff, 1u);
-				StiffItem it;
-				it.p = p; it.t = S.t; it.h = S.h; it.x0 = S.x[0]; it.x1 = S.x[1];
-				it.yeMET = cx.yeMET; it.g = cx.g; it.heat = cx.heat; it.time = cx.time; it.nH = cx.nH; it.T = cx.T;
-				it.rec = S.rec;
-				stiff[q] = it;
-				hstep[p] = 0.0f;
-				have = false;
-			} else if (done) {
+			const bool done = dp_step<REC>(P, cx, S, rows);
+			if (done) {
 				const double lam = S.x[0], e = S.x[1];
 				if (!(e >= 0.0)) st |= PSG_ST_IE_NEG;
 				if (!isfinite(lam) || !isfinite(e)) st |= PSG_ST_NAN;
@@ -1344,9 +1307,20 @@ __global__ void __launch_bounds__(32 * UPD_WARPS, MINB) k_update_queue(int t, co
 				lasthit[p] = tick;
 				hstep[p] = (float)((double)S.hnext * cx.time);
 				have = false;
+			} else if (S.steps >= DP_SWITCH) {
+				// stiff: hand the particle to k_update_stiff and free the lane
+				StiffItem it;
+				it.p = p; it.t = S.t; it.h = S.h; it.x0 = S.x[0]; it.x1 = S.x[1];
+				it.yeMET = cx.yeMET; it.g = cx.g; it.heat = cx.heat; it.time = cx.time; it.nH = cx.nH;
+				it.T = ieye2T(P, (double)ie[p], rn_dadd(rn_dsub(1.0, lambdaH[p]), P.he_e));
+				it.rec = S.rec;
+				stiff[atomicAdd(nstiff, 1u)] = it;
+				hstep[p] = 0.0f;
+				have = false;
 			}
 		}
 	}
+	if (!rows_here && !rows.wait(bar)) st |= PSG_ST_COPY;      // (no block leaves with its copy in flight)
 	if (st) atomicOr(status, st);
 }
 
@@ -1932,8 +1906,7 @@ struct BatchPlan {
 	bool gen = false, helium = false, iso = false, euler = false, surr = false, aff = false, feat_on = false;
 
 	// grids
-	unsigned dep_grid = 0, red_grid = 0, queue_grid = 0, he_grid = 0, euler_grid = 0, log_grid = 0, stiff_grid = 0;
-	int queue_minb = 1;         // the integrator's register limit: resident blocks per SM
+	unsigned dep_grid = 0, red_grid = 0, he_grid = 0, euler_grid = 0, log_grid = 0, stiff_grid = 0;
 	size_t src_R = 0;           // > 0: a recombination tick whose first src_R rays come traced and sorted (S_SRCHIT)
 };
 
@@ -2118,10 +2091,9 @@ int plan_batch(psg_context *ctx, size_t R, size_t K, const PsgTraceFill &tf, Bat
 			: (pl.aff ? occ_grid(ctx, k_deposit<false, true>, DEP_THREADS) : occ_grid(ctx, k_deposit<false, false>,
 					DEP_THREADS));
 	pl.red_grid = occ_grid(ctx, k_reduce<false, false>, 256);
-	pl.queue_minb = ctx->tune.update_minblocks >= 4 ? 4 : (ctx->tune.update_minblocks == 3 ? 3 : 1);
-	pl.queue_grid = pl.queue_minb == 4 ? occ_grid(ctx, k_update_queue<false, 4>, 32 * UPD_WARPS)
-			: pl.queue_minb == 3 ? occ_grid(ctx, k_update_queue<false, 3>, 32 * UPD_WARPS)
-			: occ_grid(ctx, k_update_queue<false, 1>, 32 * UPD_WARPS);
+	if (!pl.iso && !pl.euler && !pl.helium)
+		PSG_CUDA(!ctx->flags.on_the_spot ? cudaFuncSetAttribute(k_update_queue<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, UPD_SMEM)
+				: cudaFuncSetAttribute(k_update_queue<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, UPD_SMEM));
 	pl.he_grid = pl.euler ? occ_grid(ctx, k_update_he_euler, 128) : ctx->flags.on_the_spot
 			? occ_grid(ctx, k_update_he<false>, HEQ_THREADS) : occ_grid(ctx, k_update_he<true>, HEQ_THREADS);
 	pl.stiff_grid = pl.helium ? (ctx->flags.on_the_spot ? occ_grid(ctx, k_update_he_stiff<false>, STIFF_THREADS)
@@ -2331,26 +2303,20 @@ int enqueue_batch(psg_context *ctx, const BatchPlan &pl, const PsgBatchDev *B) {
 					ctx->launches++;
 				}
 				unsigned *cur2 = two_pass ? uv.cursors2 + t : nullptr;
-				if (P.ygrec) {
-					k_update_queue<true, 1><<<pl.queue_grid, 32 * UPD_WARPS, 0, st>>>((int)t, av.tick_act, us,
-							ctx->d_lambdaH, ctx->d_ie, ctx->d_lasthit, ctx->d_hstep, P, B, uv.cursors + t, cur2,
-							uv.stiff, uv.nstiff + t, nullptr, nullptr, ctx->d_status);
-					PSG_CHECK_LAUNCH();
+#define PSG_QUEUE(REC_)                                                                                       \
+	k_update_queue<REC_><<<sms, UPD_THREADS, UPD_SMEM, st>>>((int)t, av.tick_act, us, ctx->d_lambdaH,        \
+			ctx->d_ie, ctx->d_lasthit, ctx->d_hstep, P, B, uv.cursors + t, cur2, uv.stiff, uv.nstiff + t,      \
+			pl.surr ? uv.rej : nullptr, pl.surr ? uv.nrej + t : nullptr, ctx->d_status)
+				if (P.ygrec) PSG_QUEUE(true);
+				else PSG_QUEUE(false);
+#undef PSG_QUEUE
+				PSG_CHECK_LAUNCH();
+				if (P.ygrec)
 					k_update_stiff<true><<<pl.stiff_grid, STIFF_THREADS, 0, st>>>(uv.stiff, uv.nstiff + t,
 							uv.stiff_ctr + t, ctx->d_lambdaH, ctx->d_ie, ctx->d_lasthit, P, B, (int)t, ctx->d_status);
-				} else {
-#define PSG_QUEUE(MINB_)                                                                                       \
-	k_update_queue<false, MINB_><<<pl.queue_grid, 32 * UPD_WARPS, 0, st>>>((int)t, av.tick_act, us,          \
-			ctx->d_lambdaH, ctx->d_ie, ctx->d_lasthit, ctx->d_hstep, P, B, uv.cursors + t, cur2, uv.stiff,     \
-			uv.nstiff + t, pl.surr ? uv.rej : nullptr, pl.surr ? uv.nrej + t : nullptr, ctx->d_status)
-					if (pl.queue_minb == 4) PSG_QUEUE(4);
-					else if (pl.queue_minb == 3) PSG_QUEUE(3);
-					else PSG_QUEUE(1);
-#undef PSG_QUEUE
-					PSG_CHECK_LAUNCH();
+				else
 					k_update_stiff<false><<<pl.stiff_grid, STIFF_THREADS, 0, st>>>(uv.stiff, uv.nstiff + t,
 							uv.stiff_ctr + t, ctx->d_lambdaH, ctx->d_ie, ctx->d_lasthit, P, B, (int)t, ctx->d_status);
-				}
 				PSG_CHECK_LAUNCH();
 				ctx->launches += 2;
 				if (feat) {
@@ -2401,7 +2367,6 @@ std::vector<unsigned long long> batch_key(const psg_context *ctx, const BatchPla
 	k.push_back(ctx->n);
 	k.push_back(ctx->hit_cap);
 	k.push_back((unsigned long long)ctx->tune.deposit_long << 32 | (unsigned)ctx->tune.deposit_mid);
-	k.push_back((unsigned long long)pl.queue_minb);
 	k.push_back((unsigned long long)ctx->tune.run_short);
 	k.push_back((unsigned long long)ctx->tune.update_order);
 	k.push_back((unsigned long long)psg_sort_classes(pl.maxcount));
@@ -2768,13 +2733,6 @@ extern "C" int psg_autotune(psg_context *ctx, const psg_ray *d_rays, size_t R, s
 		psg_tune t = cur;
 		t.deposit_long = th[0];
 		t.deposit_mid = th[1];
-		rc = consider(t);
-	}
-	// the integrator's registers (occupancy against spills)
-	for (int mb : {1, 3, 4}) {
-		if (rc || mb == cur.update_minblocks) continue;
-		psg_tune t = cur;
-		t.update_minblocks = mb;
 		rc = consider(t);
 	}
 	// which runs are sorted before their sums, which put in order where summed
