@@ -43,7 +43,7 @@ enum {
 // scratch slots
 enum {
 	S_RAYS = 0, S_COUNT, S_OFFSETS, S_RAW_IPAR, S_RAW_D, S_RAW_B, S_KEYS, S_VALS,
-	S_HIT_IPAR, S_HIT_KERN, S_ACC, S_ACT, S_CUB, S_TREE, S_MISC, S_REC_U32, S_REC_F64, S_RAYLIST, S_UPD,
+	S_HIT_IPAR, S_HIT_KERN, S_ACC, S_ACT, S_CUB, S_TREE, S_MISC, S_REC_U32, S_RAYLIST, S_UPD,
 	S_EMIT, S_MAP, S_ALONG, S_MLP, S_LOG, S_SURR, S_REC, S_RECW, S_RECK, S_RECRAYS, S_SNAP, S_SCAN, S_SLOTCNT,
 	S_SRCHIT,
 	S_NSLOTS
@@ -262,9 +262,9 @@ struct PsgTraceFill {
 	size_t scap;                    // slab capacity per ray
 };
 int psg_trace_fill(psg_context *ctx, const psg_ray *d_rays, size_t nray, PsgTraceFill *tf);
-int psg_trace_sort_prepare(psg_context *ctx, size_t nray, size_t cap, unsigned long long maxcount);
-int psg_trace_sort_enqueue(psg_context *ctx, size_t nray, size_t nhit, unsigned long long maxcount, int want_kern,
-		size_t r0);
+int psg_trace_sort_prepare(psg_context *ctx, size_t nray, size_t cap, unsigned long long maxcount, int want_kern);
+int psg_trace_sort_enqueue(psg_context *ctx, const psg_ray *rays, const PsgBatchDev *B, size_t nray,
+		unsigned long long maxcount, int want_kern, size_t r0);
 int psg_trace_internal(psg_context *ctx, const psg_ray *d_rays, size_t nray, int want_kern);
 int psg_sort_classes(unsigned long long maxcount);
 int psg_trace_fill_prepare(psg_context *ctx, size_t nray);

@@ -2058,7 +2058,7 @@ int plan_batch(psg_context *ctx, size_t R, size_t K, const PsgTraceFill &tf, Bat
 	pl.aff = ctx->sat_frac > 1e-3;
 	const size_t cap = pl.cap, nray = pl.nray;
 
-	int rc = psg_trace_sort_prepare(ctx, nray, cap, pl.maxcount);
+	int rc = psg_trace_sort_prepare(ctx, nray, cap, pl.maxcount, 1);
 	if (rc) return rc;
 	// slots and the active lists
 	if (!psg_scratch(ctx, S_VALS, sizeof(uint32_t) * 2 * cap) ||
@@ -2116,7 +2116,7 @@ int enqueue_batch(psg_context *ctx, const BatchPlan &pl, const PsgBatchDev *B) {
 	const PhysParams P = psg_phys_params(ctx);
 	const int sms = ctx->sms;
 	int rc = pl.src_R ? psg_trace_rec_sort_enqueue(ctx, pl.src_R, nray, pl.maxcount, B)
-			: psg_trace_sort_enqueue(ctx, nray, pl.nhit, pl.maxcount, 1, 0);
+			: psg_trace_sort_enqueue(ctx, nullptr, B, nray, pl.maxcount, 1, 0);
 	if (rc) return rc;
 	int64_t *off64 = (int64_t *)ctx->scratch[S_OFFSETS].p;
 	uint32_t *hit_ipar = (uint32_t *)ctx->scratch[S_HIT_IPAR].p;

@@ -20,100 +20,118 @@
 
 namespace {
 
-// pluecker_() pluecker-sse.c:28-198. The reference's 8 hand-written sign
-// classes reduce to one rule per axis and per axis pair (selected by the
-// signs of dir); every product and difference rounds once, in float.
-__device__ __forceinline__ bool segment_hits_box(const float dir[3], float dist, const float s2b[3],
-		const float s2t[3]) {
-	bool up[3];
-#pragma unroll
-	for (int a = 0; a < 3; a++) {
-		up[a] = dir[a] > 0.0f;
-		const float step = rn_fmul(dist, dir[a]);
-		const float e2t = rn_fsub(s2t[a], step);
-		const float e2b = rn_fsub(s2b[a], step);
-		if (up[a] ? (s2t[a] < 0.0f) : (s2b[a] > 0.0f)) return false;
-		if (up[a] ? (e2b > 0.0f) : (e2t < 0.0f)) return false;
-	}
-#pragma unroll
-	for (int q = 0; q < 3; q++) {
-		const int i = q == 2 ? 1 : 0;
-		const int j = q == 0 ? 1 : 2;
-		const float P = up[i] ? s2t[j] : s2b[j];
-		const float R = up[i] ? s2b[j] : s2t[j];
-		const float Q = up[j] ? s2b[i] : s2t[i];
-		const float S = up[j] ? s2t[i] : s2b[i];
-		if (rn_fmul(dir[i], P) < rn_fmul(dir[j], Q) || rn_fmul(dir[i], R) > rn_fmul(dir[j], S)) return false;
-	}
-	return true;
-}
-
+// A ray as the traversal uses it. up: the direction's component is positive.
+// Mirrored along the axes where it is not, every ray goes up: sg is the
+// axis's sign, os the mirrored start negated, ad the mirrored direction and
+// reach the mirrored displacement to its end.
 struct RayGeom {
-	float s[3], dir[3], dist;
+	float s[3], dir[3];
+	float sg[3], os[3], ad[3], reach[3];
+	bool up[3];
+	float margin;      // of line_test(), per squared distance
 };
 
 __device__ __forceinline__ RayGeom load_ray(const psg_ray *__restrict__ rays, size_t r) {
 	RayGeom g;
 	const psg_ray &ry = rays[r];
+	const float dist = (float)ry.length;      // rt_trace() takes the length as float
+	float dir2 = 0.0f;
 #pragma unroll
-	for (int d = 0; d < 3; d++) { g.s[d] = ry.s[d]; g.dir[d] = ry.dir[d]; }
-	g.dist = (float)ry.length;      // rt_trace() takes the length as float
+	for (int a = 0; a < 3; a++) {
+		g.s[a] = ry.s[a];
+		g.dir[a] = ry.dir[a];
+		g.up[a] = g.dir[a] > 0.0f;
+		g.sg[a] = g.up[a] ? 1.0f : -1.0f;
+		g.os[a] = -g.sg[a] * g.s[a];
+		g.ad[a] = g.sg[a] * g.dir[a];
+		g.reach[a] = g.sg[a] * rn_fmul(dist, g.dir[a]);
+		dir2 += g.dir[a] * g.dir[a];
+	}
+	g.margin = 2e-6f * fmaxf(1.0f, dir2);
 	return g;
+}
+
+// pluecker_() pluecker-sse.c:28-198. The reference's 8 hand-written sign
+// classes are mirror images of one another, and mirroring changes no
+// magnitude: each product and difference rounds once, in float, to the
+// reference's value or its negative, and each comparison is the reference's
+// or its mirror image. lo.w and hi.w are not looked at.
+__device__ __forceinline__ bool segment_hits_box(const RayGeom &g, const float4 lo, const float4 hi) {
+	const float l[3] = {lo.x, lo.y, lo.z}, h[3] = {hi.x, hi.y, hi.z};
+	float n[3], f[3];      // the near and the far face, seen from the start
+	bool miss = false;
+#pragma unroll
+	for (int a = 0; a < 3; a++) {
+		n[a] = __fmaf_rn(g.sg[a], g.up[a] ? l[a] : h[a], g.os[a]);      // (one rounding: the product is exact)
+		f[a] = __fmaf_rn(g.sg[a], g.up[a] ? h[a] : l[a], g.os[a]);
+		miss = miss | (f[a] < 0.0f) | (rn_fsub(n[a], g.reach[a]) > 0.0f);
+	}
+#pragma unroll
+	for (int q = 0; q < 3; q++) {
+		const int i = q == 2 ? 1 : 0;
+		const int j = q == 0 ? 1 : 2;
+		miss = miss | (rn_fmul(g.ad[i], f[j]) < rn_fmul(g.ad[j], n[i])) | (rn_fmul(g.ad[i], n[j]) > rn_fmul(g.ad[j], f[i]));
+	}
+	return !miss;
 }
 
 // The line test of raytrace.c:168-195: float differences and products,
 // double sums (in the order the reference's build adds them: y and z
-// first, then x); accepted iff sml^2 >= (dc - proj)(dc + proj).
-// Candidates that miss by a wide margin are rejected in float first: the
-// float estimate r2f = d2f - projf^2 carries at most ~12 roundings of
-// relative size 2^-24 of d2 (about 7.2e-7 d2), so r2f - sml^2 > 1e-5 d2f
-// guarantees the exact test rejects too; everything closer takes the exact
-// double path, so the accepted set is the reference's.
-__device__ __forceinline__ bool line_hits_particle(const RayGeom &g, float4 q, double &dc, double &r2) {
+// first, then x; its -ffast-math lets the compiler reassociate the loop,
+// which rounds differently in rare cases, by 1 ulp of d). d: the distance to
+// the centre; r2: the squared distance to the line; a hit unless sml^2 < r2.
+struct HitDist {
+	double d, proj;
+	__device__ __forceinline__ double r2() const { return rn_dmul(rn_dsub(d, proj), rn_dadd(d, proj)); }
+};
+__device__ __forceinline__ double hit_d(const float s[3], const float4 q) {
+	const float dx = rn_fsub(q.x, s[0]), dy = rn_fsub(q.y, s[1]), dz = rn_fsub(q.z, s[2]);
+	return __dsqrt_rn(rn_dadd((double)rn_fmul(dx, dx), rn_dadd((double)rn_fmul(dy, dy), (double)rn_fmul(dz, dz))));
+}
+__device__ __forceinline__ double hit_proj(const float s[3], const float dir[3], const float4 q) {
+	const float dx = rn_fsub(q.x, s[0]), dy = rn_fsub(q.y, s[1]), dz = rn_fsub(q.z, s[2]);
+	return rn_dadd((double)rn_fmul(dx, dir[0]), rn_dadd((double)rn_fmul(dy, dir[1]), (double)rn_fmul(dz, dir[2])));
+}
+
+// Whether the line meets the particle, decided in float where that is sure:
+// r2f = fl(d2f - fl(pf^2)) differs from the exact test's r2 by at most 8
+// roundings of 2^-24 of d2 max(1, |dir|^2) (two each in the sums of d2f and
+// pf, whose terms are the exact test's own, doubled by the square, one each
+// in the square and the difference): 4.8e-7. Beyond a margin of 2e-6 the
+// exact test decides alike; within it (or with squares near the smallest
+// floats, or a NaN, which marks flagged particles) the exact one is made.
+__device__ __forceinline__ bool line_test(const RayGeom &g, const float4 q, int p, const uint32_t *__restrict__ lidx) {
 	const float dx = rn_fsub(q.x, g.s[0]), dy = rn_fsub(q.y, g.s[1]), dz = rn_fsub(q.z, g.s[2]);
-	{
-		const float pf = __fadd_rn(__fadd_rn(rn_fmul(dx, g.dir[0]), rn_fmul(dy, g.dir[1])), rn_fmul(dz, g.dir[2]));
-		const float d2f = __fadd_rn(__fadd_rn(rn_fmul(dx, dx), rn_fmul(dy, dy)), rn_fmul(dz, dz));
-		const float r2f = __fsub_rn(d2f, rn_fmul(pf, pf));
-		if (__fsub_rn(r2f, rn_fmul(q.w, q.w)) > 1e-5f * d2f) return false;
-	}
-	// the three-term sums as the reference's build evaluates them: its
-	// -ffast-math lets the compiler reassociate the loop into (y + z) + x,
-	// which rounds differently from (x + y) + z in rare cases (1 ulp of d)
-	const double proj = rn_dadd((double)rn_fmul(dx, g.dir[0]),
-			rn_dadd((double)rn_fmul(dy, g.dir[1]), (double)rn_fmul(dz, g.dir[2])));
-	const double d2 = rn_dadd((double)rn_fmul(dx, dx), rn_dadd((double)rn_fmul(dy, dy), (double)rn_fmul(dz, dz)));
-	dc = __dsqrt_rn(d2);
-	r2 = rn_dmul(rn_dsub(dc, proj), rn_dadd(dc, proj));
-	return !((double)rn_fmul(q.w, q.w) < r2);
+	const float pf = __fadd_rn(__fadd_rn(rn_fmul(dx, g.dir[0]), rn_fmul(dy, g.dir[1])), rn_fmul(dz, g.dir[2]));
+	const float d2f = __fadd_rn(__fadd_rn(rn_fmul(dx, dx), rn_fmul(dy, dy)), rn_fmul(dz, dz));
+	const float s2 = rn_fmul(q.w, q.w);
+	const float over = __fsub_rn(__fsub_rn(d2f, rn_fmul(pf, pf)), s2);
+	const float m = d2f > 1e-30f ? g.margin * d2f : __int_as_float(0x7f800000);
+	if (over < -m) return true;
+	if (over > m) return false;
+	if (__ldg(&lidx[p]) & PSG_INVALID_BIT) return false;
+	const HitDist h{hit_d(g.s, q), hit_proj(g.s, g.dir, q)};
+	return !((double)s2 < h.r2());
 }
 
 // Candidates listed in shared memory (leaf-order particle positions), tested
-// 32 at a time; accepted hits go to the ray's slab in order of discovery.
+// 32 at a time; the hits go to the ray's slab in order of discovery, as
+// positions alone: their distances are computed by the sort, with every
+// lane busy.
 __device__ __forceinline__ void test_candidates(const RayGeom &g, const int *list, int total,
-		const float4 *__restrict__ lpsml, const uint32_t *__restrict__ lidx, size_t r, size_t scap,
-		uint32_t *__restrict__ slab_ipar, double *__restrict__ slab_d, double *__restrict__ slab_b,
+		const float4 *__restrict__ lpsml, const uint32_t *__restrict__ lidx, uint32_t *__restrict__ slab, size_t scap,
 		uint32_t &nh, int lane, unsigned lt_mask) {
 	for (int k0 = 0; k0 < total; k0 += 32) {
 		const int k = k0 + lane;
 		bool acc = false;
-		double dc = 0.0, r2 = 0.0;
-		uint32_t idx = 0;
+		int p = 0;
 		if (k < total) {
-			const int p = list[k];
-			idx = __ldg(&lidx[p]);
-			if (!(idx & PSG_INVALID_BIT)) acc = line_hits_particle(g, __ldg(&lpsml[p]), dc, r2);
+			p = list[k];
+			acc = line_test(g, __ldg(&lpsml[p]), p, lidx);
 		}
 		const unsigned bal = __ballot_sync(0xffffffffu, acc);
-		if (acc) {
-			const size_t q = nh + __popc(bal & lt_mask);
-			if (q < scap) {
-				const size_t o = r * scap + q;
-				slab_ipar[o] = idx;
-				slab_d[o] = dc;
-				slab_b[o] = r2;      // (b = sqrt|r2| is taken in the sort, with every lane busy)
-			}
-		}
+		const size_t q = nh + __popc(bal & lt_mask);
+		if (acc && q < scap) slab[q] = (uint32_t)p;
 		nh += __popc(bal);
 	}
 }
@@ -126,18 +144,31 @@ __device__ __forceinline__ void test_candidates(const RayGeom &g, const int *lis
 // test. The cells tested are exactly the children of crossed cells, as in
 // the reference's walk (raytrace.c:160-208); only the order differs, and the
 // per-ray sort makes the output independent of it. The stack cannot exceed
-// 4 + 28 entries per tree level; TR_STACK leaves room for 21 levels and an
-// overflow would raise PSG_ST_STACK instead of losing cells.
-#define TR_STACK 1024
+// 4 + 28 entries per tree level (592 at 21 levels); an overflow would raise
+// PSG_ST_STACK instead of losing cells.
+//
+// Bound by instruction issue: on the 2M-particle field a ray of 690 hits
+// takes 69 rounds of cells and 60 of candidates. So the box test is one
+// branch-free form for all sign classes, the line test is FP32 but near its
+// boundary (2 candidates a ray), hits are stored as positions (4 bytes, not
+// 20), a leaf's place in the list comes from ballots and its particles are
+// listed by predicated stores, and 48 registers leave 40 warps per
+// multiprocessor. 65536 rays: 1.91 -> 1.39 ms; 65536 on 16.8M particles (1200
+// hits each) 5.0 -> 3.2 ms; 102400 on 64^3 (123 each) 0.68 -> 0.51 ms.
+// PPC: the leaves' capacity where it is 8 (the reference's), else 0 and the
+// argument.
+#define TR_STACK 640
+#define TR_REGS 48
 #define TR_MAX_WARPS 16      // warps per block: ctx->tune.trace_warps, at most this
 
-__global__ void __launch_bounds__(32 * TR_MAX_WARPS) k_trace_stack(const psg_ray *__restrict__ rays, size_t nray,
+template <int PPC>
+__global__ void __maxnreg__(TR_REGS) k_trace_stack(const psg_ray *__restrict__ rays, size_t nray,
 		const float4 *__restrict__ wlo, const float4 *__restrict__ whi,
-		const float4 *__restrict__ lpsml, const uint32_t *__restrict__ lidx, int ppc,
+		const float4 *__restrict__ lpsml, const uint32_t *__restrict__ lidx, int ppc_any,
 		uint32_t *__restrict__ count, size_t scap, uint32_t *__restrict__ slab_ipar,
-		double *__restrict__ slab_d, double *__restrict__ slab_b, unsigned long long *__restrict__ next_ray,
-		uint32_t *__restrict__ status, const unsigned *__restrict__ nlim) {
+		unsigned long long *__restrict__ next_ray, uint32_t *__restrict__ status, const unsigned *__restrict__ nlim) {
 	extern __shared__ int tr_smem[];
+	const int ppc = PPC ? PPC : ppc_any;
 	// rays past *nlim (when given: the recombination path's emitted count)
 	// are not traced; their counts stay as zeroed
 	if (nlim) nray = min(nray, (size_t)*nlim);
@@ -145,6 +176,7 @@ __global__ void __launch_bounds__(32 * TR_MAX_WARPS) k_trace_stack(const psg_ray
 	const int wib = threadIdx.x >> 5;
 	int *stack = tr_smem + wib * (TR_STACK + 32 * ppc + 32);
 	int *list = stack + TR_STACK;      // candidates waiting for a full round of 32
+	const unsigned lt_mask = (1u << lane) - 1u;
 	// persistent warps: each takes the next ray from a shared counter, so a
 	// block never idles behind its longest ray
 	for (;;) {
@@ -154,15 +186,13 @@ __global__ void __launch_bounds__(32 * TR_MAX_WARPS) k_trace_stack(const psg_ray
 	if (rr >= nray) break;
 	const size_t r = (size_t)rr;
 	const RayGeom g = load_ray(rays, r);
-	const unsigned lt_mask = (1u << lane) - 1u;
+	uint32_t *slab = slab_ipar + r * scap;
 	uint32_t nh = 0;
 	int sp = 0, nbuf = 0;
 	bool overflow = false;
 	{
 		const float4 lo = __ldg(&wlo[0]), hi = __ldg(&whi[0]);
-		const float s2b[3] = {rn_fsub(lo.x, g.s[0]), rn_fsub(lo.y, g.s[1]), rn_fsub(lo.z, g.s[2])};
-		const float s2t[3] = {rn_fsub(hi.x, g.s[0]), rn_fsub(hi.y, g.s[1]), rn_fsub(hi.z, g.s[2])};
-		if (segment_hits_box(g.dir, g.dist, s2b, s2t)) {
+		if (segment_hits_box(g, lo, hi)) {
 			const int w = __float_as_int(lo.w);
 			if (w >= 0) {
 				if (lane == 0) stack[0] = w;
@@ -171,7 +201,7 @@ __global__ void __launch_bounds__(32 * TR_MAX_WARPS) k_trace_stack(const psg_ray
 				const int cnt = min(-1 - w, ppc), ps = __float_as_int(hi.w);
 				for (int k = lane; k < cnt; k += 32) list[k] = ps + k;
 				__syncwarp();
-				test_candidates(g, list, cnt, lpsml, lidx, r, scap, slab_ipar, slab_d, slab_b, nh, lane, lt_mask);
+				test_candidates(g, list, cnt, lpsml, lidx, slab, scap, nh, lane, lt_mask);
 			}
 		}
 	}
@@ -183,42 +213,38 @@ __global__ void __launch_bounds__(32 * TR_MAX_WARPS) k_trace_stack(const psg_ray
 		const int c = valid ? stack[sp - k + node] + (lane & 7) : 0;
 		__syncwarp();
 		sp -= k;
-		float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
-		bool hit = false;
-		if (valid) {
-			lo = __ldg(&wlo[c]);
-			hi = __ldg(&whi[c]);
-			const float s2b[3] = {rn_fsub(lo.x, g.s[0]), rn_fsub(lo.y, g.s[1]), rn_fsub(lo.z, g.s[2])};
-			const float s2t[3] = {rn_fsub(hi.x, g.s[0]), rn_fsub(hi.y, g.s[1]), rn_fsub(hi.z, g.s[2])};
-			hit = segment_hits_box(g.dir, g.dist, s2b, s2t);
-		}
+		const float4 lo = __ldg(&wlo[c]), hi = __ldg(&whi[c]);
+		const bool hit = valid & segment_hits_box(g, lo, hi);
 		const int w = __float_as_int(lo.w);
-		const bool internal = hit && w >= 0;
-		const unsigned bi = __ballot_sync(0xffffffffu, internal);
-		if (internal) {
+		const unsigned bi = __ballot_sync(0xffffffffu, hit && w >= 0);
+		if (hit && w >= 0) {
 			const int pos = sp + __popc(bi & lt_mask);
 			if (pos < TR_STACK) stack[pos] = w;
 		}
 		sp += __popc(bi);
 		if (sp > TR_STACK) { overflow = true; sp = TR_STACK; }
+		// the crossed leaves' particles behind those waiting: each leaf's
+		// place from the ballots of its count's bits
 		const int cnt = (hit && w < 0) ? min(-1 - w, ppc) : 0;
-		int cs = cnt;
+		int before = 0;
 #pragma unroll
-		for (int o = 1; o < 32; o <<= 1) {
-			const int t = __shfl_up_sync(0xffffffffu, cs, o);
-			if (lane >= o) cs += t;
+		for (int bit = 0; bit < (PPC ? 4 : 8); bit++)
+			before += __popc(__ballot_sync(0xffffffffu, (cnt >> bit) & 1) & lt_mask) << bit;
+		const int ps = __float_as_int(hi.w);
+		int *const mine = list + nbuf + before;
+		if (PPC) {
+#pragma unroll
+			for (int q = 0; q < PPC; q++)
+				if (q < cnt) mine[q] = ps + q;
+		} else {
+			for (int q = 0; q < cnt; q++) mine[q] = ps + q;
 		}
-		const int total = __shfl_sync(0xffffffffu, cs, 31);
-		if (cnt) {
-			const int ps = __float_as_int(hi.w), base = nbuf + cs - cnt;
-			for (int q = 0; q < cnt; q++) list[base + q] = ps + q;
-		}
-		nbuf += total;
+		nbuf += __shfl_sync(0xffffffffu, before + cnt, 31);
 		__syncwarp();
 		// line tests only in full rounds of 32; the rest waits in the list
 		if (nbuf >= 32) {
 			const int full = nbuf & ~31, rem = nbuf - full;
-			test_candidates(g, list, full, lpsml, lidx, r, scap, slab_ipar, slab_d, slab_b, nh, lane, lt_mask);
+			test_candidates(g, list, full, lpsml, lidx, slab, scap, nh, lane, lt_mask);
 			__syncwarp();
 			const int keep = lane < rem ? list[full + lane] : 0;
 			__syncwarp();
@@ -227,7 +253,7 @@ __global__ void __launch_bounds__(32 * TR_MAX_WARPS) k_trace_stack(const psg_ray
 			__syncwarp();
 		}
 	}
-	if (nbuf) test_candidates(g, list, nbuf, lpsml, lidx, r, scap, slab_ipar, slab_d, slab_b, nh, lane, lt_mask);
+	if (nbuf) test_candidates(g, list, nbuf, lpsml, lidx, slab, scap, nh, lane, lt_mask);
 	if (lane == 0) {
 		count[r] = nh;
 		if (overflow) atomicOr(status, PSG_ST_STACK);
@@ -266,23 +292,45 @@ __device__ __forceinline__ uint32_t caller_index(const uint32_t *__restrict__ or
 	return order ? order[i] : i;
 }
 
-// The hit at slab position p of a ray as the sorted list's entry h (the slab
-// holds b^2; b = sqrt|b^2| here); with want_kern b becomes the
-// column-density factor sph_depth(b/h)/h^2 (loop.c:429-445).
-__device__ __forceinline__ void put_sorted_hit(int64_t h, uint32_t p, const uint32_t *__restrict__ raw_ipar,
-		const double *__restrict__ raw_d, const double *__restrict__ raw_b, uint32_t *__restrict__ out_ipar,
-		double *__restrict__ out_d, double *__restrict__ out_b, int want_kern, const float4 *__restrict__ psml,
-		const PhysParams &P) {
-	const uint32_t ip = raw_ipar[p];
-	const double b = __dsqrt_rn(fabs(raw_b[p]));      // the slab holds the squared distance
-	out_ipar[h] = ip;
-	out_d[h] = raw_d[p];
-	if (want_kern) {
-		const double sml = (double)psml[ip].w;
-		const double inv = __ddiv_rn(1.0, sml);
-		out_b[h] = rn_dmul(sph_depth(P, rn_dmul(b, inv)), rn_dmul(inv, inv));
+// What a sort kernel reads and writes: the rays (of a replayed batch, from its
+// per-call values), their slabs of hit positions and the sorted lists. With
+// want_kern, in the ticks, b becomes the column-density factor
+// sph_depth(b/h)/h^2 (loop.c:429-445) and the distances, which only order the
+// hits there, are not stored.
+struct SortIO {
+	const psg_ray *rays;
+	const PsgBatchDev *B;
+	const int64_t *off;
+	size_t scap, slab_r0;
+	const uint32_t *slab;
+	uint32_t *out_ipar;
+	double *out_d, *out_b;
+	int want_kern;
+	const float4 *psml;
+	const uint32_t *order;
+	__device__ __forceinline__ void ray(size_t r, float s[3], float dir[3]) const {
+		const psg_ray &ry = (B ? B->rays : rays)[r];
+#pragma unroll
+		for (int a = 0; a < 3; a++) {
+			s[a] = ry.s[a];
+			dir[a] = ry.dir[a];
+		}
+	}
+};
+
+// The hit on particle ip at distance d as the sorted list's entry h.
+__device__ __forceinline__ void put_sorted_hit(const SortIO &io, const PhysParams &P, int64_t h, uint32_t ip, double d,
+		const float s[3], const float dir[3]) {
+	const float4 q = io.psml[ip];
+	const HitDist hd{d, hit_proj(s, dir, q)};
+	const double b = __dsqrt_rn(fabs(hd.r2()));
+	io.out_ipar[h] = ip;
+	if (io.want_kern) {
+		const double inv = __ddiv_rn(1.0, (double)q.w);
+		io.out_b[h] = rn_dmul(sph_depth(P, rn_dmul(b, inv)), rn_dmul(inv, inv));
 	} else {
-		out_b[h] = b;
+		io.out_d[h] = d;
+		io.out_b[h] = b;
 	}
 }
 
@@ -292,46 +340,46 @@ __device__ __forceinline__ void put_sorted_hit(int64_t h, uint32_t p, const uint
 // 1024 hits, 16 up to 4096, 20 beyond, so that about n^2 / 2^(bits+1) pairs
 // share a key -- and the few runs of equal keys are then insertion-sorted
 // on the exact (d, ipar) -- the reference's d
-// order (loop.c:783-787) with ties broken by the caller's particle index. With want_kern the b column is replaced by the
-// column-density factor sph_depth(b/h)/h^2 of loop.c:429-445.
+// order (loop.c:783-787) with ties broken by the caller's particle index.
+// The distances are computed from the particles' positions (the slab holds
+// no more than the hits' particles) and kept in shared memory.
+template <int TPR, int IPT>
+struct SortSmem {
+	using Sort = cub::BlockRadixSort<uint32_t, TPR, IPT, uint32_t, 4>;
+	static constexpr int NMAX = TPR * IPT;
+	double d[NMAX];
+	double lo[TPR / 32], hi[TPR / 32];
+	union {
+		typename Sort::TempStorage sort;
+		struct {
+			uint32_t key[NMAX], pos[NMAX];
+		} s;
+	} u;
+};
 template <int TPR, int IPT>
 __global__ void __launch_bounds__(TPR) k_sort_block(const uint32_t *__restrict__ list,
-		const unsigned long long *__restrict__ d_nlist,
-		const int64_t *__restrict__ off, size_t scap, const uint32_t *__restrict__ slab_ipar,
-		const double *__restrict__ slab_d, const double *__restrict__ slab_b, uint32_t *__restrict__ out_ipar,
-		double *__restrict__ out_d, double *__restrict__ out_b, int want_kern, const float4 *__restrict__ psml,
-		PhysParams P, const uint32_t *__restrict__ order, size_t slab_r0) {
-	constexpr int NMAX = TPR * IPT;
-	using Sort = cub::BlockRadixSort<uint32_t, TPR, IPT, uint32_t, 4>;
-	struct Smem {
-		typename Sort::TempStorage sort;
-		uint32_t key[NMAX];
-		uint32_t pos[NMAX];
-		double lo[TPR / 32], hi[TPR / 32];
-	};
+		const unsigned long long *__restrict__ d_nlist, const SortIO io, PhysParams P) {
+	using Smem = SortSmem<TPR, IPT>;
+	constexpr int NMAX = Smem::NMAX;
 	extern __shared__ __align__(16) char sort_smem[];
 	Smem &sm = *reinterpret_cast<Smem *>(sort_smem);
+	uint32_t *const key = sm.u.s.key, *const pos = sm.u.s.pos;
 	// a persistent grid: the class's ray count is read here, so the launch
 	// needs no count from the host
 	const unsigned long long nlist = *d_nlist;
 	for (unsigned long long li = blockIdx.x; li < nlist; li += gridDim.x) {
 	const size_t r = list[li];
-	const int64_t h0 = off[r];
-	const int n = (int)(off[r + 1] - h0);
-	const uint32_t *raw_ipar = slab_ipar + (r - slab_r0) * scap;
-	const double *raw_d = slab_d + (r - slab_r0) * scap, *raw_b = slab_b + (r - slab_r0) * scap;
-	// keys: d mapped onto 24 bits over the ray's [min, max] (monotone, so
-	// equal keys only ever hide an order the fix-up below restores)
-	double dv[IPT];
+	const int64_t h0 = io.off[r];
+	const int n = (int)(io.off[r + 1] - h0);
+	const uint32_t *__restrict__ raw = io.slab + (r - io.slab_r0) * io.scap;
+	float s[3], dir[3];
+	io.ray(r, s, dir);
 	double dlo = 1e300, dhi = -1e300;
-#pragma unroll
-	for (int u = 0; u < IPT; u++) {
-		const int i = threadIdx.x * IPT + u;
-		dv[u] = i < n ? raw_d[i] : 0.0;
-		if (i < n) {
-			dlo = fmin(dlo, dv[u]);
-			dhi = fmax(dhi, dv[u]);
-		}
+	for (int i = threadIdx.x; i < n; i += TPR) {
+		const double d = hit_d(s, io.psml[raw[i]]);
+		sm.d[i] = d;
+		dlo = fmin(dlo, d);
+		dhi = fmax(dhi, d);
 	}
 #pragma unroll
 	for (int o = 16; o > 0; o >>= 1) {
@@ -357,49 +405,49 @@ __global__ void __launch_bounds__(TPR) k_sort_block(const uint32_t *__restrict__
 		const int i = threadIdx.x * IPT + u;
 		// padding takes the largest key; the sort is stable and padding
 		// follows every real item, so it stays behind them
-		k[u] = i < n ? min((uint32_t)((dv[u] - dlo) * scale), KEY_MAX) : KEY_MAX;
+		k[u] = i < n ? min((uint32_t)((sm.d[i] - dlo) * scale), KEY_MAX) : KEY_MAX;
 		v[u] = (uint32_t)i;
 	}
-	Sort(sm.sort).Sort(k, v, 0, KEY_BITS);
+	typename Smem::Sort(sm.u.sort).Sort(k, v, 0, KEY_BITS);
 	__syncthreads();
 #pragma unroll
 	for (int u = 0; u < IPT; u++) {
 		const int i = threadIdx.x * IPT + u;
-		sm.key[i] = k[u];
-		sm.pos[i] = v[u];
+		key[i] = k[u];
+		pos[i] = v[u];
 	}
 	__syncthreads();
-	// exact order inside runs of equal float keys
+	// exact order inside runs of equal keys
 	for (int i = threadIdx.x; i + 1 < n; i += TPR) {
-		if (sm.key[i] != sm.key[i + 1] || (i > 0 && sm.key[i - 1] == sm.key[i])) continue;
+		if (key[i] != key[i + 1] || (i > 0 && key[i - 1] == key[i])) continue;
 		int e = i + 1;
-		while (e + 1 < n && sm.key[e + 1] == sm.key[i]) e++;
+		while (e + 1 < n && key[e + 1] == key[i]) e++;
 		for (int a = i + 1; a <= e; a++) {
-			const uint32_t pa = sm.pos[a];
-			const double da = raw_d[pa];
-			const uint32_t ia = caller_index(order, raw_ipar[pa]);
+			const uint32_t pa = pos[a];
+			const double da = sm.d[pa];
 			int c = a;
 			while (c > i) {
-				const uint32_t pc = sm.pos[c - 1];
-				const double dc = raw_d[pc];
-				if (dc < da || (dc == da && caller_index(order, raw_ipar[pc]) < ia)) break;
-				sm.pos[c] = pc;
+				const uint32_t pc = pos[c - 1];
+				const double dc = sm.d[pc];
+				if (dc < da || (dc == da && caller_index(io.order, raw[pc]) < caller_index(io.order, raw[pa]))) break;
+				pos[c] = pc;
 				c--;
 			}
-			sm.pos[c] = pa;
+			pos[c] = pa;
 		}
 	}
 	__syncthreads();
-	for (int i = threadIdx.x; i < n; i += TPR)
-		put_sorted_hit(h0 + i, sm.pos[i], raw_ipar, raw_d, raw_b, out_ipar, out_d, out_b, want_kern, psml, P);
+	for (int i = threadIdx.x; i < n; i += TPR) {
+		const uint32_t p = pos[i];
+		put_sorted_hit(io, P, h0 + i, raw[p], sm.d[p], s, dir);
+	}
 	__syncthreads();     // shared memory is reused by the next ray
 	}
 }
 
 template <int TPR, int IPT>
 size_t sort_smem_bytes() {
-	return sizeof(typename cub::BlockRadixSort<uint32_t, TPR, IPT, uint32_t, 4>::TempStorage) + 8 * TPR * IPT +
-			16 * (TPR / 32) + 128;
+	return sizeof(SortSmem<TPR, IPT>);
 }
 
 // Rays with more hits than the largest class (PSG_SORT_MAX), a block of
@@ -418,27 +466,24 @@ struct LongHitLess {
 	}
 };
 __global__ void __launch_bounds__(LONG_NT) k_sort_long(const uint32_t *__restrict__ list,
-		const unsigned long long *__restrict__ d_nlist, const int64_t *__restrict__ off, size_t scap,
-		const uint32_t *__restrict__ slab_ipar, const double *__restrict__ slab_d, const double *__restrict__ slab_b,
-		uint32_t *__restrict__ out_ipar, double *__restrict__ out_d, double *__restrict__ out_b, int want_kern,
-		const float4 *__restrict__ psml, PhysParams P, const uint32_t *__restrict__ order, LongHit *tmp, size_t hb,
-		size_t slab_r0) {
+		const unsigned long long *__restrict__ d_nlist, const SortIO io, PhysParams P, LongHit *tmp, size_t hb) {
 	__shared__ LongHit tile[2 * LONG_NT];
 	const LongHit pad{__longlong_as_double(0x7ff0000000000000ll), ~0ull};
 	const unsigned long long nlist = *d_nlist;
 	for (unsigned long long li = blockIdx.x; li < nlist; li += gridDim.x) {
 		const size_t r = list[li];
-		const int64_t h0 = off[r];
-		const int64_t n = off[r + 1] - h0;
-		const uint32_t *raw_ipar = slab_ipar + (r - slab_r0) * scap;
-		const double *raw_d = slab_d + (r - slab_r0) * scap, *raw_b = slab_b + (r - slab_r0) * scap;
+		const int64_t h0 = io.off[r];
+		const int64_t n = io.off[r + 1] - h0;
+		const uint32_t *raw = io.slab + (r - io.slab_r0) * io.scap;
+		float s[3], dir[3];
+		io.ray(r, s, dir);
 		LongHit *a = tmp + h0;
 		for (int64_t i = threadIdx.x; i < n; i += LONG_NT)
-			a[i] = LongHit{raw_d[i], (unsigned long long)caller_index(order, raw_ipar[i]) << 32 | (unsigned long long)i};
+			a[i] = LongHit{hit_d(s, io.psml[raw[i]]),
+					(unsigned long long)caller_index(io.order, raw[i]) << 32 | (unsigned long long)i};
 		const LongHit *f = block_sort_global<LONG_NT>(a, tmp + hb + h0, n, tile, pad, LongHitLess());
 		for (int64_t i = threadIdx.x; i < n; i += LONG_NT)
-			put_sorted_hit(h0 + i, (uint32_t)f[i].ck, raw_ipar, raw_d, raw_b, out_ipar, out_d, out_b, want_kern,
-					psml, P);
+			put_sorted_hit(io, P, h0 + i, raw[(uint32_t)f[i].ck], f[i].d, s, dir);
 		__syncthreads();
 	}
 }
@@ -472,6 +517,23 @@ inline unsigned blocks(size_t n, int bs) { return (unsigned)((n + bs - 1) / bs);
 
 // S_COUNT during a traversal: the hit counts (nray + 1, u32), then their
 // exclusive scan (nray + 2, u64) at the next 16-byte boundary
+const void *trace_kernel(const psg_context *ctx) {
+	return ctx->ppc == 8 ? (const void *)k_trace_stack<8> : (const void *)k_trace_stack<0>;
+}
+size_t trace_smem(const psg_context *ctx, int warps) {
+	return sizeof(int) * (TR_STACK + 32 * (size_t)ctx->ppc + 32) * warps;
+}
+void launch_trace(psg_context *ctx, unsigned grid, int warps, const psg_ray *rays, size_t nray, uint32_t *count,
+		size_t scap, uint32_t *slab, unsigned long long *next_ray, const unsigned *nlim) {
+	const size_t smem = trace_smem(ctx, warps);
+	if (ctx->ppc == 8)
+		k_trace_stack<8><<<grid, 32 * warps, smem, ctx->stream>>>(rays, nray, ctx->d_wide_lo, ctx->d_wide_hi,
+				ctx->d_leaf_psml, ctx->d_leaf_idx, 8, count, scap, slab, next_ray, ctx->d_status, nlim);
+	else
+		k_trace_stack<0><<<grid, 32 * warps, smem, ctx->stream>>>(rays, nray, ctx->d_wide_lo, ctx->d_wide_hi,
+				ctx->d_leaf_psml, ctx->d_leaf_idx, ctx->ppc, count, scap, slab, next_ray, ctx->d_status, nlim);
+	ctx->launches++;
+}
 size_t count_bytes(size_t nray) { return 16 * ((sizeof(uint32_t) * (nray + 1) + 15) / 16) + 8 * (nray + 2) + 64; }
 unsigned long long *count_scan(uint32_t *count, size_t nray) {
 	return (unsigned long long *)((char *)count + 16 * ((sizeof(uint32_t) * (nray + 1) + 15) / 16));
@@ -556,8 +618,8 @@ static SrcHits src_hits(psg_context *ctx) {
 int psg_trace_src_batch(psg_context *ctx, const psg_ray *d_rays, size_t nray) {
 	PsgTraceFill tf;
 	int rc = psg_trace_fill(ctx, d_rays, nray, &tf);
-	if (!rc) rc = psg_trace_sort_prepare(ctx, nray, tf.nhit, tf.maxcount);
-	if (!rc) rc = psg_trace_sort_enqueue(ctx, nray, tf.nhit, tf.maxcount, 1, 0);
+	if (!rc) rc = psg_trace_sort_prepare(ctx, nray, tf.nhit, tf.maxcount, 1);
+	if (!rc) rc = psg_trace_sort_enqueue(ctx, d_rays, nullptr, nray, tf.maxcount, 1, 0);
 	if (rc) return rc;
 	// the layout depends on a grow-only capacity, not on this call's hit
 	// total, so that calls of similar totals share one captured tick graph
@@ -596,18 +658,13 @@ int psg_trace_rec_fill_enqueue(psg_context *ctx, const psg_ray *buf, size_t R, s
 	unsigned long long *d_max = ctx->d_counters + 4;
 	unsigned long long *next_ray = ctx->d_counters + 9;
 	const size_t scap = ctx->slab_cap;
-	const size_t slots = cap_rec * scap;
 	uint32_t *slab_ipar = (uint32_t *)ctx->scratch[S_REC_U32].p;
-	double *slab_f64 = (double *)ctx->scratch[S_REC_F64].p;
 	const int trw = std::max(1, std::min(TR_MAX_WARPS, ctx->tune.trace_warps));
-	const size_t smem = sizeof(int) * (TR_STACK + 32 * (size_t)ctx->ppc + 32) * trw;
 	const SrcHits h = src_hits(ctx);
 	PSG_CUDA(cudaMemsetAsync(count, 0, sizeof(uint32_t) * (nray + 1), st));
 	PSG_CUDA(cudaMemsetAsync(d_max, 0, 2 * sizeof(unsigned long long), st));
 	PSG_CUDA(cudaMemsetAsync(next_ray, 0, sizeof(unsigned long long), st));
-	k_trace_stack<<<ctx->trace_grid, 32 * trw, smem, st>>>(buf + R, cap_rec, ctx->d_wide_lo, ctx->d_wide_hi,
-			ctx->d_leaf_psml, ctx->d_leaf_idx, ctx->ppc, count + R, scap, slab_ipar, slab_f64, slab_f64 + slots,
-			next_ray, ctx->d_status, nlim);
+	launch_trace(ctx, ctx->trace_grid, trw, buf + R, cap_rec, count + R, scap, slab_ipar, next_ray, nlim);
 	PSG_CHECK_LAUNCH();
 	k_rec_counts<<<(unsigned)std::min<size_t>(blocks(nray, 256), 4 * (size_t)ctx->sms), 256, 0, st>>>(B, R, h.off,
 			cap_rec, scap, count, ctx->d_counters + 3, ctx->d_status);
@@ -616,7 +673,7 @@ int psg_trace_rec_fill_enqueue(psg_context *ctx, const psg_ray *buf, size_t R, s
 	k_offsets64<<<blocks(nray + 1, 256), 256, 0, st>>>(scan, count, nray, off64, d_max, cap,
 			ctx->d_counters + 24, ctx->d_status);
 	PSG_CHECK_LAUNCH();
-	ctx->launches += 5;
+	ctx->launches += 4;
 	return PSG_OK;
 }
 
@@ -630,7 +687,7 @@ int psg_trace_rec_sort_enqueue(psg_context *ctx, size_t R, size_t nray, unsigned
 			(double *)ctx->scratch[S_HIT_KERN].p);
 	PSG_CHECK_LAUNCH();
 	ctx->launches++;
-	return psg_trace_sort_enqueue(ctx, nray, 0, maxcount, 1, R);
+	return psg_trace_sort_enqueue(ctx, nullptr, B, nray, maxcount, 1, R);
 }
 
 // Sizes the buffers psg_trace_rec_fill_enqueue uses for nray rays (allocates;
@@ -641,15 +698,14 @@ int psg_trace_fill_prepare(psg_context *ctx, size_t nray) {
 	if (!psg_scratch(ctx, S_COUNT, count_bytes(nray)) ||
 			!psg_scratch(ctx, S_SCAN, sizeof(unsigned long long) * (scan_tiles(nray + 1) + 1)) ||
 			!psg_scratch(ctx, S_OFFSETS, sizeof(int64_t) * (nray + 1) + 256) ||
-			!psg_scratch(ctx, S_REC_U32, sizeof(uint32_t) * (slots ? slots : 1)) ||
-			!psg_scratch(ctx, S_REC_F64, sizeof(double) * 2 * (slots ? slots : 1)))
+			!psg_scratch(ctx, S_REC_U32, sizeof(uint32_t) * (slots ? slots : 1)))
 		return PSG_E_NOMEM;
 	const int trw = std::max(1, std::min(TR_MAX_WARPS, ctx->tune.trace_warps));
-	const size_t smem = sizeof(int) * (TR_STACK + 32 * (size_t)ctx->ppc + 32) * trw;
+	const size_t smem = trace_smem(ctx, trw);
 	if (smem > 48 * 1024)
-		PSG_CUDA(cudaFuncSetAttribute(k_trace_stack, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+		PSG_CUDA(cudaFuncSetAttribute(trace_kernel(ctx), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
 	int per_sm = 1;
-	PSG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trace_stack, 32 * trw, smem));
+	PSG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_kernel(ctx), 32 * trw, smem));
 	ctx->trace_grid = (unsigned)std::min<size_t>(blocks(nray, trw), (size_t)std::max(per_sm, 1) * ctx->sms);
 	return PSG_OK;
 }
@@ -671,31 +727,26 @@ int psg_trace_fill(psg_context *ctx, const psg_ray *d_rays, size_t nray, PsgTrac
 	unsigned long long *d_max = ctx->d_counters + 4;
 	unsigned long long *next_ray = ctx->d_counters + 9;
 	const int sms = ctx->sms;
-	const int ppc = ctx->ppc;
 	const int trw = std::max(1, std::min(TR_MAX_WARPS, ctx->tune.trace_warps));
-	const size_t smem = sizeof(int) * (TR_STACK + 32 * (size_t)ppc + 32) * trw;
+	const size_t smem = trace_smem(ctx, trw);
 	if (smem > 48 * 1024)
-		PSG_CUDA(cudaFuncSetAttribute(k_trace_stack, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+		PSG_CUDA(cudaFuncSetAttribute(trace_kernel(ctx), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
 	size_t scap = 0;
 	unsigned long long hdr[2] = {0, 0};      // longest list, hit total
 	for (int attempt = 0; attempt < 2; attempt++) {
 		scap = ctx->slab_cap ? ctx->slab_cap : 1024;
 		const size_t slots = nray * scap;
 		uint32_t *slab_ipar = (uint32_t *)psg_scratch(ctx, S_REC_U32, sizeof(uint32_t) * (slots ? slots : 1));
-		double *slab_f64 = (double *)psg_scratch(ctx, S_REC_F64, sizeof(double) * 2 * (slots ? slots : 1));
-		if (!slab_ipar || !slab_f64) return PSG_E_NOMEM;
+		if (!slab_ipar) return PSG_E_NOMEM;
 		PSG_CUDA(cudaMemsetAsync(count + nray, 0, sizeof(uint32_t), st));
 		PSG_CUDA(cudaMemsetAsync(d_max, 0, 2 * sizeof(unsigned long long), st));
 		psg_mark_begin(ctx, PSG_K_TRACE_FILL);
 		if (nray) {
 			PSG_CUDA(cudaMemsetAsync(next_ray, 0, sizeof(unsigned long long), st));
 			int per_sm = 1;
-			PSG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trace_stack, 32 * trw, smem));
+			PSG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_kernel(ctx), 32 * trw, smem));
 			const unsigned tgrid = (unsigned)std::min<size_t>(blocks(nray, trw), (size_t)std::max(per_sm, 1) * sms);
-			k_trace_stack<<<tgrid, 32 * trw, smem, st>>>(d_rays, nray, ctx->d_wide_lo,
-					ctx->d_wide_hi, ctx->d_leaf_psml, ctx->d_leaf_idx, ppc, count, scap, slab_ipar,
-					slab_f64, slab_f64 + slots, next_ray, ctx->d_status, nullptr);
-			ctx->launches++;
+			launch_trace(ctx, tgrid, trw, d_rays, nray, count, scap, slab_ipar, next_ray, nullptr);
 		}
 		PSG_CHECK_LAUNCH();
 		psg_mark_end(ctx);
@@ -728,16 +779,16 @@ int psg_trace_fill(psg_context *ctx, const psg_ray *d_rays, size_t nray, PsgTrac
 	return PSG_OK;
 }
 
-// Buffers of the sorted hit lists for up to cap hits: S_HIT_IPAR, S_RAW_D
-// (sorted d at + cap), S_HIT_KERN (b, or the column-density factor), and
-// the class lists. Allocates; call before a stream capture.
-int psg_trace_sort_prepare(psg_context *ctx, size_t nray, size_t cap, unsigned long long maxcount) {
+// Buffers of the sorted hit lists for up to cap hits: S_HIT_IPAR, S_HIT_KERN
+// (b, or with want_kern the column-density factor), without want_kern S_RAW_D
+// (d), and the class lists. Allocates; call before a stream capture.
+int psg_trace_sort_prepare(psg_context *ctx, size_t nray, size_t cap, unsigned long long maxcount, int want_kern) {
 	const size_t hb = cap ? cap : 1;
 	uint32_t *hit_ipar = (uint32_t *)psg_scratch(ctx, S_HIT_IPAR, sizeof(uint32_t) * hb);
-	double *hit_db = (double *)psg_scratch(ctx, S_RAW_D, sizeof(double) * 2 * hb);
+	double *hit_d = want_kern ? nullptr : (double *)psg_scratch(ctx, S_RAW_D, sizeof(double) * hb);
 	double *hit_b = (double *)psg_scratch(ctx, S_HIT_KERN, sizeof(double) * hb);
 	uint32_t *lists = (uint32_t *)psg_scratch(ctx, S_RAYLIST, sizeof(uint32_t) * (SORT_NCLS + 1) * (nray + 1));
-	if (!hit_ipar || !hit_db || !hit_b || !lists) return PSG_E_NOMEM;
+	if (!hit_ipar || (!want_kern && !hit_d) || !hit_b || !lists) return PSG_E_NOMEM;
 	ctx->hit_cap = hb;
 	// the long rays' two halves of (d, key) pairs, at their list offsets
 	if (maxcount > PSG_SORT_MAX && !psg_scratch(ctx, S_KEYS, sizeof(LongHit) * 2 * hb)) return PSG_E_NOMEM;
@@ -774,20 +825,24 @@ int psg_sort_classes(unsigned long long maxcount) {
 // Launch sizes are fixed by nray (the persistent class kernels read their
 // ray counts on the device), so it can be captured in a graph; with
 // maxcount above PSG_SORT_MAX the long rays' kernel runs too.
-int psg_trace_sort_enqueue(psg_context *ctx, size_t nray, size_t nhit, unsigned long long maxcount,
-		int want_kern, size_t r0) {
-	(void)nhit;
+// B: the rays are read from it on the device (a captured batch), else rays.
+int psg_trace_sort_enqueue(psg_context *ctx, const psg_ray *rays, const PsgBatchDev *B, size_t nray,
+		unsigned long long maxcount, int want_kern, size_t r0) {
 	cudaStream_t st = ctx->stream;
 	const size_t hb = ctx->hit_cap;
-	const size_t scap = ctx->slab_cap;
-	const size_t slots = (nray - r0) * scap;
-	int64_t *off64 = (int64_t *)ctx->scratch[S_OFFSETS].p;
-	uint32_t *hit_ipar = (uint32_t *)ctx->scratch[S_HIT_IPAR].p;
-	double *hit_d = (double *)ctx->scratch[S_RAW_D].p + hb;
-	double *hit_b = (double *)ctx->scratch[S_HIT_KERN].p;
-	uint32_t *slab_ipar = (uint32_t *)ctx->scratch[S_REC_U32].p;
-	double *slab_d = (double *)ctx->scratch[S_REC_F64].p;
-	double *slab_b = slab_d + slots;
+	SortIO io;
+	io.rays = rays;
+	io.B = B;
+	io.off = (const int64_t *)ctx->scratch[S_OFFSETS].p;
+	io.scap = ctx->slab_cap;
+	io.slab_r0 = r0;
+	io.slab = (const uint32_t *)ctx->scratch[S_REC_U32].p;
+	io.out_ipar = (uint32_t *)ctx->scratch[S_HIT_IPAR].p;
+	io.out_d = want_kern ? nullptr : (double *)ctx->scratch[S_RAW_D].p;
+	io.out_b = (double *)ctx->scratch[S_HIT_KERN].p;
+	io.want_kern = want_kern;
+	io.psml = ctx->d_psml;
+	io.order = ctx->d_order;
 	if (nray <= r0) return PSG_OK;
 	psg_mark_begin(ctx, PSG_K_SORT);
 	{
@@ -795,7 +850,7 @@ int psg_trace_sort_enqueue(psg_context *ctx, size_t nray, size_t nhit, unsigned 
 		unsigned long long *d_ncls = ctx->d_counters + 16, *d_nlong = ctx->d_counters + 25;
 		PSG_CUDA(cudaMemsetAsync(d_ncls, 0, SORT_NCLS * sizeof(unsigned long long), st));
 		PSG_CUDA(cudaMemsetAsync(d_nlong, 0, sizeof(unsigned long long), st));
-		k_sort_classify<<<blocks(nray - r0, 256), 256, 0, st>>>(r0, nray, off64, lists, nray + 1, d_ncls, d_nlong);
+		k_sort_classify<<<blocks(nray - r0, 256), 256, 0, st>>>(r0, nray, io.off, lists, nray + 1, d_ncls, d_nlong);
 		PSG_CHECK_LAUNCH();
 		const PhysParams PP = psg_phys_params(ctx);
 		const size_t stride = nray + 1;
@@ -805,8 +860,7 @@ int psg_trace_sort_enqueue(psg_context *ctx, size_t nray, size_t nhit, unsigned 
 		auto launch_block = [&](auto kern, int tpr, size_t smem, int c) -> int {
 			if (c >= ncls) return PSG_OK;
 			const unsigned grid = (unsigned)std::min<size_t>(nray - r0, (size_t)ctx->sort_grid[c]);
-			kern<<<grid, tpr, smem, st>>>(lists + c * stride, d_ncls + c, off64, scap, slab_ipar, slab_d,
-					slab_b, hit_ipar, hit_d, hit_b, want_kern, ctx->d_psml, PP, ctx->d_order, r0);
+			kern<<<grid, tpr, smem, st>>>(lists + c * stride, d_ncls + c, io, PP);
 			PSG_CHECK_LAUNCH();
 			ctx->launches++;
 			return PSG_OK;
@@ -824,9 +878,8 @@ int psg_trace_sort_enqueue(psg_context *ctx, size_t nray, size_t nhit, unsigned 
 		if (maxcount > PSG_SORT_MAX) {
 			// rays longer than the shared-memory classes: a block each
 			const unsigned grid = (unsigned)std::min<size_t>(nray - r0, (size_t)ctx->sms);
-			k_sort_long<<<grid, LONG_NT, 0, st>>>(lists + SORT_NCLS * stride, d_nlong, off64, scap, slab_ipar,
-					slab_d, slab_b, hit_ipar, hit_d, hit_b, want_kern, ctx->d_psml, PP, ctx->d_order,
-					(LongHit *)ctx->scratch[S_KEYS].p, hb, r0);
+			k_sort_long<<<grid, LONG_NT, 0, st>>>(lists + SORT_NCLS * stride, d_nlong, io, PP,
+					(LongHit *)ctx->scratch[S_KEYS].p, hb);
 			PSG_CHECK_LAUNCH();
 			ctx->launches++;
 		}
@@ -837,15 +890,15 @@ int psg_trace_sort_enqueue(psg_context *ctx, size_t nray, size_t nhit, unsigned 
 
 // Traces nray device-resident rays: fill, buffers sized to the hits, sort.
 // Leaves in scratch: S_OFFSETS, S_HIT_IPAR (sorted leaf-order indices),
-// S_RAW_D (sorted d at + hit_cap) and S_HIT_KERN (sorted b, or with
+// S_RAW_D (sorted d, without want_kern) and S_HIT_KERN (sorted b, or with
 // want_kern the column-density factor).
 int psg_trace_internal(psg_context *ctx, const psg_ray *d_rays, size_t nray, int want_kern) {
 	PsgTraceFill tf;
 	int rc = psg_trace_fill(ctx, d_rays, nray, &tf);
 	if (rc) return rc;
-	rc = psg_trace_sort_prepare(ctx, nray, tf.nhit, tf.maxcount);
+	rc = psg_trace_sort_prepare(ctx, nray, tf.nhit, tf.maxcount, want_kern);
 	if (rc) return rc;
-	return psg_trace_sort_enqueue(ctx, nray, tf.nhit, tf.maxcount, want_kern, 0);
+	return psg_trace_sort_enqueue(ctx, d_rays, nullptr, nray, tf.maxcount, want_kern, 0);
 }
 
 __global__ void k_caller_index(size_t n, const uint32_t *__restrict__ in, const uint32_t *__restrict__ order,
@@ -875,7 +928,7 @@ static int download_hits(psg_context *ctx, size_t nray, int64_t *offsets, psg_xt
 	if (nhit) {
 		std::vector<uint32_t> ip(nhit);
 		std::vector<double> d(nhit), b(nhit);
-		double *hit_d = (double *)ctx->scratch[S_RAW_D].p + ctx->hit_cap;
+		double *hit_d = (double *)ctx->scratch[S_RAW_D].p;
 		// hits carry internal particle positions: the caller's indices
 		const uint32_t *hit_ipar = (const uint32_t *)ctx->scratch[S_HIT_IPAR].p;
 		if (ctx->d_order) {

@@ -240,12 +240,15 @@ __global__ void k_emit_wide(Cells c, int ncell, float4 *__restrict__ out_lo, flo
 
 // The traversal's copy of the particles in the box (the first nvalid of the
 // leaf order, which the particle arrays are already in) and their index,
-// marked when flagged PF_INVALID (psystem.h:28).
+// marked when flagged PF_INVALID (psystem.h:28); a flagged one's copy has no
+// position (NaN), which sends it to the line test's look at the mark.
 __global__ void k_gather_particles(size_t nvalid, const float4 *__restrict__ psml, const int8_t *__restrict__ flag,
 		float4 *__restrict__ lpsml, uint32_t *__restrict__ lidx) {
 	const size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
 	if (k >= nvalid) return;
-	lpsml[k] = psml[k];
+	float4 q = psml[k];
+	if (flag[k] & 1) q.x = __int_as_float(0x7fffffff);
+	lpsml[k] = q;
 	lidx[k] = (uint32_t)k | ((flag[k] & 1) ? PSG_INVALID_BIT : 0u);
 }
 
@@ -384,7 +387,7 @@ extern "C" int psg_build_tree(psg_context *ctx, int ppc) {
 	// 4: bottom-up sizes and boxes
 	for (int l = nlevels - 1; l >= 0; l--) {
 		const int b = level_begin[l], e = level_end[l];
-		k_bottom_up<<<blocks(e - b, 128), 128, 0, st>>>(c, b, e, ctx->d_leaf_psml);
+		k_bottom_up<<<blocks(e - b, 128), 128, 0, st>>>(c, b, e, ctx->d_psml);
 		PSG_CHECK_LAUNCH();
 	}
 	// 5: depth-first numbering and output
