@@ -274,16 +274,23 @@ __device__ __forceinline__ bool below_cutoff(double TM, double Nph) {
 	return TM < 0.0 || __ddiv_rn(TM, Nph) < 1e-10;
 }
 
-// Deposit of one ray by a group of NT threads (a warp, a 128-thread quarter
-// or a whole block): hits are taken NT at a time; optical depths are summed
-// with an FP64 scan over the group; the first hit whose absorption exceeds
-// its neutral atoms (loop.c:482-485) or after which TM/Nph < 1e-10
-// (loop.c:585) is found with a group min, settled by its own thread, and the
-// scan restarts after it (or, in the AFF form, the rest of the step goes to
-// settle_capped()). Transmitted photons before hit j are
-// TM*exp(-(sum of earlier tau)); after it, TM_j minus the absorbed photons,
-// as loop.c:580 updates TM. Each hit writes photons/NH at its index, or -1
-// where the reference deposits nothing. wsum and wb carry the per-warp scan
+// Deposit of one ray. Its hits are taken in steps of V (32, 128 or 512, by
+// the ray's length: psg_tune's thresholds), which fix the arithmetic: optical
+// depths are summed with an FP64 scan over the step (within 32 hits, then
+// over these sums in order); the first hit whose absorption exceeds its
+// neutral atoms (loop.c:482-485) or after which TM/Nph < 1e-10 (loop.c:585)
+// is settled on its own, and the scan restarts after it (or, in the AFF form,
+// the rest of the step goes to settle_capped()). Transmitted photons before
+// hit j are TM*exp(-(sum of earlier tau)); after it, TM_j minus the absorbed
+// photons, as loop.c:580 updates TM. Each hit writes photons/NH at its index,
+// or -1 where the reference deposits nothing.
+//
+// The group of E threads (a warp, a 128-thread quarter or the whole block)
+// that executes a step may be narrower than it: it then takes the step in
+// chunks of E hits and carries the sums from chunk to chunk, in the same
+// order, so the deposits do not depend on E. A warp needs no barriers and
+// wastes fewer lanes on a ray's end, a wide group ends a long ray sooner:
+// k_ray_class chooses by the tick's load. wsum and wb carry the per-warp scan
 // totals (wb: the affine maps' offsets).
 struct DepShared {
 	double wsum[32];
@@ -318,106 +325,222 @@ __device__ __forceinline__ void acc_store(double *__restrict__ acc, int nacc, ui
 	}
 }
 
+// What a deposit reads of a hit: the column-density factor and its
+// particle's neutral fractions and mass.
+template <bool GEN>
+struct DepHit {
+	double kern, lam, l1, l2;
+	float mass;
+	__device__ __forceinline__ void load(int64_t h, bool state, const uint32_t *__restrict__ hipar,
+			const double *__restrict__ hkern, const double *__restrict__ lambdaH, const float *__restrict__ mass_,
+			const PhysParams &P) {
+		const uint32_t p = hipar[h];
+		kern = hkern[h];
+		if (state) {
+			lam = lambdaH[p];
+			mass = mass_[p];
+			if (GEN) {
+				l1 = P.lamHeI[p];
+				l2 = P.lamHeII[p];
+			}
+		}
+	}
+};
+// ... and makes of it (hydrogen)
+struct DepTau {
+	double tau, NHI, NH_inv;
+	__device__ __forceinline__ DepTau() : tau(0.0), NHI(0.0), NH_inv(0.0) {}
+	__device__ __forceinline__ DepTau(const DepHit<false> &x, double sigma, const PhysParams &P) {
+		const double NH = rn_dmul((double)x.mass, P.H_PER_MASS);
+		NHI = rn_dmul(x.lam, NH);
+		tau = rn_dmul(sigma, rn_dmul(x.kern, NHI));
+		NH_inv = __ddiv_rn(1.0, NH);
+	}
+};
+
+// Inclusive sum of v over the group's lanes in the step's order, and run,
+// the step's sum before this chunk on entry, after it on return.
+template <int E>
+__device__ __forceinline__ double chunk_scan(double v, double &run, int t, DepShared &sh, int bar) {
+	const int lane = t & 31, wid = t >> 5;
+	constexpr int NW = E / 32;
+	double wi = v;
+#pragma unroll
+	for (int o = 1; o < 32; o <<= 1) {
+		const double u = __shfl_up_sync(0xffffffffu, wi, o);
+		if (lane >= o) wi += u;
+	}
+	double before = run;
+	if (NW == 1) {
+		run += __shfl_sync(0xffffffffu, wi, 31);
+	} else {
+		if (lane == 31) sh.wsum[wid] = wi;
+		if (t == 0) sh.first = E;
+		group_sync<E>(bar);
+#pragma unroll
+		for (int k = 0; k < NW; k++) {
+			const double u = sh.wsum[k];
+			if (k < wid) before += u;
+			run += u;
+		}
+	}
+	return before + wi;
+}
+// The chunk's first lane with ev (E: none). For wide groups sh.first has been
+// set to E since the last use (chunk_scan).
+template <int E>
+__device__ __forceinline__ int chunk_first(bool ev, int t, DepShared &sh, int bar) {
+	if (E == 32) {
+		const unsigned b = __ballot_sync(0xffffffffu, ev);
+		return b ? __ffs(b) - 1 : E;
+	}
+	if (ev) atomicMin(&sh.first, t);
+	group_sync<E>(bar);
+	return sh.first;
+}
+// lane f's value in all lanes
+template <int E>
+__device__ __forceinline__ double chunk_bcast(double v, int f, int t, DepShared &sh, int bar) {
+	if (E == 32) return __shfl_sync(0xffffffffu, v, f);
+	if (t == f) sh.tm = v;
+	group_sync<E>(bar);
+	return sh.tm;
+}
+
 // Past a capped hit f the step mixes capped hits, which take TM to
 // TM - NHI (loop.c:482-485, 580), and uncapped ones, TM to TM*exp(-tau):
-// affine maps, whose composition is associative. A group scan of the maps
-// gives TM before every hit for a guessed capped/uncapped pattern; the hits
-// before the first whose decision (or the 1e-10 cut) disagrees with the
+// affine maps, whose composition is associative. A scan of the maps over the
+// step gives TM before every hit for a guessed capped/uncapped pattern; the
+// hits before the first whose decision (or the 1e-10 cut) disagrees with the
 // guess are settled, that one is settled from its exact TM, and the next
 // pass guesses from this pass's decisions. TM changes slowly along a capped
 // run, so a step settles in a few passes instead of one per capped hit.
-// Called by every thread of the group with start = f + 1 and TM after f;
-// returns with the step settled (or the ray done). The deposit takes this
-// form (AFF) when the previous batch capped more than 1e-3 of its hits: on
-// a ray with few capped hits, its registers slow the common path.
-template <int NT>
-__device__ __forceinline__ void settle_capped(int t, bool valid, double tau, double NHI, double NH_inv, double Nph,
-		int start, double &TM, bool &done, double &delta, unsigned &nsat, DepShared &sh, int bar) {
+// Called by every thread of the group in chunk c0 of the step at base with
+// cur, delta the chunk's own hit, start = the step's index of f + 1 and TM
+// after f; returns with the step settled (or the ray done), the later
+// chunks' deposits stored. A group narrower than the step reads those
+// chunks' hits again in every pass and keeps a bit of guess per chunk. The
+// deposit takes this form (AFF) when the previous batch capped more than
+// 1e-3 of its hits: on a ray with few capped hits, its registers slow the
+// common path.
+template <int E>
+__device__ __forceinline__ void settle_capped(int V, int t, int c0, int64_t base, int64_t h1, const DepTau &cur, bool cur_valid,
+		double sigma, double Nph, double heat_factor, const uint32_t *__restrict__ hipar,
+		const double *__restrict__ hkern, const double *__restrict__ lambdaH, const float *__restrict__ mass,
+		const PhysParams &P, int want_heat, double *__restrict__ acc, int start, double &TM, bool &done, double &delta,
+		unsigned &nsat, DepShared &sh, int bar) {
 	const int lane = t & 31, wid = t >> 5;
-	constexpr int NW = NT / 32;
-	const double m1 = (valid && tau != 0.0) ? -expm1(-tau) : 0.0;
-	bool pcap = valid && t >= start && tau != 0.0 && TM * m1 > NHI;
-	while (start < NT) {
-		const bool pb = valid && t >= start && tau != 0.0;
-		double A = 1.0, B = 0.0;            // this hit's map, TM -> A*TM + B
-		if (pb) {
-			if (pcap) B = -NHI;
-			else A = 1.0 - m1;
+	constexpr int NW = E / 32;
+	const int nc = (int)min((int64_t)(V / E), (h1 - base + E - 1) / E);
+	auto hit = [&](int c, bool &valid) {
+		if (c == c0) {
+			valid = cur_valid;
+			return cur;
 		}
-#pragma unroll
-		for (int o = 1; o < 32; o <<= 1) {
-			const double pa = __shfl_up_sync(0xffffffffu, A, o);
-			const double pv = __shfl_up_sync(0xffffffffu, B, o);
-			if (lane >= o) {
-				B = A * pv + B;
-				A = A * pa;
+		const int64_t h = base + c * E + t;
+		valid = h < h1;
+		if (!valid) return DepTau();
+		DepHit<false> x;
+		x.load(h, true, hipar, hkern, lambdaH, mass, P);
+		return DepTau(x, sigma, P);
+	};
+	auto put = [&](int c, double d) {
+		if (c == c0) delta = d;
+		else acc_store(acc, want_heat ? 2 : 1, (uint32_t)(base + c * E + t), d,
+				want_heat && d >= 0.0 ? rn_dmul(heat_factor, d) : 0.0, 0.0, 0.0);
+	};
+	// the first guess: every hit capped that TM after f would cap
+	unsigned guess = 0;
+	for (int c = c0; c < nc; c++) {
+		bool valid;
+		const DepTau x = hit(c, valid);
+		if (valid && c > c0) put(c, -1.0);
+		const double m1 = (valid && x.tau != 0.0) ? -expm1(-x.tau) : 0.0;
+		if (valid && c * E + t >= start && x.tau != 0.0 && TM * m1 > x.NHI) guess |= 1u << c;
+	}
+	while (start < V) {
+		double ra = 1.0, rb = 0.0;           // the maps of the step's chunks so far
+		int m = V;                           // the first hit whose decision disagrees
+		double TMm = 0.0;
+		unsigned next = 0;
+		for (int c = start / E; c < nc; c++) {
+			bool valid;
+			const DepTau x = hit(c, valid);
+			const bool pcap = (guess >> c) & 1u;
+			const bool pb = valid && c * E + t >= start && x.tau != 0.0;
+			const double m1 = pb ? -expm1(-x.tau) : 0.0;
+			double A = 1.0, B = 0.0;            // this hit's map, TM -> A*TM + B
+			if (pb) {
+				if (pcap) B = -x.NHI;
+				else A = 1.0 - m1;
 			}
-		}
-		// the maps of the hits before this one: the lower lanes', after
-		// the earlier warps'
-		double xa = __shfl_up_sync(0xffffffffu, A, 1), xb = __shfl_up_sync(0xffffffffu, B, 1);
-		if (lane == 0) { xa = 1.0; xb = 0.0; }
-		double ta = A, tb = B;               // the whole step's map
-		if (NW > 1) {
-			if (lane == 31) { sh.wsum[wid] = A; sh.wb[wid] = B; }
-			if (t == 0) sh.first = NT;
-			group_sync<NT>(bar);
-			double ea = 1.0, eb = 0.0;
-			ta = 1.0;
-			tb = 0.0;
 #pragma unroll
-			for (int k = 0; k < NW; k++) {
-				const double wa = sh.wsum[k], wb = sh.wb[k];
-				if (k < wid) {
-					eb = wa * eb + wb;
-					ea = wa * ea;
+			for (int o = 1; o < 32; o <<= 1) {
+				const double pa = __shfl_up_sync(0xffffffffu, A, o);
+				const double pv = __shfl_up_sync(0xffffffffu, B, o);
+				if (lane >= o) {
+					B = A * pv + B;
+					A = A * pa;
 				}
-				tb = wa * tb + wb;
-				ta = wa * ta;
 			}
-			xb = xa * eb + xb;
-			xa = xa * ea;
-		} else {
-			ta = __shfl_sync(0xffffffffu, A, 31);
-			tb = __shfl_sync(0xffffffffu, B, 31);
+			// the maps of the hits before this one: the lower lanes', after
+			// the earlier warps'
+			double xa = __shfl_up_sync(0xffffffffu, A, 1), xb = __shfl_up_sync(0xffffffffu, B, 1);
+			if (lane == 0) { xa = 1.0; xb = 0.0; }
+			double ea = ra, eb = rb;
+			if (NW > 1) {
+				if (lane == 31) { sh.wsum[wid] = A; sh.wb[wid] = B; }
+				if (t == 0) sh.first = E;
+				group_sync<E>(bar);
+#pragma unroll
+				for (int k = 0; k < NW; k++) {
+					const double wa = sh.wsum[k], wb = sh.wb[k];
+					if (k < wid) {
+						eb = wa * eb + wb;
+						ea = wa * ea;
+					}
+					rb = wa * rb + wb;
+					ra = wa * ra;
+				}
+			} else {
+				const double wa = __shfl_sync(0xffffffffu, A, 31), wb = __shfl_sync(0xffffffffu, B, 31);
+				rb = wa * rb + wb;
+				ra = wa * ra;
+			}
+			if (V > 32) {
+				xb = xa * eb + xb;
+				xa = xa * ea;
+			}
+			double absorb = 0.0, after = 0.0;
+			bool cap = false, bad = false;
+			if (pb) {
+				const double TMj = xa * TM + xb;
+				absorb = TMj * m1;
+				cap = absorb > x.NHI;
+				after = cap ? TMj - x.NHI : TMj - absorb;
+				bad = (cap != pcap) || below_cutoff(after, Nph);
+			}
+			if (cap) next |= 1u << c;
+			if (m == V) {
+				const int f = chunk_first<E>(bad, t, sh, bar);
+				if (pb && t <= f) {        // the settled hits, and hit m from its exact TM
+					put(c, rn_dmul(cap ? x.NHI : absorb, x.NH_inv));
+					if (cap) nsat++;
+				}
+				if (f < E) {
+					m = c * E + f;
+					TMm = chunk_bcast<E>(after, f, t, sh, bar);
+				}
+			}
+			group_sync<E>(bar);       // shared words are rewritten by the next scan
 		}
-		double TMj = 0.0, absorb = 0.0, after = 0.0;
-		bool cap = false, bad = false;
-		if (pb) {
-			TMj = xa * TM + xb;
-			absorb = TMj * m1;
-			cap = absorb > NHI;
-			after = cap ? TMj - NHI : TMj - absorb;
-			bad = (cap != pcap) || below_cutoff(after, Nph);
-		}
-		int m;
-		if (NW == 1) {
-			const unsigned ev = __ballot_sync(0xffffffffu, bad);
-			m = ev ? __ffs(ev) - 1 : NT;
-		} else {
-			if (bad) atomicMin(&sh.first, t);
-			group_sync<NT>(bar);
-			m = sh.first;
-		}
-		if (pb && t <= m) {        // the settled hits, and hit m from its exact TM
-			delta = rn_dmul(cap ? NHI : absorb, NH_inv);
-			if (cap) nsat++;
-		}
-		if (m == NT) {
-			TM = ta * TM + tb;
-			group_sync<NT>(bar);       // shared words are rewritten by the next scan
+		if (m == V) {
+			TM = ra * TM + rb;
 			break;
 		}
-		if (NW == 1) {
-			TM = __shfl_sync(0xffffffffu, after, m);
-		} else {
-			if (t == m) sh.tm = after;
-			group_sync<NT>(bar);
-			TM = sh.tm;
-		}
+		TM = TMm;
 		start = m + 1;
-		pcap = cap;
-		group_sync<NT>(bar);
+		guess = next;
 		if (below_cutoff(TM, Nph)) {
 			done = true;
 			break;
@@ -425,13 +548,11 @@ __device__ __forceinline__ void settle_capped(int t, bool valid, double tau, dou
 	}
 }
 
-template <int NT, bool AFF>
-__device__ void deposit_ray(const psg_ray &ray, int64_t h0, int64_t h1, int t,
+template <int E, bool AFF>
+__device__ __forceinline__ void deposit_ray(int V, const psg_ray &ray, int64_t h0, int64_t h1, int t,
 		const uint32_t *__restrict__ hipar, const double *__restrict__ hkern,
 		const double *__restrict__ lambdaH, const float *__restrict__ mass, const PhysParams &P, int want_heat,
 		double *__restrict__ acc, DepShared &sh, unsigned &nsat, double &lost, int bar) {
-	const int lane = t & 31, wid = t >> 5;
-	constexpr int NW = NT / 32;
 	const double Nph = ray.Nph;
 	const double freq = ray.freq;
 	const bool skip_ray = (Nph == 0.0);
@@ -439,117 +560,74 @@ __device__ void deposit_ray(const psg_ray &ray, int64_t h0, int64_t h1, int t,
 	const double heat_factor = rn_dmul(P.H_PER_MASS, fdim(freq, P.HI_ENERGY));
 	double TM = Nph;
 	bool done = skip_ray;
-	// the next step's loads are issued one step ahead
-	double np_kern = 0.0, np_lam = 0.0;
-	float np_mass = 1.0f;
-	{
-		const int64_t h = h0 + t;
-		if (h < h1) {
-			const uint32_t p = hipar[h];
-			np_kern = hkern[h];
-			if (!done) { np_lam = lambdaH[p]; np_mass = mass[p]; }
-		}
-	}
-	for (int64_t base = h0; base < h1; base += NT) {
-		const int64_t h = base + t;
-		const bool valid = h < h1;
-		const double kern_c = np_kern, lam_c = np_lam;
-		const float mass_c = np_mass;
-		const uint32_t slot_c = (uint32_t)h;      // (a hit's deposits sit at its own index)
-		{
-			const int64_t hn = h + NT;
-			if (hn < h1) {
-				const uint32_t p = hipar[hn];
-				np_kern = hkern[hn];
-				if (!done) { np_lam = lambdaH[p]; np_mass = mass[p]; }
-			}
-		}
-		double tau = 0.0, NHI = 0.0, NH_inv = 0.0, delta = -1.0;
-		if (valid && !done) {
-			const double NH = rn_dmul((double)mass_c, P.H_PER_MASS);
-			NHI = rn_dmul(lam_c, NH);
-			tau = rn_dmul(sigma, rn_dmul(kern_c, NHI));
-			NH_inv = __ddiv_rn(1.0, NH);
-		}
-		int start = 0;
-		while (!done && start < NT) {
-			const bool part = valid && t >= start && tau != 0.0;
-			const double my_tau = part ? tau : 0.0;
-			double wi = my_tau;
-#pragma unroll
-			for (int o = 1; o < 32; o <<= 1) {
-				const double v = __shfl_up_sync(0xffffffffu, wi, o);
-				if (lane >= o) wi += v;
-			}
-			double woff = 0.0, total;
-			if (NW == 1) {
-				total = __shfl_sync(0xffffffffu, wi, 31);
-			} else {
-				if (lane == 31) sh.wsum[wid] = wi;
-				if (t == 0) sh.first = NT;
-				group_sync<NT>(bar);
-				total = 0.0;
-#pragma unroll
-				for (int k = 0; k < NW; k++) {
-					const double v = sh.wsum[k];
-					if (k < wid) woff += v;
-					total += v;
+	// the next chunk's loads are issued one chunk ahead
+	DepHit<false> np{0.0, 0.0, 0.0, 0.0, 1.0f};
+	if (h0 + t < h1) np.load(h0 + t, !done, hipar, hkern, lambdaH, mass, P);
+	for (int64_t base = h0; base < h1; base += V) {
+		double run = 0.0;      // the sum of the step's optical depths since its last restart
+		bool settled = false;  // ... by settle_capped()
+		for (int c = 0; c * E < V && base + c * E < h1 && !settled; c++) {
+			const int64_t h = base + c * E + t;
+			const bool valid = h < h1;
+			DepTau x;
+			double delta = -1.0;
+			if (valid && !done) x = DepTau(np, sigma, P);
+			if (h + E < h1) np.load(h + E, !done, hipar, hkern, lambdaH, mass, P);
+			int start = 0;
+			while (!done && start < E) {
+				const bool part = valid && t >= start && x.tau != 0.0;
+				const double my_tau = part ? x.tau : 0.0;
+				double after_run = run;
+				const double incl = chunk_scan<E>(my_tau, after_run, t, sh, bar);
+				double TMj = 0.0, absorb = 0.0, TMafter = 0.0;
+				bool capped = false, cut = false;
+				if (part) {
+					const double excl = incl - my_tau;
+					TMj = TM * exp(-excl);
+					absorb = TMj * -expm1(-my_tau);
+					TMafter = TMj - absorb;
+					capped = absorb > x.NHI;
+					cut = below_cutoff(TMafter, Nph);
+				}
+				const int f = chunk_first<E>(capped || cut, t, sh, bar);
+				if (part && t < f) delta = rn_dmul(absorb, x.NH_inv);
+				if (f == E) {
+					run = after_run;
+					group_sync<E>(bar);       // shared words are rewritten by the next scan
+					break;
+				}
+				double TMnew = 0.0;
+				if (t == f) {
+					TMnew = TMafter;
+					if (capped) {
+						absorb = x.NHI;
+						TMnew = TMj - x.NHI;
+						nsat++;
+					}
+					delta = rn_dmul(absorb, x.NH_inv);
+				}
+				TM = chunk_bcast<E>(TMnew, f, t, sh, bar);
+				run = 0.0;
+				if (below_cutoff(TM, Nph)) done = true;
+				start = f + 1;
+				group_sync<E>(bar);
+				if (AFF && !done) {
+					// f was capped: the rest of the step through the affine-map scan
+					settle_capped<E>(V, t, c, base, h1, x, valid, sigma, Nph, heat_factor, hipar, hkern, lambdaH, mass, P,
+							want_heat, acc, c * E + start, TM, done, delta, nsat, sh, bar);
+					settled = true;
+					break;
 				}
 			}
-			double TMj = 0.0, absorb = 0.0, TMafter = 0.0;
-			bool capped = false, cut = false;
-			if (part) {
-				const double excl = (woff + wi) - my_tau;
-				TMj = TM * exp(-excl);
-				absorb = TMj * -expm1(-my_tau);
-				TMafter = TMj - absorb;
-				capped = absorb > NHI;
-				cut = below_cutoff(TMafter, Nph);
-			}
-			int f;
-			if (NW == 1) {
-				const unsigned ev = __ballot_sync(0xffffffffu, capped || cut);
-				f = ev ? __ffs(ev) - 1 : NT;
-			} else {
-				if (capped || cut) atomicMin(&sh.first, t);
-				group_sync<NT>(bar);
-				f = sh.first;
-			}
-			if (part && t < f) delta = rn_dmul(absorb, NH_inv);
-			if (f == NT) {
-				TM = TM * exp(-total);
-				group_sync<NT>(bar);       // shared words are rewritten by the next step
-				break;
-			}
-			double TMnew = 0.0;
-			if (t == f) {
-				TMnew = TMafter;
-				if (capped) {
-					absorb = NHI;
-					TMnew = TMj - NHI;
-					nsat++;
-				}
-				delta = rn_dmul(absorb, NH_inv);
-				if (NW > 1) sh.tm = TMnew;
-			}
-			if (NW == 1) {
-				TM = __shfl_sync(0xffffffffu, TMnew, f);
-			} else {
-				group_sync<NT>(bar);
-				TM = sh.tm;
-			}
-			if (below_cutoff(TM, Nph)) done = true;
-			start = f + 1;
-			group_sync<NT>(bar);
-			if (AFF && !done) {
-				// f was capped: the rest of the step through the affine-map scan
-				settle_capped<NT>(t, valid, tau, NHI, NH_inv, Nph, start, TM, done, delta, nsat, sh, bar);
-				break;
+			if (valid) {
+				acc_store(acc, want_heat ? 2 : 1, (uint32_t)h, delta,
+						want_heat && delta >= 0.0 ? rn_dmul(heat_factor, delta) : 0.0, 0.0, 0.0);
 			}
 		}
-		if (valid) {
-			acc_store(acc, want_heat ? 2 : 1, slot_c, delta,
-					want_heat && delta >= 0.0 ? rn_dmul(heat_factor, delta) : 0.0, 0.0, 0.0);
+		if (settled) {      // (the loads ahead are of a chunk that has been settled)
+			if (base + V + t < h1) np.load(base + V + t, !done, hipar, hkern, lambdaH, mass, P);
+		} else if (!done) {
+			TM = TM * exp(-run);
 		}
 	}
 	if (t == 0 && !skip_ray) lost += TM;
@@ -562,13 +640,11 @@ __device__ void deposit_ray(const psg_ray &ray, int64_t h0, int64_t h1, int t,
 // increments (nacc of them per hit), with the secondary
 // ionisation and heating of loop.c:513-552 (whose HeII terms the
 // reference's statements drop, loop.c:523,542).
-template <int NT>
-__device__ void deposit_ray_gen(const psg_ray &ray, int64_t h0, int64_t h1, int t,
+template <int E>
+__device__ __forceinline__ void deposit_ray_gen(int V, const psg_ray &ray, int64_t h0, int64_t h1, int t,
 		const uint32_t *__restrict__ hipar, const double *__restrict__ hkern,
 		const double *__restrict__ lambdaH, const float *__restrict__ mass, const PhysParams &P, int want_heat,
 		double *__restrict__ acc, int nacc, DepShared &sh, unsigned &nsat, double &lost, int bar) {
-	const int lane = t & 31, wid = t >> 5;
-	constexpr int NW = NT / 32;
 	const double Nph = ray.Nph;
 	const double freq = ray.freq;
 	const bool skip_ray = (Nph == 0.0);
@@ -578,174 +654,144 @@ __device__ void deposit_ray_gen(const psg_ray &ray, int64_t h0, int64_t h1, int 
 	const double hf0 = P.H_PER_MASS * dE0, hf1 = P.HE_PER_MASS * dE1, hf2 = P.HE_PER_MASS * dE2;
 	double TM = Nph;
 	bool done = skip_ray;
-	// the next step's loads are issued one step ahead
-	double np_kern = 0.0, np_lam = 0.0, np_l1 = 0.0, np_l2 = 0.0;
-	float np_mass = 1.0f;
-	{
-		const int64_t h = h0 + t;
-		if (h < h1) {
-			const uint32_t p = hipar[h];
-			np_kern = hkern[h];
-			if (!done) { np_lam = lambdaH[p]; np_mass = mass[p]; np_l1 = P.lamHeI[p]; np_l2 = P.lamHeII[p]; }
-		}
-	}
-	for (int64_t base = h0; base < h1; base += NT) {
-		const int64_t h = base + t;
-		const bool valid = h < h1;
-		const double kern_c = np_kern, lam_c = np_lam, l1_c = np_l1, l2_c = np_l2;
-		const float mass_c = np_mass;
-		const uint32_t slot_c = (uint32_t)h;      // (a hit's deposits sit at its own index)
-		{
-			const int64_t hn = h + NT;
-			if (hn < h1) {
-				const uint32_t p = hipar[hn];
-				np_kern = hkern[hn];
-				if (!done) { np_lam = lambdaH[p]; np_mass = mass[p]; np_l1 = P.lamHeI[p]; np_l2 = P.lamHeII[p]; }
-			}
-		}
-		// species s = 0 HI, 1 HeI, 2 HeII: atoms N_s, optical depth t_s
-		double tau = 0.0, NHI = 0.0, NH_inv = 0.0, delta = -1.0;
-		double N1 = 0.0, N2 = 0.0, t0 = 0.0, t1 = 0.0, t2 = 0.0, NHe_inv = 0.0, xe = 0.0;
-		double d0 = 0.0, d1 = 0.0, d2 = 0.0;
-		bool he = false;
-		if (valid && !done) {
-			const double NH = (double)mass_c * P.H_PER_MASS;
-			const double NHe = (double)mass_c * P.HE_PER_MASS;
-			NHI = lam_c * NH;
-			t0 = sigma * (kern_c * NHI);
-			tau = 0.0 + t0;
-			he = !P.h_only && NHe != 0.0;
-			if (he) {
-				N1 = l1_c * NHe;
-				t1 = sHeI * (kern_c * N1);
-				tau += t1;
-				N2 = l2_c * NHe;
-				t2 = sHeII * (kern_c * N2);
-				tau += t2;
-			}
-			NH_inv = 1.0 / NH;
-			NHe_inv = 1.0 / NHe;
-			xe = ye_he(P, lam_c, l1_c, l2_c) * NH / (NH + NHe);     // loop.c:512-513
-			if (xe > 1.0) xe = 1.0;
-		}
-		int start = 0;
-		while (!done && start < NT) {
-			const bool part = valid && t >= start && tau != 0.0;
-			const double my_tau = part ? tau : 0.0;
-			double wi = my_tau;
-#pragma unroll
-			for (int o = 1; o < 32; o <<= 1) {
-				const double v = __shfl_up_sync(0xffffffffu, wi, o);
-				if (lane >= o) wi += v;
-			}
-			double woff = 0.0, total;
-			if (NW == 1) {
-				total = __shfl_sync(0xffffffffu, wi, 31);
-			} else {
-				if (lane == 31) sh.wsum[wid] = wi;
-				if (t == 0) sh.first = NT;
-				group_sync<NT>(bar);
-				total = 0.0;
-#pragma unroll
-				for (int k = 0; k < NW; k++) {
-					const double v = sh.wsum[k];
-					if (k < wid) woff += v;
-					total += v;
-				}
-			}
-			double TMj = 0.0, absorb = 0.0, TMafter = 0.0;
-			bool capped = false, cut = false;
-			double a0 = 0.0, a1 = 0.0, a2 = 0.0;
-			if (part) {
-				const double excl = (woff + wi) - my_tau;
-				TMj = TM * exp(-excl);
-				absorb = TMj * -expm1(-my_tau);
-				TMafter = TMj - absorb;
-				a0 = t0 / my_tau * absorb;
-				capped = a0 > NHI;
+	// the next chunk's loads are issued one chunk ahead
+	DepHit<true> np{0.0, 0.0, 0.0, 0.0, 1.0f};
+	if (h0 + t < h1) np.load(h0 + t, !done, hipar, hkern, lambdaH, mass, P);
+	for (int64_t base = h0; base < h1; base += V) {
+		double run = 0.0;      // the sum of the step's optical depths since its last restart
+		for (int c = 0; c * E < V && base + c * E < h1; c++) {
+			const int64_t h = base + c * E + t;
+			const bool valid = h < h1;
+			// species s = 0 HI, 1 HeI, 2 HeII: atoms N_s, optical depth t_s
+			double tau = 0.0, NHI = 0.0, NH_inv = 0.0, delta = -1.0;
+			double N1 = 0.0, N2 = 0.0, t0 = 0.0, t1 = 0.0, t2 = 0.0, NHe_inv = 0.0, xe = 0.0;
+			double d0 = 0.0, d1 = 0.0;
+			double d2 = 0.0;
+			bool he = false;
+			if (valid && !done) {
+				const double NH = (double)np.mass * P.H_PER_MASS;
+				const double NHe = (double)np.mass * P.HE_PER_MASS;
+				NHI = np.lam * NH;
+				t0 = sigma * (np.kern * NHI);
+				tau = 0.0 + t0;
+				he = !P.h_only && NHe != 0.0;
 				if (he) {
-					a1 = t1 / my_tau * absorb;
-					a2 = t2 / my_tau * absorb;
-					capped = capped || a1 > N1 || a2 > N2;
+					N1 = np.l1 * NHe;
+					t1 = sHeI * (np.kern * N1);
+					tau += t1;
+					N2 = np.l2 * NHe;
+					t2 = sHeII * (np.kern * N2);
+					tau += t2;
 				}
-				cut = below_cutoff(TMafter, Nph);
+				NH_inv = 1.0 / NH;
+				NHe_inv = 1.0 / NHe;
+				xe = ye_he(P, np.lam, np.l1, np.l2) * NH / (NH + NHe);     // loop.c:512-513
+				if (xe > 1.0) xe = 1.0;
 			}
-			int f;
-			if (NW == 1) {
-				const unsigned ev = __ballot_sync(0xffffffffu, capped || cut);
-				f = ev ? __ffs(ev) - 1 : NT;
-			} else {
-				if (capped || cut) atomicMin(&sh.first, t);
-				group_sync<NT>(bar);
-				f = sh.first;
-			}
-			if (part && t < f) {
-				d0 = a0 * NH_inv;
-				if (he) { d1 = a1 * NHe_inv; d2 = a2 * NHe_inv; }
-				delta = d0;
-			}
-			if (f == NT) {
-				TM = TM * exp(-total);
-				group_sync<NT>(bar);       // shared words are rewritten by the next step
-				break;
-			}
-			double TMnew = 0.0;
-			if (t == f) {
-				TMnew = TMafter;
-				if (capped) {
-					if (a0 > NHI) { a0 = NHI; nsat++; }
-					double ab = a0;
+			if (h + E < h1) np.load(h + E, !done, hipar, hkern, lambdaH, mass, P);
+			int start = 0;
+			while (!done && start < E) {
+				const bool part = valid && t >= start && tau != 0.0;
+				const double my_tau = part ? tau : 0.0;
+				double after_run = run;
+				const double incl = chunk_scan<E>(my_tau, after_run, t, sh, bar);
+				double TMj = 0.0, absorb = 0.0, TMafter = 0.0;
+				bool capped = false, cut = false;
+				double a0 = 0.0, a1 = 0.0, a2 = 0.0;
+				if (part) {
+					const double excl = incl - my_tau;
+					TMj = TM * exp(-excl);
+					absorb = TMj * -expm1(-my_tau);
+					TMafter = TMj - absorb;
+					a0 = t0 / my_tau * absorb;
+					capped = a0 > NHI;
 					if (he) {
-						if (a1 > N1) { a1 = N1; nsat++; }
-						if (a2 > N2) { a2 = N2; nsat++; }
-						ab += (a1 + a2);
+						a1 = t1 / my_tau * absorb;
+						a2 = t2 / my_tau * absorb;
+						capped = capped || a1 > N1 || a2 > N2;
 					}
-					TMnew = TMj - ab;
+					cut = below_cutoff(TMafter, Nph);
 				}
-				d0 = a0 * NH_inv;
-				if (he) { d1 = a1 * NHe_inv; d2 = a2 * NHe_inv; }
-				delta = d0;
-				if (NW > 1) sh.tm = TMnew;
+				const int f = chunk_first<E>(capped || cut, t, sh, bar);
+				if (part && t < f) {
+					d0 = a0 * NH_inv;
+					if (he) { d1 = a1 * NHe_inv; d2 = a2 * NHe_inv; }
+					delta = d0;
+				}
+				if (f == E) {
+					run = after_run;
+					group_sync<E>(bar);       // shared words are rewritten by the next scan
+					break;
+				}
+				double TMnew = 0.0;
+				if (t == f) {
+					TMnew = TMafter;
+					if (capped) {
+						if (a0 > NHI) { a0 = NHI; nsat++; }
+						double ab = a0;
+						if (he) {
+							if (a1 > N1) { a1 = N1; nsat++; }
+							if (a2 > N2) { a2 = N2; nsat++; }
+							ab += (a1 + a2);
+						}
+						TMnew = TMj - ab;
+					}
+					d0 = a0 * NH_inv;
+					if (he) { d1 = a1 * NHe_inv; d2 = a2 * NHe_inv; }
+					delta = d0;
+				}
+				TM = chunk_bcast<E>(TMnew, f, t, sh, bar);
+				run = 0.0;
+				if (below_cutoff(TM, Nph)) done = true;
+				start = f + 1;
+				group_sync<E>(bar);
 			}
-			if (NW == 1) {
-				TM = __shfl_sync(0xffffffffu, TMnew, f);
-			} else {
-				group_sync<NT>(bar);
-				TM = sh.tm;
+			if (valid) {
+				// loop.c:512-552: yGdep increments and heat of the hit
+				double y0 = delta, y1 = 0.0, y2 = 0.0, heat = 0.0;
+				if (delta >= 0.0) {
+					if (P.secondary && xe > 0.0) {
+						const double lx = log10(xe);
+						y0 = d0 + (d0 * dE0 / P.HI_ENERGY * secion_get(P, 0, dE0, lx) +
+								d1 * dE1 / P.HI_ENERGY * secion_get(P, 0, dE1, lx));
+						heat = hf0 * d0 * secion_get(P, 2, dE0, lx);
+						if (he) {
+							y1 = d1 + (d0 * dE0 / P.HEI_ENERGY * secion_get(P, 1, dE0, lx) +
+									d1 * dE1 / P.HEI_ENERGY * secion_get(P, 1, dE1, lx));
+							heat += hf1 * d1 * secion_get(P, 2, dE1, lx);
+							y2 = d2;
+						}
+					} else {
+						heat = hf0 * d0;
+						if (he) {
+							y1 = d1;
+							y2 = d2;
+							heat += d1 * hf1;
+							heat += d2 * hf2;
+						}
+					}
+				}
+				acc_store(acc, nacc, (uint32_t)h, y0, heat, y1, y2);
 			}
-			if (below_cutoff(TM, Nph)) done = true;
-			start = f + 1;
-			group_sync<NT>(bar);
 		}
-		if (valid) {
-			// loop.c:512-552: yGdep increments and heat of the hit
-			double y0 = delta, y1 = 0.0, y2 = 0.0, heat = 0.0;
-			if (delta >= 0.0) {
-				if (P.secondary && xe > 0.0) {
-					const double lx = log10(xe);
-					y0 = d0 + (d0 * dE0 / P.HI_ENERGY * secion_get(P, 0, dE0, lx) +
-							d1 * dE1 / P.HI_ENERGY * secion_get(P, 0, dE1, lx));
-					heat = hf0 * d0 * secion_get(P, 2, dE0, lx);
-					if (he) {
-						y1 = d1 + (d0 * dE0 / P.HEI_ENERGY * secion_get(P, 1, dE0, lx) +
-								d1 * dE1 / P.HEI_ENERGY * secion_get(P, 1, dE1, lx));
-						heat += hf1 * d1 * secion_get(P, 2, dE1, lx);
-						y2 = d2;
-					}
-				} else {
-					heat = hf0 * d0;
-					if (he) {
-						y1 = d1;
-						y2 = d2;
-						heat += d1 * hf1;
-						heat += d2 * hf2;
-					}
-				}
-			}
-			acc_store(acc, nacc, slot_c, y0, heat, y1, y2);
-		}
+		if (!done) TM = TM * exp(-run);
 	}
 	if (t == 0 && !skip_ray) lost += TM;
+}
+
+// One ray of any length by a group of E threads: the step V of its length
+// class, at least E.
+template <int E, bool GEN, bool AFF>
+__device__ __forceinline__ void deposit_any(const psg_ray &ray, int64_t h0, int64_t h1, int t, int dep_long, int dep_mid,
+		const uint32_t *__restrict__ hipar, const double *__restrict__ hkern, const double *__restrict__ lambdaH,
+		const float *__restrict__ mass, const PhysParams &P, int want_heat, double *__restrict__ acc, int nacc,
+		DepShared &sh, unsigned &nsat, double &lost, int bar) {
+	const int64_t n = h1 - h0;
+	const int V = max(E, n > dep_mid ? 512 : n > dep_long ? 128 : 32);
+	if (GEN)
+		deposit_ray_gen<E>(V, ray, h0, h1, t, hipar, hkern, lambdaH, mass, P, want_heat, acc, nacc, sh, nsat, lost, bar);
+	else
+		deposit_ray<E, AFF>(V, ray, h0, h1, t, hipar, hkern, lambdaH, mass, P, want_heat, acc, sh, nsat, lost, bar);
 }
 
 // A tick's rays by deposit group: long rays (a whole block each), middle
@@ -768,7 +814,7 @@ template <bool GEN, bool AFF>
 __global__ void __launch_bounds__(DEP_THREADS, 2) k_deposit(int t, const TickRays *__restrict__ tick_rays,
 		unsigned *__restrict__ unit_ctr, const PsgBatchDev *__restrict__ B,
 		const uint32_t *__restrict__ long_rays, const uint32_t *__restrict__ mid_rays,
-		const uint32_t *__restrict__ short_rays,
+		const uint32_t *__restrict__ short_rays, int dep_long, int dep_mid,
 		const int64_t *__restrict__ off, const uint32_t *__restrict__ hipar, const double *__restrict__ hkern,
 		const double *__restrict__ lambdaH, const float *__restrict__ mass,
 		PhysParams P, int want_heat, double *__restrict__ acc, int nacc, unsigned long long *__restrict__ n_sat,
@@ -785,46 +831,35 @@ __global__ void __launch_bounds__(DEP_THREADS, 2) k_deposit(int t, const TickRay
 	const int nlong = T.nlong, nmid = T.nmid, nshort = T.nshort;
 	const int nmid_blocks = (nmid + 3) / 4;
 	const int nunits = nlong + nmid_blocks + (nshort + DEP_THREADS / 32 - 1) / (DEP_THREADS / 32);
-	for (;;) {
-		if (tid == 0) s_unit = (int)atomicAdd(unit_ctr + t, 1u);
-		__syncthreads();
-		const int u = s_unit;
-		__syncthreads();       // (also: the previous unit's shared state is no longer read)
-		if (u >= nunits) break;
+	// the first unit is the block's own index, later ones come from the
+	// counter (a tick with no more units than blocks touches it not at all)
+	for (int u = (int)blockIdx.x; u < nunits;) {
 		if (u < nlong) {
 			const uint32_t r = long_rays[T.l0 + u];
-			if (GEN)
-				deposit_ray_gen<DEP_THREADS>(rays[r], off[r], off[r + 1], tid, hipar, hkern, lambdaH, mass, P,
-						want_heat, acc, nacc, sh_block, nsat, tm_lost, 0);
-			else
-				deposit_ray<DEP_THREADS, AFF>(rays[r], off[r], off[r + 1], tid, hipar, hkern, lambdaH, mass, P,
-						want_heat, acc, sh_block, nsat, tm_lost, 0);
+			deposit_any<DEP_THREADS, GEN, AFF>(rays[r], off[r], off[r + 1], tid, dep_long, dep_mid, hipar, hkern, lambdaH,
+					mass, P, want_heat, acc, nacc, sh_block, nsat, tm_lost, 0);
 		} else if (u < nlong + nmid_blocks) {
 			const int q = tid >> 7;
 			const int m = (u - nlong) * 4 + q;
 			if (m < nmid) {
 				const uint32_t r = mid_rays[T.m0 + m];
-				if (GEN)
-					deposit_ray_gen<128>(rays[r], off[r], off[r + 1], tid & 127, hipar, hkern, lambdaH, mass, P,
-							want_heat, acc, nacc, sh_quarter[q], nsat, tm_lost, 1 + q);
-				else
-					deposit_ray<128, AFF>(rays[r], off[r], off[r + 1], tid & 127, hipar, hkern, lambdaH, mass, P,
-							want_heat, acc, sh_quarter[q], nsat, tm_lost, 1 + q);
+				deposit_any<128, GEN, AFF>(rays[r], off[r], off[r + 1], tid & 127, dep_long, dep_mid, hipar, hkern, lambdaH,
+						mass, P, want_heat, acc, nacc, sh_quarter[q], nsat, tm_lost, 1 + q);
 			}
 		} else {
 			const int w = (u - nlong - nmid_blocks) * (DEP_THREADS / 32) + wid;
 			if (w < nshort) {
 				const uint32_t r = short_rays[T.s0 + w];
-				if (off[r + 1] > off[r]) {
-					if (GEN)
-						deposit_ray_gen<32>(rays[r], off[r], off[r + 1], lane, hipar, hkern, lambdaH, mass, P,
-								want_heat, acc, nacc, sh_warp[wid], nsat, tm_lost, 0);
-					else
-						deposit_ray<32, AFF>(rays[r], off[r], off[r + 1], lane, hipar, hkern, lambdaH, mass, P,
-								want_heat, acc, sh_warp[wid], nsat, tm_lost, 0);
-				}
+				if (off[r + 1] > off[r])
+					deposit_any<32, GEN, AFF>(rays[r], off[r], off[r + 1], lane, dep_long, dep_mid, hipar, hkern, lambdaH,
+							mass, P, want_heat, acc, nacc, sh_warp[wid], nsat, tm_lost, 0);
 			}
 		}
+		if (nunits <= (int)gridDim.x) break;
+		if (tid == 0) s_unit = (int)(gridDim.x + atomicAdd(unit_ctr + t, 1u));
+		__syncthreads();
+		u = s_unit;
+		__syncthreads();       // (also: the unit's shared state is no longer read)
 	}
 	for (int o = 16; o > 0; o >>= 1) nsat += __shfl_down_sync(0xffffffffu, nsat, o);
 	if (lane == 0 && nsat) atomicAdd(n_sat, (unsigned long long)nsat);
@@ -852,14 +887,30 @@ __global__ void k_tick_rays(int K, size_t R, size_t nray, const unsigned long lo
 }
 
 // Rays of the batch split into long, middle and short lists (ray order
-// kept): cls = 1 for long, 1 << 32 for middle, so one scan counts both.
-// (dep_long and dep_mid: the thresholds, DEP_LONG and DEP_MID unless tuned)
-__global__ void k_ray_class(size_t nray, const int64_t *__restrict__ off, int dep_long, int dep_mid,
-		unsigned long long *__restrict__ cls) {
+// kept): cls = 1 for long, 1 << 32 for middle, so one scan counts both. Which
+// group executes a ray does not change its deposits; it is at most as wide
+// as the ray's step (psg_tune's thresholds). Where the tick has work for many
+// narrow groups they are better: a warp takes the rays of up to as many hits
+// as each resident warp gets of the tick, a quarter those of up to as many
+// as each resident block gets. Measured (deposit per call, groups as wide as
+// the steps -> by load): 8 x 8192 rays of 690 hits 1.95 -> 1.24 ms, 4 x 65536
+// of 1200 15.8 -> 11.2 ms, 6 x 3100 of 550 0.50 -> 0.41 ms; helium 4 x 8192
+// 5.7 -> 2.6 ms, 8 x 1324 of 320 3.58 -> 1.45 ms. 1024 rays of 120 hits are
+// too few to narrow (26 hits per warp): at 192 instead of 96 the deposit took
+// 2.05 instead of 1.71 ms. The warp's bound stops at DEP_WARP_MAX: past it
+// the longest rays trail the tick (65536 rays of up to 4000 hits: 14.3 ms
+// without the bound; 384, 768 and 1500 measure within 5%).
+#define DEP_WARP_MAX 768
+__global__ void k_ray_class(size_t nray, size_t R, const int64_t *__restrict__ off, int dep_long, int dep_mid,
+		int dep_warps, unsigned long long *__restrict__ cls) {
 	const size_t r = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
 	if (r >= nray) return;
 	const int64_t n = off[r + 1] - off[r];
-	cls[r] = n > dep_mid ? 1ull : (n > dep_long ? (1ull << 32) : 0ull);
+	const size_t t0 = r / R * R;
+	const int64_t H = off[t0 + R] - off[t0];      // the tick's hits
+	const int64_t wlim = max((int64_t)dep_long, min((int64_t)DEP_WARP_MAX, H / dep_warps));
+	const int64_t qlim = max((int64_t)dep_mid, H / (dep_warps / (DEP_THREADS / 32)));
+	cls[r] = n > max(wlim, qlim) ? 1ull : (n > wlim ? (1ull << 32) : 0ull);
 }
 
 // (each list has room for every ray of the batch)
@@ -2154,7 +2205,8 @@ int enqueue_batch(psg_context *ctx, const BatchPlan &pl, const PsgBatchDev *B) {
 	uint32_t *ray_lists = (uint32_t *)ctx->scratch[S_RAYLIST].p;
 	uint32_t *long_rays = ray_lists, *mid_rays = ray_lists + nray, *short_rays = ray_lists + 2 * nray;
 	UpdView uv = upd_view(ctx, pl);
-	k_ray_class<<<blocks(nray, 256), 256, 0, st>>>(nray, off64, ctx->tune.deposit_long, ctx->tune.deposit_mid, cls);
+	k_ray_class<<<blocks(nray, 256), 256, 0, st>>>(nray, R, off64, ctx->tune.deposit_long, ctx->tune.deposit_mid,
+			(int)pl.dep_grid * (DEP_THREADS / 32), cls);
 	PSG_CHECK_LAUNCH();
 	PSG_CUDA(scan_enqueue(st, cls, nray, cls_scan, tiles, Widen()));
 	k_ray_lists<<<blocks(nray, 256), 256, 0, st>>>(nray, cls, cls_scan, long_rays, mid_rays, short_rays);
@@ -2207,15 +2259,15 @@ int enqueue_batch(psg_context *ctx, const BatchPlan &pl, const PsgBatchDev *B) {
 		psg_mark_begin(ctx, PSG_K_DEPOSIT);
 		if (pl.gen)
 			k_deposit<true, false><<<pl.dep_grid, DEP_THREADS, 0, st>>>((int)t, uv.tick_rays, uv.dep_ctr, B,
-					long_rays, mid_rays, short_rays, off64, hit_ipar, hit_kern, ctx->d_lambdaH, ctx->d_mass, P,
+					long_rays, mid_rays, short_rays, ctx->tune.deposit_long, ctx->tune.deposit_mid, off64, hit_ipar, hit_kern, ctx->d_lambdaH, ctx->d_mass, P,
 					pl.want_heat, acc, pl.nacc, d_nsat, d_lost);
 		else if (pl.aff)
 			k_deposit<false, true><<<pl.dep_grid, DEP_THREADS, 0, st>>>((int)t, uv.tick_rays, uv.dep_ctr, B,
-					long_rays, mid_rays, short_rays, off64, hit_ipar, hit_kern, ctx->d_lambdaH, ctx->d_mass, P,
+					long_rays, mid_rays, short_rays, ctx->tune.deposit_long, ctx->tune.deposit_mid, off64, hit_ipar, hit_kern, ctx->d_lambdaH, ctx->d_mass, P,
 					pl.want_heat, acc, pl.nacc, d_nsat, d_lost);
 		else
 			k_deposit<false, false><<<pl.dep_grid, DEP_THREADS, 0, st>>>((int)t, uv.tick_rays, uv.dep_ctr, B,
-					long_rays, mid_rays, short_rays, off64, hit_ipar, hit_kern, ctx->d_lambdaH, ctx->d_mass, P,
+					long_rays, mid_rays, short_rays, ctx->tune.deposit_long, ctx->tune.deposit_mid, off64, hit_ipar, hit_kern, ctx->d_lambdaH, ctx->d_mass, P,
 					pl.want_heat, acc, pl.nacc, d_nsat, d_lost);
 		PSG_CHECK_LAUNCH();
 		ctx->launches++;
