@@ -1002,46 +1002,71 @@ __device__ __forceinline__ bool upd_looks_slow(float hstep, double time, double 
 	return !(hstep > 0.0f) || 4.0 * (double)hstep < time || g > lam0;
 }
 
+// The particle of an active pair and what its update reads of it: loaded
+// before the pair's deposits are summed, so that these gathers and the
+// deposits' are in flight together.
+template <bool ISO>
+struct PairState {
+	uint32_t p;
+	int32_t hits;
+	int64_t lasthit;
+	double lam;
+	float ie, rho, yeMET, hstep;
+	__device__ __forceinline__ PairState(uint32_t p_, const int32_t *__restrict__ hits_,
+			const int64_t *__restrict__ lasthit_, const double *__restrict__ lambdaH, const float *__restrict__ ie_,
+			const float *__restrict__ rho_, const float *__restrict__ yeMET_, const float *__restrict__ hstep_, bool slow,
+			bool rec)
+		: p(p_), hits(hits_[p_]), lasthit(0), lam(0.0), ie(0.f), rho(0.f), yeMET(0.f), hstep(0.f) {
+		if (ISO || slow || rec) {
+			lasthit = lasthit_[p];
+			lam = lambdaH[p];
+		}
+		if (ISO || rec) {
+			ie = ie_[p];
+			rho = rho_[p];
+			yeMET = yeMET_[p];
+		}
+		if (slow) hstep = hstep_[p];
+	}
+};
+
 // The particle's summed deposits of the tick: isothermal, the closed-form
 // update_pars() step (loop.c:653-770); otherwise the sums for the integrator
 // (with act_slow, whether the integrator should claim it first).
 template <bool ISO, bool REC>
-__device__ __forceinline__ void finish_particle(int a, double g, double heat, int nh,
-		const uint32_t *__restrict__ act_ipar, int32_t *__restrict__ hits, double *__restrict__ act_g,
+__device__ __forceinline__ void finish_particle(int a, const PairState<ISO> &x, double g, double heat, int nh,
+		int32_t *__restrict__ hits, double *__restrict__ act_g,
 		double *__restrict__ act_heat, double *__restrict__ lambdaH, float *__restrict__ ie,
-		int64_t *__restrict__ lasthit, const float *__restrict__ rho, const float *__restrict__ yeMET,
-		const float *__restrict__ hstep, UpdRec *__restrict__ rec, int lo, const double *__restrict__ gcarry,
+		int64_t *__restrict__ lasthit, UpdRec *__restrict__ rec, int lo, const double *__restrict__ gcarry,
 		uint8_t *__restrict__ act_slow, const PhysParams &P, int64_t tick, double tick_time,
 		uint32_t *__restrict__ status) {
-	const uint32_t p = act_ipar[a];
-	hits[p] += nh;
+	const uint32_t p = x.p;
+	hits[p] = x.hits + nh;
 	if (gcarry) g += gcarry[p];      // photons left over by an earlier explicit step (loop.c:745)
+	const double time = rn_dmul((double)(tick - x.lasthit), tick_time);
 	if (!ISO) {
 		if (act_g) {        // read by the integrator queue, the surrogate and the update log
 			act_g[a] = g;
 			act_heat[a] = heat;
 		}
-		if (act_slow)
-			act_slow[a] = upd_looks_slow(hstep[p], rn_dmul((double)(tick - lasthit[p]), tick_time), g, lambdaH[p]);
+		if (act_slow) act_slow[a] = upd_looks_slow(x.hstep, time, g, x.lam);
 		if (!rec) return;      // sums only: the integrator builds its own records
 		UpdRec r;
-		r.time = rn_dmul((double)(tick - lasthit[p]), tick_time);
-		r.lam0 = lambdaH[p];
+		r.time = time;
+		r.lam0 = x.lam;
 		r.g = g;
 		r.heat = heat;
-		r.ie0 = ie[p];
-		r.rho = rho[p];
-		r.yeMET = yeMET[p];
+		r.ie0 = x.ie;
+		r.rho = x.rho;
+		r.yeMET = x.yeMET;
 		r.p = p;
 		rec[a - lo] = r;    // records of one tick, from its first active particle
 		return;
 	}
-	const double time = rn_dmul((double)(tick - lasthit[p]), tick_time);
-	const double lam0 = lambdaH[p];
-	const double T = ieye2T(P, (double)ie[p], rn_dadd(rn_dsub(1.0, lam0), P.he_e));
-	const double nH = rn_dmul(P.H_PER_MASS, (double)rho[p]);
-	double lam = lam0, grec = 0.0;
-	const uint32_t st = solve_step_iso(P, lam, (double)yeMET[p], g, time, nH, T, REC ? &grec : nullptr);
+	const double T = ieye2T(P, (double)x.ie, rn_dadd(rn_dsub(1.0, x.lam), P.he_e));
+	const double nH = rn_dmul(P.H_PER_MASS, (double)x.rho);
+	double lam = x.lam, grec = 0.0;
+	const uint32_t st = solve_step_iso(P, lam, (double)x.yeMET, g, time, nH, T, REC ? &grec : nullptr);
 	lambdaH[p] = lam;
 	if (REC) P.ygrec[p] = (float)fmax(0.0, (double)P.ygrec[p] + grec);     // x[3], solve.c:183,211,218
 	ie[p] = (float)Tye2ie(P, T, rn_dadd(rn_dsub(1.0, lam), P.he_e));
@@ -1050,19 +1075,14 @@ __device__ __forceinline__ void finish_particle(int a, double g, double heat, in
 }
 
 // Runs of up to short_max (at most RUN_SHORT) hits stay in placement order; their
-// sums go in hit order all the same. Up to 4 hits by selection (each step
-// the smallest hit index above the last: at most 16 reads, in L1); up to 8
-// and 16 through a bitonic network in registers (fully unrolled: 24 and 80
-// compare-exchanges). Longer runs are sorted and read in order.
-__device__ __forceinline__ uint32_t next_in_run(const uint32_t *__restrict__ vals, uint32_t s0, uint32_t s1,
-		int64_t prev) {
-	uint32_t best = 0xFFFFFFFFu;
-	for (uint32_t q = s0; q < s1; q++) {
-		const uint32_t v = vals[q];
-		if ((int64_t)v > prev && v < best) best = v;
-	}
-	return best;
-}
+// sums go in hit order all the same, through a bitonic network in registers
+// (8 entries up to 8 hits, 16 up to 16: 24 and 80 compare-exchanges). Longer
+// runs are sorted and read in order. Either way the deposits are gathered
+// eight at a time and then added one by one: the sum waits for two rounds of
+// loads, not for one per hit (a run of 32 hits took 32 of them, and its warp
+// with it). k_reduce per call, with the pair's state loaded ahead: 8 ticks of
+// 1.7e6 pairs 844 -> 544 us, 4 of 1.5e7 6.0 -> 3.7 ms, 100 isothermal ones of
+// 7e4 pairs 2.05 -> 1.57 ms.
 template <int N>
 __device__ __forceinline__ void bitonic_regs(uint32_t (&v)[N]) {
 #pragma unroll
@@ -1082,35 +1102,45 @@ __device__ __forceinline__ void bitonic_regs(uint32_t (&v)[N]) {
 		}
 	}
 }
-template <int N, typename F>
-__device__ __forceinline__ void visit_sorted_regs(const uint32_t *__restrict__ vals, uint32_t s0, uint32_t n, F f) {
+// D: a hit's deposits as loaded; load(hit) gathers them (of a padding entry
+// it returns none), add(D) adds them.
+template <int N, typename D, typename L, typename A>
+__device__ __forceinline__ void visit_sorted_regs(const uint32_t *__restrict__ vals, uint32_t s0, uint32_t n, L load,
+		A add) {
 	uint32_t v[N];
 #pragma unroll
 	for (int i = 0; i < N; i++) v[i] = (uint32_t)i < n ? vals[s0 + i] : 0xFFFFFFFFu;
 	bitonic_regs<N>(v);
 #pragma unroll
-	for (int i = 0; i < N; i++)
-		if ((uint32_t)i < n) f(v[i]);
+	for (int b = 0; b < N; b += 8) {
+		D d[8];
+#pragma unroll
+		for (int i = 0; i < 8; i++) d[i] = load(v[b + i], (uint32_t)(b + i) < n);
+#pragma unroll
+		for (int i = 0; i < 8; i++) add(d[i]);
+	}
 }
-// f(hit) for every hit of the run [s0, s1) in hit order; runs longer than
-// short_max (4, 8 or 16: the tuner's run_short) are read as stored (sorted)
-template <typename F>
+// every hit of the run [s0, s1) in hit order; runs longer than short_max (4,
+// 8 or 16: the tuner's run_short) are read as stored (sorted)
+template <typename D, typename L, typename A>
 __device__ __forceinline__ void visit_run(const uint32_t *__restrict__ vals, uint32_t s0, uint32_t s1,
-		uint32_t short_max, F f) {
+		uint32_t short_max, L load, A add) {
 	const uint32_t n = s1 - s0;
-	if (n > short_max) {
-		for (uint32_t k = s0; k < s1; k++) f(vals[k]);
-	} else if (n <= 4) {
-		int64_t prev = -1;
-		for (uint32_t i = 0; i < n; i++) {
-			const uint32_t h = next_in_run(vals, s0, s1, prev);
-			prev = h;
-			f(h);
-		}
-	} else if (n <= 8) {
-		visit_sorted_regs<8>(vals, s0, n, f);
+	if (n <= 8 && n <= short_max) {
+		visit_sorted_regs<8, D>(vals, s0, n, load, add);
+	} else if (n <= short_max) {
+		visit_sorted_regs<RUN_SHORT, D>(vals, s0, n, load, add);
 	} else {
-		visit_sorted_regs<RUN_SHORT>(vals, s0, n, f);
+		for (uint32_t k = s0; k < s1; k += 8) {
+			uint32_t v[8];
+			D d[8];
+#pragma unroll
+			for (int i = 0; i < 8; i++) v[i] = k + i < s1 ? vals[k + i] : 0u;
+#pragma unroll
+			for (int i = 0; i < 8; i++) d[i] = load(v[i], k + i < s1);
+#pragma unroll
+			for (int i = 0; i < 8; i++) add(d[i]);
+		}
 	}
 }
 
@@ -1191,29 +1221,35 @@ __global__ void __launch_bounds__(256, ISO && !REC ? 5 : 4) k_reduce(int t, cons
 			e += nwarp) {
 		const int a = (int)long_act[e];
 		if (act_seg[a + 1] - act_seg[a] <= RUN_THREAD) continue;      // (a thread's, below)
+		const PairState<ISO> x(act_ipar[a], hits, lasthit, lambdaH, ie, rho, yeMET, hstep, act_slow, rec);
 		double sg, sh;
 		int sn;
 		warp_segment_sum(acc, vals, want_heat, act_seg[a], act_seg[a + 1], lane, sg, sh, sn);
 		if (lane == 0)
-			finish_particle<ISO, REC>(a, sg, sh, sn, act_ipar, hits, act_g, act_heat, lambdaH, ie, lasthit, rho, yeMET,
-					hstep, rec, lo, gcarry, act_slow, P, tick, tick_time, status);
+			finish_particle<ISO, REC>(a, x, sg, sh, sn, hits, act_g, act_heat, lambdaH, ie, lasthit, rec, lo, gcarry,
+					act_slow, P, tick, tick_time, status);
 	}
 	for (int a = lo + (int)(blockIdx.x * blockDim.x + threadIdx.x); a < hi; a += (int)(gridDim.x * blockDim.x)) {
 		const uint32_t s0 = act_seg[a], s1 = act_seg[a + 1];
 		if (s1 - s0 > RUN_THREAD) continue;
+		const PairState<ISO> x(act_ipar[a], hits, lasthit, lambdaH, ie, rho, yeMET, hstep, act_slow, rec);
 		double g = 0.0, heat = 0.0;
 		int nh = 0;
-		visit_run(vals, s0, s1, short_max, [&](uint32_t hk) {
-			if (want_heat) {
-				const double2 d = reinterpret_cast<const double2 *>(acc)[hk];
-				if (d.x >= 0.0) { g += d.x; heat += d.y; nh++; }
-			} else {
-				const double d = acc[hk];
-				if (d >= 0.0) { g += d; nh++; }
-			}
-		});
-		finish_particle<ISO, REC>(a, g, heat, nh, act_ipar, hits, act_g, act_heat, lambdaH, ie, lasthit, rho, yeMET,
-				hstep, rec, lo, gcarry, act_slow, P, tick, tick_time, status);
+		if (want_heat) {
+			const double2 *acc2 = reinterpret_cast<const double2 *>(acc);
+			visit_run<double2>(vals, s0, s1, short_max,
+					[&](uint32_t hk, bool on) { return on ? acc2[hk] : make_double2(-1.0, 0.0); },
+					[&](double2 d) {
+						if (d.x >= 0.0) { g += d.x; heat += d.y; nh++; }
+					});
+		} else {
+			visit_run<double>(vals, s0, s1, short_max, [&](uint32_t hk, bool on) { return on ? acc[hk] : -1.0; },
+					[&](double d) {
+						if (d >= 0.0) { g += d; nh++; }
+					});
+		}
+		finish_particle<ISO, REC>(a, x, g, heat, nh, hits, act_g, act_heat, lambdaH, ie, lasthit, rec, lo, gcarry,
+				act_slow, P, tick, tick_time, status);
 	}
 }
 
@@ -1574,18 +1610,23 @@ __global__ void __launch_bounds__(256) k_sum_he(int t, const int32_t *__restrict
 		if (s1 - s0 > RUN_THREAD) continue;
 		double g0 = 0.0, g1 = 0.0, g2 = 0.0, heat = 0.0;
 		int nh = 0;
-		visit_run(vals, s0, s1, short_max, [&](uint32_t h) {
-			const size_t hk = h;
-			const double2 x = acc2[2 * hk];
-			if (x.x >= 0.0) {
-				const double2 y = acc2[2 * hk + 1];
-				g0 += x.x;
-				g1 += y.x;
-				g2 += y.y;
-				if (want_heat) heat += x.y;
-				nh++;
-			}
-		});
+		struct Four {
+			double2 x, y;
+		};
+		visit_run<Four>(vals, s0, s1, short_max,
+				[&](uint32_t hk, bool on) {
+					return on ? Four{acc2[2 * (size_t)hk], acc2[2 * (size_t)hk + 1]}
+							: Four{make_double2(-1.0, 0.0), make_double2(0.0, 0.0)};
+				},
+				[&](const Four &d) {
+					if (d.x.x >= 0.0) {
+						g0 += d.x.x;
+						g1 += d.y.x;
+						g2 += d.y.y;
+						if (want_heat) heat += d.x.y;
+						nh++;
+					}
+				});
 		sum_g0[a] = g0;
 		sum_g1[a] = g1;
 		sum_g2[a] = g2;
