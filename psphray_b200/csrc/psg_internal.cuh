@@ -112,10 +112,12 @@ struct psg_context {
 	                             // ray) hit the particle, -1 never: the emitters of the next tick
 	uint32_t *d_order = nullptr; // after a tree build the arrays above are in leaf order:
 	                             // position k holds the caller's particle d_order[k] (null: caller order)
+	uint32_t *d_order_buf = nullptr;   // its memory, kept while the arrays are
 
 	// octree, depth-first order
 	int have_tree = 0;
 	size_t ncell = 0, nleaf = 0, skipped = 0, nvalid = 0;
+	size_t leaf_cap = 0, cell_cap = 0;   // entries the tree's particle and cell arrays hold
 	int depth = 0;
 	float4 *d_cell_lo = nullptr;  // bot.xyz, w = index past the subtree (int bits)
 	float4 *d_cell_hi = nullptr;  // top.xyz, w = first particle in leaf order (int bits)

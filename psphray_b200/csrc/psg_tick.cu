@@ -2455,8 +2455,14 @@ std::vector<unsigned long long> batch_key(const psg_context *ctx, const BatchPla
 	k.push_back(ctx->log_cap);
 	k.push_back((unsigned long long)(uintptr_t)ctx->log_count);
 	const void *dev[] = {ctx->d_psml, ctx->d_order, ctx->d_mass, ctx->d_rho, ctx->d_yeMET, ctx->d_ie, ctx->d_lambdaH,
-		ctx->d_hits, ctx->d_lasthit, ctx->d_hstep, ctx->d_gcarry, ctx->d_status, ctx->d_counters};
+		ctx->d_hits, ctx->d_lasthit, ctx->d_hstep, ctx->d_gcarry, ctx->d_status, ctx->d_counters, ctx->d_wide_lo,
+		ctx->d_wide_hi, ctx->d_leaf_psml, ctx->d_leaf_idx};
 	for (const void *q : dev) k.push_back((unsigned long long)(uintptr_t)q);
+	// (the field's arrays outlive a reload: what else a captured tick holds of it)
+	unsigned long long boxbits = 0;
+	memcpy(&boxbits, &ctx->boxsize, 8);
+	k.push_back(boxbits);
+	k.push_back((unsigned long long)ctx->ppc);
 	k.push_back(ctx->n);
 	k.push_back(ctx->hit_cap);
 	k.push_back((unsigned long long)ctx->tune.deposit_long << 32 | (unsigned)ctx->tune.deposit_mid);

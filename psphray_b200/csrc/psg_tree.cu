@@ -293,13 +293,17 @@ extern "C" int psg_build_tree(psg_context *ctx, int ppc) {
 	if (prc) return prc;
 
 	// particles in leaf order
-	if (ctx->d_leaf_psml) cudaFree(ctx->d_leaf_psml);
-	if (ctx->d_leaf_idx) cudaFree(ctx->d_leaf_idx);
-	ctx->d_leaf_psml = nullptr;
-	ctx->d_leaf_idx = nullptr;
 	ctx->have_tree = 0;
-	PSG_CUDA(cudaMalloc(&ctx->d_leaf_psml, sizeof(float4) * (nvalid + 1)));
-	PSG_CUDA(cudaMalloc(&ctx->d_leaf_idx, sizeof(uint32_t) * (nvalid + 1)));
+	if (ctx->leaf_cap < nvalid + 1) {
+		if (ctx->d_leaf_psml) cudaFree(ctx->d_leaf_psml);
+		if (ctx->d_leaf_idx) cudaFree(ctx->d_leaf_idx);
+		ctx->d_leaf_psml = nullptr;
+		ctx->d_leaf_idx = nullptr;
+		ctx->leaf_cap = 0;
+		PSG_CUDA(cudaMalloc(&ctx->d_leaf_psml, sizeof(float4) * (nvalid + 1)));
+		PSG_CUDA(cudaMalloc(&ctx->d_leaf_idx, sizeof(uint32_t) * (nvalid + 1)));
+		ctx->leaf_cap = nvalid + 1;
+	}
 	if (nvalid)
 		k_gather_particles<<<blocks(nvalid, 256), 256, 0, st>>>(nvalid, ctx->d_psml, ctx->d_flag,
 				ctx->d_leaf_psml, ctx->d_leaf_idx);
@@ -397,18 +401,21 @@ extern "C" int psg_build_tree(psg_context *ctx, int ppc) {
 		k_preorder<<<blocks(e - b, 128), 128, 0, st>>>(c, b, e);
 		PSG_CHECK_LAUNCH();
 	}
-	if (ctx->d_cell_lo) cudaFree(ctx->d_cell_lo);
-	if (ctx->d_cell_hi) cudaFree(ctx->d_cell_hi);
-	ctx->d_cell_lo = ctx->d_cell_hi = nullptr;
-	PSG_CUDA(cudaMalloc(&ctx->d_cell_lo, sizeof(float4) * (ncell + 1)));
-	PSG_CUDA(cudaMalloc(&ctx->d_cell_hi, sizeof(float4) * (ncell + 1)));
+	// the cell arrays are kept while they are large enough (an eighth over, as
+	// the cells of a moving field's next tree differ a little)
+	if (ctx->cell_cap < ncell + 1) {
+		for (float4 **q : {&ctx->d_cell_lo, &ctx->d_cell_hi, &ctx->d_wide_lo, &ctx->d_wide_hi}) {
+			if (*q) cudaFree(*q);
+			*q = nullptr;
+		}
+		ctx->cell_cap = 0;
+		const size_t cc = ncell + 1 + ncell / 8;
+		for (float4 **q : {&ctx->d_cell_lo, &ctx->d_cell_hi, &ctx->d_wide_lo, &ctx->d_wide_hi})
+			PSG_CUDA(cudaMalloc(q, sizeof(float4) * cc));
+		ctx->cell_cap = cc;
+	}
 	k_emit<<<blocks(ncell + 1, 256), 256, 0, st>>>(c, (int)ncell, (uint32_t)nvalid, ctx->d_cell_lo, ctx->d_cell_hi);
 	PSG_CHECK_LAUNCH();
-	if (ctx->d_wide_lo) cudaFree(ctx->d_wide_lo);
-	if (ctx->d_wide_hi) cudaFree(ctx->d_wide_hi);
-	ctx->d_wide_lo = ctx->d_wide_hi = nullptr;
-	PSG_CUDA(cudaMalloc(&ctx->d_wide_lo, sizeof(float4) * ncell));
-	PSG_CUDA(cudaMalloc(&ctx->d_wide_hi, sizeof(float4) * ncell));
 	k_emit_wide<<<blocks(ncell, 256), 256, 0, st>>>(c, (int)ncell, ctx->d_wide_lo, ctx->d_wide_hi);
 	PSG_CHECK_LAUNCH();
 	PSG_CUDA(cudaStreamSynchronize(st));
