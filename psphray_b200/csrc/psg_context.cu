@@ -595,6 +595,58 @@ static int to_caller(psg_context *ctx, T *host, const T *dev) {
 	return PSG_OK;
 }
 
+// Several arrays at once: one kernel puts them all into the caller's order,
+// their copies follow, one wait ends them (for a small field each launch and
+// wait costs more than its bytes).
+struct ReadJob {
+	void *host;
+	const void *dev;
+	int item;          // bytes of an element: 4 or 8
+	size_t off;        // in the staging memory
+};
+#define READ_JOBS 5
+struct ReadJobs {
+	ReadJob j[READ_JOBS];
+	int n;
+};
+__global__ void k_scatter_all(size_t n, const uint32_t *__restrict__ g, ReadJobs jobs, char *__restrict__ out) {
+	const size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+	if (k >= n) return;
+	const size_t c = g[k];
+#pragma unroll
+	for (int i = 0; i < READ_JOBS; i++) {
+		if (i >= jobs.n) break;
+		const ReadJob &q = jobs.j[i];
+		if (q.item == 8) ((uint64_t *)(out + q.off))[c] = ((const uint64_t *)q.dev)[k];
+		else ((uint32_t *)(out + q.off))[c] = ((const uint32_t *)q.dev)[k];
+	}
+}
+static int read_arrays(psg_context *ctx, ReadJobs jobs) {
+	const size_t n = ctx->n;
+	cudaStream_t s = ctx->stream;
+	int m = 0;
+	size_t bytes = 0;
+	for (int i = 0; i < jobs.n; i++) {
+		if (!jobs.j[i].host) continue;
+		jobs.j[m] = jobs.j[i];
+		jobs.j[m++].off = bytes;
+		bytes += (jobs.j[i].item * n + 255) & ~(size_t)255;
+	}
+	jobs.n = m;
+	char *stage = nullptr;
+	if (ctx->d_order && m) {
+		stage = (char *)psg_scratch(ctx, S_MAP, bytes);
+		if (!stage) return PSG_E_NOMEM;
+		k_scatter_all<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, ctx->d_order, jobs, stage);
+		PSG_CHECK_LAUNCH();
+	}
+	for (int i = 0; i < m; i++)
+		PSG_CUDA(cudaMemcpyAsync(jobs.j[i].host, stage ? stage + jobs.j[i].off : jobs.j[i].dev, jobs.j[i].item * n,
+				cudaMemcpyDeviceToHost, s));
+	PSG_CUDA(cudaStreamSynchronize(s));
+	return PSG_OK;
+}
+
 // host array (caller order) -> device array (internal order)
 template <typename T>
 static int from_caller(psg_context *ctx, T *dev, const T *host) {
@@ -618,13 +670,8 @@ extern "C" int psg_get_state(psg_context *ctx, double *lambdaH, float *ie, int32
 	if (!ctx) return PSG_E_INVAL;
 	if (!ctx->n) return psg_fail(ctx, PSG_E_INVAL, "psg_get_state: no particles loaded");
 	PSG_CUDA(cudaSetDevice(ctx->device));
-	int rc = 0;
-	if (lambdaH && (rc = to_caller(ctx, lambdaH, ctx->d_lambdaH))) return rc;
-	if (ie && (rc = to_caller(ctx, ie, ctx->d_ie))) return rc;
-	if (hits && (rc = to_caller(ctx, hits, ctx->d_hits))) return rc;
-	if (lasthit && (rc = to_caller(ctx, lasthit, ctx->d_lasthit))) return rc;
-	PSG_CUDA(cudaStreamSynchronize(ctx->stream));
-	return PSG_OK;
+	return read_arrays(ctx, {{{lambdaH, ctx->d_lambdaH, 8, 0}, {ie, ctx->d_ie, 4, 0}, {hits, ctx->d_hits, 4, 0},
+			{lasthit, ctx->d_lasthit, 8, 0}}, 4});
 }
 
 extern "C" int psg_set_state(psg_context *ctx, const double *lambdaH, const float *ie,
@@ -655,14 +702,8 @@ extern "C" int psg_get_he_state(psg_context *ctx, double *lambdaHeI, double *lam
 	if (!ctx) return PSG_E_INVAL;
 	if (!ctx->n) return psg_fail(ctx, PSG_E_INVAL, "psg_get_he_state: no particles loaded");
 	PSG_CUDA(cudaSetDevice(ctx->device));
-	int rc = 0;
-	if (lambdaHeI && (rc = to_caller(ctx, lambdaHeI, ctx->d_lamHeI))) return rc;
-	if (lambdaHeII && (rc = to_caller(ctx, lambdaHeII, ctx->d_lamHeII))) return rc;
-	if (yeMET && (rc = to_caller(ctx, yeMET, ctx->d_yeMET))) return rc;
-	if (yGrecHeII && (rc = to_caller(ctx, yGrecHeII, ctx->d_ygrecHe1))) return rc;
-	if (yGrecHeIII && (rc = to_caller(ctx, yGrecHeIII, ctx->d_ygrecHe2))) return rc;
-	PSG_CUDA(cudaStreamSynchronize(ctx->stream));
-	return PSG_OK;
+	return read_arrays(ctx, {{{lambdaHeI, ctx->d_lamHeI, 8, 0}, {lambdaHeII, ctx->d_lamHeII, 8, 0},
+			{yeMET, ctx->d_yeMET, 4, 0}, {yGrecHeII, ctx->d_ygrecHe1, 4, 0}, {yGrecHeIII, ctx->d_ygrecHe2, 4, 0}}, 5});
 }
 
 extern "C" int psg_set_he_state(psg_context *ctx, const double *lambdaHeI, const double *lambdaHeII,
@@ -683,11 +724,7 @@ extern "C" int psg_get_rec_state(psg_context *ctx, float *yGrecHII, int32_t *src
 	if (!ctx) return PSG_E_INVAL;
 	if (!ctx->n) return psg_fail(ctx, PSG_E_INVAL, "psg_get_rec_state: no particles loaded");
 	PSG_CUDA(cudaSetDevice(ctx->device));
-	int rc = 0;
-	if (yGrecHII && (rc = to_caller(ctx, yGrecHII, ctx->d_ygrec))) return rc;
-	if (srcmark && (rc = to_caller(ctx, srcmark, ctx->d_srcmark))) return rc;
-	PSG_CUDA(cudaStreamSynchronize(ctx->stream));
-	return PSG_OK;
+	return read_arrays(ctx, {{{yGrecHII, ctx->d_ygrec, 4, 0}, {srcmark, ctx->d_srcmark, 4, 0}}, 2});
 }
 
 extern "C" int psg_set_rec_state(psg_context *ctx, const float *yGrecHII, const int32_t *srcmark) {

