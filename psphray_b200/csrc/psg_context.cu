@@ -556,7 +556,9 @@ static int permute_array(psg_context *ctx, T *arr, const uint32_t *g, void *tmp)
 
 int psg_permute_particles(psg_context *ctx, const uint32_t *g) {
 	const size_t n = ctx->n;
-	void *tmp = psg_scratch(ctx, S_MAP, sizeof(float4) * n);
+	// (room for the state calls' staging too: grown later, it would be freed and
+	// allocated again in the first call)
+	void *tmp = psg_scratch(ctx, S_MAP, 24 * n + 2048);
 	if (!tmp) return PSG_E_NOMEM;
 	int rc = 0;
 	if ((rc = permute_array(ctx, ctx->d_psml, g, tmp)) || (rc = permute_array(ctx, ctx->d_mass, g, tmp)) ||

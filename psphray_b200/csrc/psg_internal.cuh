@@ -117,6 +117,7 @@ struct psg_context {
 	// octree, depth-first order
 	int have_tree = 0;
 	size_t ncell = 0, nleaf = 0, skipped = 0, nvalid = 0;
+	int level_start[4] = {};      // first cell (level order) of levels 1 to 3 where the tree has all 8^l of them, else 0
 	size_t leaf_cap = 0, cell_cap = 0;   // entries the tree's particle and cell arrays hold
 	int depth = 0;
 	float4 *d_cell_lo = nullptr;  // bot.xyz, w = index past the subtree (int bits)
@@ -168,7 +169,6 @@ struct psg_context {
 	size_t hit_cap = 0;                         // hits the sorted-list buffers hold
 	size_t batch_cap = 0;                       // hits the tick batches' per-hit buffers hold
 	unsigned sort_grid[8] = {};                 // persistent grids of the per-ray sort's classes
-	unsigned trace_grid = 0;                    // persistent grid of the traversal (psg_trace_fill_prepare)
 	psg_tune tune{4, 96, 384, 1, 8, 16, 1};        // launch shapes (psg_set_tune, psg_autotune)
 	long host_syncs = 0;                        // host synchronisations of the current call
 	void *graphs = nullptr;                     // captured tick batches (psg_tick.cu)

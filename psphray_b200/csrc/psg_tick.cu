@@ -2716,7 +2716,6 @@ int psg_run_ticks_rec_graph(psg_context *ctx, const psg_ray *d_rays, size_t R, s
 	key.push_back(ctx->rec_seed);
 	key.push_back((unsigned long long)ctx->rec_disable_lte);
 	key.push_back((unsigned long long)(uintptr_t)ctx->d_srcmark);
-	key.push_back(ctx->trace_grid);
 	key.push_back((unsigned long long)ctx->tune.trace_warps);
 	rc = launch_graph(ctx, std::move(key), tick_enqueue, K);
 	if (rc) return rc;

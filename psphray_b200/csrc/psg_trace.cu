@@ -118,9 +118,10 @@ __device__ __forceinline__ bool line_test(const RayGeom &g, const float4 q, int 
 // 32 at a time; the hits go to the ray's slab in order of discovery, as
 // positions alone: their distances are computed by the sort, with every
 // lane busy.
+// With count (several warps share the ray) the slab's places are taken from it.
 __device__ __forceinline__ void test_candidates(const RayGeom &g, const int *list, int total,
 		const float4 *__restrict__ lpsml, const uint32_t *__restrict__ lidx, uint32_t *__restrict__ slab, size_t scap,
-		uint32_t &nh, int lane, unsigned lt_mask) {
+		uint32_t &nh, uint32_t *__restrict__ count, int lane, unsigned lt_mask) {
 	for (int k0 = 0; k0 < total; k0 += 32) {
 		const int k = k0 + lane;
 		bool acc = false;
@@ -130,6 +131,11 @@ __device__ __forceinline__ void test_candidates(const RayGeom &g, const int *lis
 			acc = line_test(g, __ldg(&lpsml[p]), p, lidx);
 		}
 		const unsigned bal = __ballot_sync(0xffffffffu, acc);
+		if (count) {
+			if (!bal) continue;
+			if (lane == 0) nh = atomicAdd(count, (uint32_t)__popc(bal));
+			nh = __shfl_sync(0xffffffffu, nh, 0);
+		}
 		const size_t q = nh + __popc(bal & lt_mask);
 		if (acc && q < scap) slab[q] = (uint32_t)p;
 		nh += __popc(bal);
@@ -157,16 +163,24 @@ __device__ __forceinline__ void test_candidates(const RayGeom &g, const int *lis
 // hits each) 5.0 -> 3.2 ms; 102400 on 64^3 (123 each) 0.68 -> 0.51 ms.
 // PPC: the leaves' capacity where it is 8 (the reference's), else 0 and the
 // argument.
+//
+// SPLIT: with fewer rays than resident warps (a host's few rays) a ray's walk is a serial chain of L2 round
+// trips on an idle machine, so it is divided among nstart warps, each from one
+// cell of an upper level of the tree on (from index start0; plan_trace
+// chooses the level, which the tree has in full, so that levels 1, 2 and 3
+// start at cells 1, 9 and 73). 32 rays on 32^3: 47 -> 19 us; 1024 rays on
+// 64^3: 162 -> 109 us.
 #define TR_STACK 640
 #define TR_REGS 48
 #define TR_MAX_WARPS 16      // warps per block: ctx->tune.trace_warps, at most this
 
-template <int PPC>
+template <int PPC, bool SPLIT>
 __global__ void __maxnreg__(TR_REGS) k_trace_stack(const psg_ray *__restrict__ rays, size_t nray,
 		const float4 *__restrict__ wlo, const float4 *__restrict__ whi,
 		const float4 *__restrict__ lpsml, const uint32_t *__restrict__ lidx, int ppc_any,
 		uint32_t *__restrict__ count, size_t scap, uint32_t *__restrict__ slab_ipar,
-		unsigned long long *__restrict__ next_ray, uint32_t *__restrict__ status, const unsigned *__restrict__ nlim) {
+		unsigned long long *__restrict__ next_ray, uint32_t *__restrict__ status, const unsigned *__restrict__ nlim,
+		int start0, int nstart) {
 	extern __shared__ int tr_smem[];
 	const int ppc = PPC ? PPC : ppc_any;
 	// rays past *nlim (when given: the recombination path's emitted count)
@@ -183,16 +197,24 @@ __global__ void __maxnreg__(TR_REGS) k_trace_stack(const psg_ray *__restrict__ r
 	unsigned long long rr = 0;
 	if (lane == 0) rr = atomicAdd(next_ray, 1ull);
 	rr = __shfl_sync(0xffffffffu, rr, 0);
-	if (rr >= nray) break;
-	const size_t r = (size_t)rr;
+	if (rr >= (SPLIT ? nray * nstart : nray)) break;
+	const size_t r = SPLIT ? (size_t)rr / (unsigned)nstart : (size_t)rr;
+	const int root = SPLIT ? start0 + (int)((size_t)rr - r * (unsigned)nstart) : 0;
 	const RayGeom g = load_ray(rays, r);
 	uint32_t *slab = slab_ipar + r * scap;
+	uint32_t *const shared_count = SPLIT ? count + r : nullptr;
 	uint32_t nh = 0;
 	int sp = 0, nbuf = 0;
 	bool overflow = false;
 	{
-		const float4 lo = __ldg(&wlo[0]), hi = __ldg(&whi[0]);
-		if (segment_hits_box(g, lo, hi)) {
+		const float4 lo = __ldg(&wlo[root]), hi = __ldg(&whi[root]);
+		bool hit = segment_hits_box(g, lo, hi);
+		if (SPLIT)      // and its ancestors, as the walk from the root tests them
+			for (int c = root; c > 0 && hit;) {
+				c = (c - 1) >> 3;
+				hit = segment_hits_box(g, __ldg(&wlo[c]), __ldg(&whi[c]));
+			}
+		if (hit) {
 			const int w = __float_as_int(lo.w);
 			if (w >= 0) {
 				if (lane == 0) stack[0] = w;
@@ -201,7 +223,7 @@ __global__ void __maxnreg__(TR_REGS) k_trace_stack(const psg_ray *__restrict__ r
 				const int cnt = min(-1 - w, ppc), ps = __float_as_int(hi.w);
 				for (int k = lane; k < cnt; k += 32) list[k] = ps + k;
 				__syncwarp();
-				test_candidates(g, list, cnt, lpsml, lidx, slab, scap, nh, lane, lt_mask);
+				test_candidates(g, list, cnt, lpsml, lidx, slab, scap, nh, shared_count, lane, lt_mask);
 			}
 		}
 	}
@@ -244,7 +266,7 @@ __global__ void __maxnreg__(TR_REGS) k_trace_stack(const psg_ray *__restrict__ r
 		// line tests only in full rounds of 32; the rest waits in the list
 		if (nbuf >= 32) {
 			const int full = nbuf & ~31, rem = nbuf - full;
-			test_candidates(g, list, full, lpsml, lidx, slab, scap, nh, lane, lt_mask);
+			test_candidates(g, list, full, lpsml, lidx, slab, scap, nh, shared_count, lane, lt_mask);
 			__syncwarp();
 			const int keep = lane < rem ? list[full + lane] : 0;
 			__syncwarp();
@@ -253,9 +275,9 @@ __global__ void __maxnreg__(TR_REGS) k_trace_stack(const psg_ray *__restrict__ r
 			__syncwarp();
 		}
 	}
-	if (nbuf) test_candidates(g, list, nbuf, lpsml, lidx, slab, scap, nh, lane, lt_mask);
+	if (nbuf) test_candidates(g, list, nbuf, lpsml, lidx, slab, scap, nh, shared_count, lane, lt_mask);
 	if (lane == 0) {
-		count[r] = nh;
+		if (!SPLIT) count[r] = nh;
 		if (overflow) atomicOr(status, PSG_ST_STACK);
 	}
 	__syncwarp();
@@ -518,20 +540,58 @@ inline unsigned blocks(size_t n, int bs) { return (unsigned)((n + bs - 1) / bs);
 // S_COUNT during a traversal: the hit counts (nray + 1, u32), then their
 // exclusive scan (nray + 2, u64) at the next 16-byte boundary
 const void *trace_kernel(const psg_context *ctx) {
-	return ctx->ppc == 8 ? (const void *)k_trace_stack<8> : (const void *)k_trace_stack<0>;
+	return ctx->ppc == 8 ? (const void *)k_trace_stack<8, false> : (const void *)k_trace_stack<0, false>;
 }
 size_t trace_smem(const psg_context *ctx, int warps) {
 	return sizeof(int) * (TR_STACK + 32 * (size_t)ctx->ppc + 32) * warps;
 }
-void launch_trace(psg_context *ctx, unsigned grid, int warps, const psg_ray *rays, size_t nray, uint32_t *count,
+// The traversal's launch: its persistent grid, and where the rays are few the
+// tree level whose cells divide each of them: the deepest of 1 to 3 that the
+// tree has in full and that makes at most twice as many parts as there are
+// resident warps (more would only be cells that miss). Recombination rays are
+// not divided: a fifth of the box long, each lies in a cell or two of these
+// levels (100 of them on 1M particles: 55 us whole, 64 us divided).
+struct TracePlan {
+	unsigned grid = 0;
+	int warps = 1, start0 = 0, nstart = 0;
+};
+int plan_trace(psg_context *ctx, size_t nray, bool divide, TracePlan *t) {
+	t->warps = std::max(1, std::min(TR_MAX_WARPS, ctx->tune.trace_warps));
+	const size_t smem = trace_smem(ctx, t->warps);
+	const void *kern[2] = {trace_kernel(ctx), ctx->ppc == 8 ? (const void *)k_trace_stack<8, true>
+			: (const void *)k_trace_stack<0, true>};
+	if (smem > 48 * 1024)
+		for (const void *k : kern)
+			PSG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+	int per_sm = 1;
+	PSG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern[0], 32 * t->warps, smem));
+	const size_t resident = (size_t)std::max(per_sm, 1) * ctx->sms;
+	size_t units = nray;
+	t->nstart = 0;
+	for (int l = 1; l <= 3 && divide && ctx->level_start[l]; l++)
+		if (nray << (3 * l) <= 2 * resident * t->warps) {
+			t->start0 = ctx->level_start[l];
+			t->nstart = 1 << (3 * l);
+			units = nray << (3 * l);
+		}
+	t->grid = (unsigned)std::min<size_t>(blocks(units, t->warps), resident);
+	return PSG_OK;
+}
+// (with t.nstart the rays' counts have to be zero)
+void launch_trace(psg_context *ctx, const TracePlan &t, const psg_ray *rays, size_t nray, uint32_t *count,
 		size_t scap, uint32_t *slab, unsigned long long *next_ray, const unsigned *nlim) {
-	const size_t smem = trace_smem(ctx, warps);
-	if (ctx->ppc == 8)
-		k_trace_stack<8><<<grid, 32 * warps, smem, ctx->stream>>>(rays, nray, ctx->d_wide_lo, ctx->d_wide_hi,
-				ctx->d_leaf_psml, ctx->d_leaf_idx, 8, count, scap, slab, next_ray, ctx->d_status, nlim);
-	else
-		k_trace_stack<0><<<grid, 32 * warps, smem, ctx->stream>>>(rays, nray, ctx->d_wide_lo, ctx->d_wide_hi,
-				ctx->d_leaf_psml, ctx->d_leaf_idx, ctx->ppc, count, scap, slab, next_ray, ctx->d_status, nlim);
+	const size_t smem = trace_smem(ctx, t.warps);
+	auto go = [&](auto kern) {
+		kern<<<t.grid, 32 * t.warps, smem, ctx->stream>>>(rays, nray, ctx->d_wide_lo, ctx->d_wide_hi, ctx->d_leaf_psml,
+				ctx->d_leaf_idx, ctx->ppc, count, scap, slab, next_ray, ctx->d_status, nlim, t.start0, t.nstart);
+	};
+	if (t.nstart) {
+		if (ctx->ppc == 8) go(k_trace_stack<8, true>);
+		else go(k_trace_stack<0, true>);
+	} else {
+		if (ctx->ppc == 8) go(k_trace_stack<8, false>);
+		else go(k_trace_stack<0, false>);
+	}
 	ctx->launches++;
 }
 size_t count_bytes(size_t nray) { return 16 * ((sizeof(uint32_t) * (nray + 1) + 15) / 16) + 8 * (nray + 2) + 64; }
@@ -659,12 +719,14 @@ int psg_trace_rec_fill_enqueue(psg_context *ctx, const psg_ray *buf, size_t R, s
 	unsigned long long *next_ray = ctx->d_counters + 9;
 	const size_t scap = ctx->slab_cap;
 	uint32_t *slab_ipar = (uint32_t *)ctx->scratch[S_REC_U32].p;
-	const int trw = std::max(1, std::min(TR_MAX_WARPS, ctx->tune.trace_warps));
+	TracePlan t;
+	const int rc = plan_trace(ctx, cap_rec, false, &t);
+	if (rc) return rc;
 	const SrcHits h = src_hits(ctx);
 	PSG_CUDA(cudaMemsetAsync(count, 0, sizeof(uint32_t) * (nray + 1), st));
 	PSG_CUDA(cudaMemsetAsync(d_max, 0, 2 * sizeof(unsigned long long), st));
 	PSG_CUDA(cudaMemsetAsync(next_ray, 0, sizeof(unsigned long long), st));
-	launch_trace(ctx, ctx->trace_grid, trw, buf + R, cap_rec, count + R, scap, slab_ipar, next_ray, nlim);
+	launch_trace(ctx, t, buf + R, cap_rec, count + R, scap, slab_ipar, next_ray, nlim);
 	PSG_CHECK_LAUNCH();
 	k_rec_counts<<<(unsigned)std::min<size_t>(blocks(nray, 256), 4 * (size_t)ctx->sms), 256, 0, st>>>(B, R, h.off,
 			cap_rec, scap, count, ctx->d_counters + 3, ctx->d_status);
@@ -700,13 +762,6 @@ int psg_trace_fill_prepare(psg_context *ctx, size_t nray) {
 			!psg_scratch(ctx, S_OFFSETS, sizeof(int64_t) * (nray + 1) + 256) ||
 			!psg_scratch(ctx, S_REC_U32, sizeof(uint32_t) * (slots ? slots : 1)))
 		return PSG_E_NOMEM;
-	const int trw = std::max(1, std::min(TR_MAX_WARPS, ctx->tune.trace_warps));
-	const size_t smem = trace_smem(ctx, trw);
-	if (smem > 48 * 1024)
-		PSG_CUDA(cudaFuncSetAttribute(trace_kernel(ctx), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-	int per_sm = 1;
-	PSG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_kernel(ctx), 32 * trw, smem));
-	ctx->trace_grid = (unsigned)std::min<size_t>(blocks(nray, trw), (size_t)std::max(per_sm, 1) * ctx->sms);
 	return PSG_OK;
 }
 
@@ -726,11 +781,9 @@ int psg_trace_fill(psg_context *ctx, const psg_ray *d_rays, size_t nray, PsgTrac
 	int64_t *off64 = (int64_t *)offmem;
 	unsigned long long *d_max = ctx->d_counters + 4;
 	unsigned long long *next_ray = ctx->d_counters + 9;
-	const int sms = ctx->sms;
-	const int trw = std::max(1, std::min(TR_MAX_WARPS, ctx->tune.trace_warps));
-	const size_t smem = trace_smem(ctx, trw);
-	if (smem > 48 * 1024)
-		PSG_CUDA(cudaFuncSetAttribute(trace_kernel(ctx), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+	TracePlan tp;
+	const int prc = plan_trace(ctx, nray, true, &tp);
+	if (prc) return prc;
 	size_t scap = 0;
 	unsigned long long hdr[2] = {0, 0};      // longest list, hit total
 	for (int attempt = 0; attempt < 2; attempt++) {
@@ -738,15 +791,12 @@ int psg_trace_fill(psg_context *ctx, const psg_ray *d_rays, size_t nray, PsgTrac
 		const size_t slots = nray * scap;
 		uint32_t *slab_ipar = (uint32_t *)psg_scratch(ctx, S_REC_U32, sizeof(uint32_t) * (slots ? slots : 1));
 		if (!slab_ipar) return PSG_E_NOMEM;
-		PSG_CUDA(cudaMemsetAsync(count + nray, 0, sizeof(uint32_t), st));
+		PSG_CUDA(cudaMemsetAsync(tp.nstart ? count : count + nray, 0, sizeof(uint32_t) * (tp.nstart ? nray + 1 : 1), st));
 		PSG_CUDA(cudaMemsetAsync(d_max, 0, 2 * sizeof(unsigned long long), st));
 		psg_mark_begin(ctx, PSG_K_TRACE_FILL);
 		if (nray) {
 			PSG_CUDA(cudaMemsetAsync(next_ray, 0, sizeof(unsigned long long), st));
-			int per_sm = 1;
-			PSG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_kernel(ctx), 32 * trw, smem));
-			const unsigned tgrid = (unsigned)std::min<size_t>(blocks(nray, trw), (size_t)std::max(per_sm, 1) * sms);
-			launch_trace(ctx, tgrid, trw, d_rays, nray, count, scap, slab_ipar, next_ray, nullptr);
+			launch_trace(ctx, tp, d_rays, nray, count, scap, slab_ipar, next_ray, nullptr);
 		}
 		PSG_CHECK_LAUNCH();
 		psg_mark_end(ctx);

@@ -425,6 +425,8 @@ extern "C" int psg_build_tree(psg_context *ctx, int ppc) {
 	ctx->skipped = n - nvalid;
 	ctx->depth = nlevels - 1;
 	ctx->ppc = ppc;
+	for (int l = 1; l <= 3; l++)      // (level l is whole where every cell above it was split)
+		ctx->level_start[l] = l < nlevels && level_end[l] - level_begin[l] == 1 << (3 * l) ? level_begin[l] : 0;
 	ctx->have_tree = 1;
 	return PSG_OK;
 }
