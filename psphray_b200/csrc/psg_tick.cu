@@ -801,18 +801,21 @@ struct TickRays {
 	int l0, nlong, m0, nmid, s0, nshort, pad0, pad1;
 };
 
-// Work units of a tick: [0, nlong) take one long ray each with all
-// DEP_THREADS threads; the next ceil(nmid/4) take four middle rays each, 128
-// threads per ray; the rest take DEP_THREADS/32 short rays, one per warp.
-// The grid is persistent: blocks claim units from the tick's counter, so
-// the launch needs no count from the host.
+// A tick's rays: blocks take the long ones, all their threads on each, then
+// their 128-thread quarters the middle ones, then their warps the short ones;
+// a group that is done moves on by itself. (Units of 16 short rays per block
+// kept 15 warps waiting for the longest ray of each unit.) The grid is
+// persistent and needs no count from the host: a group's first ray is the
+// one of its own index, dealt so that few rays spread over all blocks, the
+// quarters and warps from the blocks without a long ray on; further ones come
+// from the tick's two counters. Deposit per call: 8 x 8192 rays on 2M
+// particles 1.24 -> 0.96 ms, 4 x 65536 on 16.8M 10.7 -> 8.5 ms, helium 4 x 8192
+// 2.6 -> 2.1 ms, 6 x 3100 0.41 -> 0.38 ms; 100 x 1024 unchanged
 #define DEP_THREADS 512
-#define DEP_LONG 96       // more hits than this: a group of threads, else a warp
-#define DEP_MID 384       // more hits than this: the whole block, else a 128-thread quarter
 
 template <bool GEN, bool AFF>
 __global__ void __launch_bounds__(DEP_THREADS, 2) k_deposit(int t, const TickRays *__restrict__ tick_rays,
-		unsigned *__restrict__ unit_ctr, const PsgBatchDev *__restrict__ B,
+		unsigned *__restrict__ ctr, int nctr, const PsgBatchDev *__restrict__ B,
 		const uint32_t *__restrict__ long_rays, const uint32_t *__restrict__ mid_rays,
 		const uint32_t *__restrict__ short_rays, int dep_long, int dep_mid,
 		const int64_t *__restrict__ off, const uint32_t *__restrict__ hipar, const double *__restrict__ hkern,
@@ -822,44 +825,44 @@ __global__ void __launch_bounds__(DEP_THREADS, 2) k_deposit(int t, const TickRay
 	__shared__ DepShared sh_block;
 	__shared__ DepShared sh_quarter[4];
 	__shared__ DepShared sh_warp[DEP_THREADS / 32];
-	__shared__ int s_unit;
+	__shared__ int s_next[4];
 	const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
 	unsigned nsat = 0;
 	double tm_lost = 0.0;
 	const psg_ray *__restrict__ rays = B->rays;      // read here: a replayed graph serves any call's rays
 	const TickRays T = tick_rays[t];
-	const int nlong = T.nlong, nmid = T.nmid, nshort = T.nshort;
-	const int nmid_blocks = (nmid + 3) / 4;
-	const int nunits = nlong + nmid_blocks + (nshort + DEP_THREADS / 32 - 1) / (DEP_THREADS / 32);
-	// the first unit is the block's own index, later ones come from the
-	// counter (a tick with no more units than blocks touches it not at all)
-	for (int u = (int)blockIdx.x; u < nunits;) {
-		if (u < nlong) {
-			const uint32_t r = long_rays[T.l0 + u];
-			deposit_any<DEP_THREADS, GEN, AFF>(rays[r], off[r], off[r + 1], tid, dep_long, dep_mid, hipar, hkern, lambdaH,
-					mass, P, want_heat, acc, nacc, sh_block, nsat, tm_lost, 0);
-		} else if (u < nlong + nmid_blocks) {
-			const int q = tid >> 7;
-			const int m = (u - nlong) * 4 + q;
-			if (m < nmid) {
-				const uint32_t r = mid_rays[T.m0 + m];
-				deposit_any<128, GEN, AFF>(rays[r], off[r], off[r + 1], tid & 127, dep_long, dep_mid, hipar, hkern, lambdaH,
-						mass, P, want_heat, acc, nacc, sh_quarter[q], nsat, tm_lost, 1 + q);
-			}
-		} else {
-			const int w = (u - nlong - nmid_blocks) * (DEP_THREADS / 32) + wid;
-			if (w < nshort) {
-				const uint32_t r = short_rays[T.s0 + w];
-				if (off[r + 1] > off[r])
-					deposit_any<32, GEN, AFF>(rays[r], off[r], off[r + 1], lane, dep_long, dep_mid, hipar, hkern, lambdaH,
-							mass, P, want_heat, acc, nacc, sh_warp[wid], nsat, tm_lost, 0);
-			}
+	const int G = (int)gridDim.x;
+	if ((int)blockIdx.x < T.nlong) {      // (fewer than G: each has more than 1/G of the tick's hits)
+		const uint32_t r = long_rays[T.l0 + (int)blockIdx.x];
+		deposit_any<DEP_THREADS, GEN, AFF>(rays[r], off[r], off[r + 1], tid, dep_long, dep_mid, hipar, hkern, lambdaH, mass,
+				P, want_heat, acc, nacc, sh_block, nsat, tm_lost, 0);
+	}
+	// (with few rays the blocks that had a long one take no more: F others share)
+	const int L = min(T.nlong, G / 2), F = G - L, b = (int)blockIdx.x - L;
+	const int q = tid >> 7;
+	for (int u = b >= 0 ? q * F + b : -1; u < T.nmid;) {
+		if (u >= 0) {
+			const uint32_t r = mid_rays[T.m0 + u];
+			deposit_any<128, GEN, AFF>(rays[r], off[r], off[r + 1], tid & 127, dep_long, dep_mid, hipar, hkern, lambdaH, mass,
+					P, want_heat, acc, nacc, sh_quarter[q], nsat, tm_lost, 1 + q);
 		}
-		if (nunits <= (int)gridDim.x) break;
-		if (tid == 0) s_unit = (int)(gridDim.x + atomicAdd(unit_ctr + t, 1u));
-		__syncthreads();
-		u = s_unit;
-		__syncthreads();       // (also: the unit's shared state is no longer read)
+		if (T.nmid <= 4 * F) break;
+		if ((tid & 127) == 0) s_next[q] = 4 * F + (int)atomicAdd(ctr + t, 1u);
+		group_sync<128>(1 + q);
+		u = s_next[q];
+		group_sync<128>(1 + q);
+	}
+	constexpr int NW = DEP_THREADS / 32;
+	// (a warp each where that fits beside the middle ones, else as warps come free)
+	const int D = 4 * T.nmid + T.nshort <= NW * F ? NW * F : 0;
+	for (int u = D && b >= 0 ? (NW - 1 - wid) * F + b : -1; u < T.nshort;) {
+		const uint32_t r = u >= 0 ? short_rays[T.s0 + u] : 0u;
+		if (u >= 0 && off[r + 1] > off[r])
+			deposit_any<32, GEN, AFF>(rays[r], off[r], off[r + 1], lane, dep_long, dep_mid, hipar, hkern, lambdaH, mass, P,
+					want_heat, acc, nacc, sh_warp[wid], nsat, tm_lost, 0);
+		if (D) break;
+		if (lane == 0) u = (int)atomicAdd(ctr + nctr + t, 1u);
+		u = __shfl_sync(0xffffffffu, u, 0);
 	}
 	for (int o = 16; o > 0; o >>= 1) nsat += __shfl_down_sync(0xffffffffu, nsat, o);
 	if (lane == 0 && nsat) atomicAdd(n_sat, (unsigned long long)nsat);
@@ -893,13 +896,13 @@ __global__ void k_tick_rays(int K, size_t R, size_t nray, const unsigned long lo
 // narrow groups they are better: a warp takes the rays of up to as many hits
 // as each resident warp gets of the tick, a quarter those of up to as many
 // as each resident block gets. Measured (deposit per call, groups as wide as
-// the steps -> by load): 8 x 8192 rays of 690 hits 1.95 -> 1.24 ms, 4 x 65536
-// of 1200 15.8 -> 11.2 ms, 6 x 3100 of 550 0.50 -> 0.41 ms; helium 4 x 8192
-// 5.7 -> 2.6 ms, 8 x 1324 of 320 3.58 -> 1.45 ms. 1024 rays of 120 hits are
+// the steps -> by load): 8 x 8192 rays of 690 hits 1.95 -> 0.96 ms, 4 x 65536
+// of 1200 15.8 -> 8.5 ms, 6 x 3100 of 550 0.50 -> 0.38 ms; helium 4 x 8192
+// 5.7 -> 2.1 ms, 8 x 1324 of 320 3.58 -> 1.47 ms. 1024 rays of 120 hits are
 // too few to narrow (26 hits per warp): at 192 instead of 96 the deposit took
 // 2.05 instead of 1.71 ms. The warp's bound stops at DEP_WARP_MAX: past it
-// the longest rays trail the tick (65536 rays of up to 4000 hits: 14.3 ms
-// without the bound; 384, 768 and 1500 measure within 5%).
+// the longest rays trail the tick (65536 rays of up to 4000 hits: 14.3
+// instead of 11.2 ms without the bound; 384, 768 and 1500 within 5%).
 #define DEP_WARP_MAX 768
 __global__ void k_ray_class(size_t nray, size_t R, const int64_t *__restrict__ off, int dep_long, int dep_mid,
 		int dep_warps, unsigned long long *__restrict__ cls) {
@@ -2097,7 +2100,7 @@ UpdView upd_view(psg_context *ctx, const BatchPlan &pl) {
 	v.nstiff = v.cursors + (pl.K + 1);
 	v.nrej = v.nstiff + (pl.K + 1);
 	v.dep_ctr = v.nrej + (pl.K + 1);
-	v.cursors2 = v.dep_ctr + (pl.K + 1);       // the integrator's second pass (update_order)
+	v.cursors2 = v.dep_ctr + 2 * (pl.K + 1);   // the integrator's second pass (update_order)
 	v.stiff_ctr = v.cursors2 + (pl.K + 1);     // the stiff finish's
 	v.tick_rays = (TickRays *)(((uintptr_t)(v.stiff_ctr + pl.K + 1) + 31) & ~(uintptr_t)31);
 	v.stiff = (StiffItem *)(((uintptr_t)(v.tick_rays + pl.K) + 15) & ~(uintptr_t)15);
@@ -2106,7 +2109,7 @@ UpdView upd_view(psg_context *ctx, const BatchPlan &pl) {
 	return v;
 }
 size_t upd_bytes(const BatchPlan &pl) {
-	return sizeof(double) * (pl.helium ? 4 : 2) * pl.cap + sizeof(unsigned) * 6 * (pl.K + 1) + sizeof(TickRays) * pl.K +
+	return sizeof(double) * (pl.helium ? 4 : 2) * pl.cap + sizeof(unsigned) * 7 * (pl.K + 1) + sizeof(TickRays) * pl.K +
 			(pl.iso ? 0 : sizeof(StiffItem) * pl.pcap + pl.cap) + (pl.surr ? sizeof(uint32_t) * pl.pcap : 0) + 512;
 }
 
@@ -2258,7 +2261,7 @@ int enqueue_batch(psg_context *ctx, const BatchPlan &pl, const PsgBatchDev *B) {
 
 	// the long-segment lists and (not isothermal) the integrator's work
 	// cursors, stiff lists and the deposit's unit counters
-	PSG_CUDA(cudaMemsetAsync(uv.cursors, 0, sizeof(unsigned) * 6 * (K + 1), st));
+	PSG_CUDA(cudaMemsetAsync(uv.cursors, 0, sizeof(unsigned) * 7 * (K + 1), st));
 	if (pl.surr) PSG_CUDA(cudaMemsetAsync(ctx->d_counters + 8, 0, sizeof(unsigned long long), st));
 	UpdRec *urec = (!pl.helium && pl.euler) ? (UpdRec *)ctx->scratch[S_REC].p : nullptr;
 	HeStiffItem *hstiff = pl.helium ? (HeStiffItem *)ctx->scratch[S_REC].p : nullptr;
@@ -2299,15 +2302,15 @@ int enqueue_batch(psg_context *ctx, const BatchPlan &pl, const PsgBatchDev *B) {
 	for (size_t t = 0; t < K; t++) {
 		psg_mark_begin(ctx, PSG_K_DEPOSIT);
 		if (pl.gen)
-			k_deposit<true, false><<<pl.dep_grid, DEP_THREADS, 0, st>>>((int)t, uv.tick_rays, uv.dep_ctr, B,
+			k_deposit<true, false><<<pl.dep_grid, DEP_THREADS, 0, st>>>((int)t, uv.tick_rays, uv.dep_ctr, (int)K + 1, B,
 					long_rays, mid_rays, short_rays, ctx->tune.deposit_long, ctx->tune.deposit_mid, off64, hit_ipar, hit_kern, ctx->d_lambdaH, ctx->d_mass, P,
 					pl.want_heat, acc, pl.nacc, d_nsat, d_lost);
 		else if (pl.aff)
-			k_deposit<false, true><<<pl.dep_grid, DEP_THREADS, 0, st>>>((int)t, uv.tick_rays, uv.dep_ctr, B,
+			k_deposit<false, true><<<pl.dep_grid, DEP_THREADS, 0, st>>>((int)t, uv.tick_rays, uv.dep_ctr, (int)K + 1, B,
 					long_rays, mid_rays, short_rays, ctx->tune.deposit_long, ctx->tune.deposit_mid, off64, hit_ipar, hit_kern, ctx->d_lambdaH, ctx->d_mass, P,
 					pl.want_heat, acc, pl.nacc, d_nsat, d_lost);
 		else
-			k_deposit<false, false><<<pl.dep_grid, DEP_THREADS, 0, st>>>((int)t, uv.tick_rays, uv.dep_ctr, B,
+			k_deposit<false, false><<<pl.dep_grid, DEP_THREADS, 0, st>>>((int)t, uv.tick_rays, uv.dep_ctr, (int)K + 1, B,
 					long_rays, mid_rays, short_rays, ctx->tune.deposit_long, ctx->tune.deposit_mid, off64, hit_ipar, hit_kern, ctx->d_lambdaH, ctx->d_mass, P,
 					pl.want_heat, acc, pl.nacc, d_nsat, d_lost);
 		PSG_CHECK_LAUNCH();

@@ -77,3 +77,27 @@ def test_groups_do_not_change_deposits(physics, long, mid, boost):
     if helium:
         for k in ("lambdaHeI", "lambdaHeII"):
             np.testing.assert_array_equal(he_a[k][free], he_b[k][free])
+
+
+@pytest.mark.parametrize("physics", ["iso", "helium"])
+@pytest.mark.parametrize("n", [1100, 1200, 2500])
+def test_more_rays_than_quarters(physics, n):
+    """As above, the bright rays behind a crowd that 128-thread quarters take,
+    just fewer and more of them than the chip holds."""
+    helium = physics == "helium"
+    units = Units(hmf=0.76 if helium else 1.0)
+    f = fields.uniform_field(40, 5, units=units)
+    phys = api.Physics(units, isothermal=physics == "iso", h_only=not helium, secondary_ionization=helium)
+    nph = float(f.mass[0]) * phys.unit("H_PER_MASS")
+    bright, crowd = _rays(f, 37, nph, 2), _crowd(f, n)
+    a, he_a, sat_a = _run(f, phys, [bright], 32, 32)
+    b, he_b, sat_b = _run(f, phys, [np.concatenate([crowd, bright])], 32, 32)
+    c, _, _ = _run(f, phys, [crowd], 32, 32)
+    free = c["lasthit"] == 0
+    assert (free & (a["lasthit"] == 1)).sum() > 2000
+    assert sat_a == sat_b
+    for k in ("lambdaH", "ie", "hits", "lasthit"):
+        np.testing.assert_array_equal(a[k][free], b[k][free])
+    if helium:
+        for k in ("lambdaHeI", "lambdaHeII"):
+            np.testing.assert_array_equal(he_a[k][free], he_b[k][free])
