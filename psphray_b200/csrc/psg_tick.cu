@@ -147,15 +147,26 @@ __global__ void k_act_build(size_t KN, uint32_t N, int K, const unsigned long lo
 
 // one warp per ray: every hit into its key's run, at the slot its counter
 // (the run's end, counting down) gives; vals[slot] = the hit. The counters
-// are left at the runs' first slots (zeroed before the next batch).
+// are left at the runs' first slots (zeroed before the next batch). What
+// bounds it: L2's rate of returning atomics and 4-byte scattered stores, and
+// past L2's size the sectors those stores write back and read again. So a
+// tick whose slots take more than SLOT_PART bytes is placed in parts, the
+// particles [p0, p0 + np) (whose slots are one stretch of vals) in a launch
+// each; a part more costs a read of ipar. Slots group, 4 x 79M hits on 16.8M
+// particles: one launch 10.6 ms, parts of 160 MB 9.1, 80 MB 8.8, 40 MB 9.6,
+// 20 MB 11.8.
+#define SLOT_PART ((size_t)80 << 20)
 __global__ void k_slot_place(size_t nray, int R, uint32_t N, const int64_t *__restrict__ off,
-		const uint32_t *__restrict__ ipar, uint32_t *__restrict__ cnt, uint32_t *__restrict__ vals) {
+		const uint32_t *__restrict__ ipar, uint32_t *__restrict__ cnt, uint32_t *__restrict__ vals, uint32_t p0,
+		uint32_t np) {
 	const size_t r = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) / 32;
 	const int lane = threadIdx.x & 31;
 	if (r >= nray) return;
 	const size_t kb = (r / (size_t)R) * N;
-	for (int64_t h = off[r] + lane; h < off[r + 1]; h += 32)
-		vals[atomicSub(&cnt[kb + ipar[h]], 1u) - 1u] = (uint32_t)h;
+	for (int64_t h = off[r] + lane; h < off[r + 1]; h += 32) {
+		const uint32_t p = ipar[h];
+		if (p - p0 < np) vals[atomicSub(&cnt[kb + p], 1u) - 1u] = (uint32_t)h;
+	}
 }
 
 // Runs longer than the tuner's run_short (particles next to a source), in three tiers: up to
@@ -2236,8 +2247,12 @@ int enqueue_batch(psg_context *ctx, const BatchPlan &pl, const PsgBatchDev *B) {
 	k_act_build<<<(unsigned)std::min<size_t>(blocks(pl.KN, 256), (size_t)sms * 16), 256, 0, st>>>(pl.KN, N, (int)K,
 			kbase, av.act_ipar, av.act_seg, av.tick_act, d_nact, kcnt);
 	PSG_CHECK_LAUNCH();
-	k_slot_place<<<blocks(nray * 32, 256), 256, 0, st>>>(nray, (int)R, N, off64, hit_ipar, kcnt, vals);
-	PSG_CHECK_LAUNCH();
+	const size_t parts = std::min<size_t>(sizeof(uint32_t) * (cap / K) / SLOT_PART + 1, 16);
+	const uint32_t np = (uint32_t)((N + parts - 1) / parts);
+	for (uint32_t p0 = 0; p0 < N; p0 += np) {
+		k_slot_place<<<blocks(nray * 32, 256), 256, 0, st>>>(nray, (int)R, N, off64, hit_ipar, kcnt, vals, p0, np);
+		PSG_CHECK_LAUNCH();
+	}
 	ctx->launches += 8;
 	unsigned long long *d_nsat = ctx->d_counters + 1;      // (zeroed by the caller, per call)
 	psg_mark_end(ctx);
