@@ -91,6 +91,47 @@ __device__ __forceinline__ double div3(double x) {
 	return __fma_rn(__fma_rn(-3.0, q, x), y, q);
 }
 
+// Where rhs_he reads its rate rows (7 float4 of the table's 8 hold columns):
+// in device memory, or those of log T from PSG_WIN_LOGT on in the block's
+// shared memory, the others in device memory.
+struct HeRows {
+	const float4 *row;
+	__device__ __forceinline__ HeRows at(const PhysParams &P, int idx) const { return {P.ar_he + 8 * (size_t)idx}; }
+	__device__ __forceinline__ float4 operator[](int c) const { return row[c]; }
+};
+#define HE_WIN_F4 7
+struct HeWindowRow {
+	const float4 *sm, *gl;
+	bool in;
+	__device__ __forceinline__ float4 operator[](int c) const {
+		float4 v;
+		if (in) v = sm[c];
+		else v = gl[c];
+		return v;
+	}
+};
+struct HeWindow {
+	const float4 *sm;
+	int lo, n;
+	// The block copies the rows into buf, 112 bytes each (an odd number of
+	// 16-byte banks), and every thread waits for bar before its first row.
+	__device__ __forceinline__ void start(const PhysParams &P, float4 *buf, int rows, uint64_t *bar) {
+		sm = buf;
+		lo = P.ar_win_lo;
+		n = min(rows, P.ar_nrows - lo);
+		const uint32_t b = (uint32_t)__cvta_generic_to_shared(bar), d = (uint32_t)__cvta_generic_to_shared(buf);
+		const uint32_t row = HE_WIN_F4 * sizeof(float4);
+		if (threadIdx.x == 0) rate_bar_arm(b, n * row);
+		__syncthreads();      // (armed before a copy ends or anyone waits)
+		for (int j = threadIdx.x; j < n; j += blockDim.x)
+			rate_bar_copy(d + j * row, P.ar_he + 8 * (size_t)(lo + j), row, b);
+	}
+	__device__ __forceinline__ HeWindowRow at(const PhysParams &P, int idx) const {
+		const int w = idx - lo;
+		return {sm + HE_WIN_F4 * w, P.ar_he + 8 * (size_t)idx, (unsigned)w < (unsigned)n};
+	}
+};
+
 // function() solve.c:76-141 with helium (the rates of FETCH_VARS
 // solve.c:42-73); x = (lambdaH, lambdaHeI, lambdaHeII, ie), the derivative
 // per unit normalised time. On the spot (case B) the helium equations use
@@ -100,8 +141,9 @@ __device__ __forceinline__ double div3(double x) {
 // solve.c, each rounded; the rates come two columns to a 16-byte load from
 // the row of tabfun_get() tabfun.c:38-58 (clamped rows, a NaN temperature
 // included: offset 0), FP32 value + slope * offset in FP64.
+template <typename ROWS = HeRows>
 __device__ __forceinline__ void rhs_he(const PhysParams &P, const HeCtx &c, const double x[4], double dx[4],
-		double *rec = nullptr) {
+		double *rec = nullptr, const ROWS &rows = ROWS()) {
 	const double xHI = x[0], xHII = 1.0 - x[0], xHeII = x[2];
 	const double xHeIII = 1.0 - x[2] - x[1];
 	const double ye = (xHII + P.he_f * (xHeII + 2 * xHeIII)) + c.yeMET;
@@ -118,7 +160,7 @@ __device__ __forceinline__ void rhs_he(const PhysParams &P, const HeCtx &c, cons
 			du = logT - __fma_rn((double)idx, P.ar_step, P.ar_min);
 		}
 	}
-	const float4 *row = P.ar_he + 8 * (size_t)idx;
+	const auto row = rows.at(P, idx);
 	const float4 q0 = row[0], q1 = row[1], q2 = row[2];
 #define PSG_RATE(v, s, col) (__fma_rn((double)(s), du, (double)(v)) * P.ar_he_scale[col])
 	const double nH = c.nH, t = c.t;
@@ -405,9 +447,9 @@ __device__ __forceinline__ void he_dp_start(HeDp &S, const double k1[4], const d
 // One pass over the lanes' next work: for fresh lanes the slope at x first,
 // then for all lanes one attempted step. fresh must be the warp's when other
 // lanes call too: anyfresh says whether any lane's is set.
-template <bool REC>
+template <bool REC, typename ROWS = HeRows>
 __device__ __forceinline__ void he_dp_step(const PhysParams &P, const HeCtx &c, HeDp &S, bool fresh, bool anyfresh,
-		double *k, int stride) {
+		double *k, int stride, const ROWS &rows = ROWS()) {
 	double e[4], y[4], q[3], h = 0.0;
 #pragma unroll 1
 	for (int st = anyfresh ? -1 : 0; st < 6; st++) {
@@ -440,7 +482,7 @@ __device__ __forceinline__ void he_dp_step(const PhysParams &P, const HeCtx &c, 
 			}
 		}
 		double dx[4], r[3];
-		rhs_he(P, c, y, dx, REC ? r : nullptr);
+		rhs_he(P, c, y, dx, REC ? r : nullptr, rows);
 		if (st < 0) {
 			he_dp_start<REC>(S, dx, r, k, stride);
 		} else if (st < 5) {

@@ -206,6 +206,32 @@ struct RateRows {
 		for (int c = 0; c < 4; c++) v[c] = row[c];
 	}
 };
+// An mbarrier armed for that many bytes, a bulk copy counted on it, and the
+// wait for all of them (false if they did not come within the limit; it takes
+// microseconds).
+__device__ __forceinline__ void rate_bar_arm(uint32_t bar, uint32_t bytes) {
+	asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+	asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+	asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void rate_bar_copy(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
+	asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src),
+			"r"(bytes), "r"(bar)
+			: "memory");
+}
+__device__ __forceinline__ bool rate_bar_wait(uint64_t *bar) {
+	const uint32_t b = (uint32_t)__cvta_generic_to_shared(bar);
+	for (int i = 0; i < (1 << 22); i++) {
+		uint32_t done;
+		asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n\t"
+					 "selp.u32 %0, 1, 0, p;\n\t}\n"
+					 : "=r"(done)
+					 : "r"(b)
+					 : "memory");
+		if (done) return true;
+	}
+	return false;
+}
 struct RateWindow {
 	const float4 *sm;
 	int lo, n;
@@ -218,29 +244,10 @@ struct RateWindow {
 		if (threadIdx.x == 0) {
 			const uint32_t b = (uint32_t)__cvta_generic_to_shared(bar), d = (uint32_t)__cvta_generic_to_shared(buf);
 			const uint32_t bytes = (uint32_t)n * (5 * sizeof(float4));
-			asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(b) : "memory");
-			asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-			asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"(bytes) : "memory");
-			if (bytes)
-				asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(d),
-						"l"(P.ar_win), "r"(bytes), "r"(b)
-						: "memory");
+			rate_bar_arm(b, bytes);
+			if (bytes) rate_bar_copy(d, P.ar_win, bytes, b);
 		}
 		__syncthreads();      // (the barrier is armed before anyone waits on it)
-	}
-	// false if the copy did not end within the limit (it takes microseconds)
-	__device__ __forceinline__ bool wait(uint64_t *bar) const {
-		const uint32_t b = (uint32_t)__cvta_generic_to_shared(bar);
-		for (int i = 0; i < (1 << 22); i++) {
-			uint32_t done;
-			asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n\t"
-						 "selp.u32 %0, 1, 0, p;\n\t}\n"
-						 : "=r"(done)
-						 : "r"(b)
-						 : "memory");
-			if (done) return true;
-		}
-		return false;
 	}
 	__device__ __forceinline__ void get(const PhysParams &P, int idx, float4 v[4]) const {
 		const unsigned w = (unsigned)(idx - lo);

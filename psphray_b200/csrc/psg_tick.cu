@@ -1388,7 +1388,7 @@ __global__ void __launch_bounds__(UPD_THREADS, 1) k_update_queue(int t, const in
 		}
 		if (!__any_sync(0xffffffffu, have)) break;
 		if (!rows_here) {
-			rows_here = rows.wait(bar);
+			rows_here = rate_bar_wait(bar);
 			if (!rows_here) {      // (never seen: fall back on device memory, and say so)
 				rows.n = 0;
 				st |= PSG_ST_COPY;
@@ -1421,7 +1421,7 @@ __global__ void __launch_bounds__(UPD_THREADS, 1) k_update_queue(int t, const in
 			}
 		}
 	}
-	if (!rows_here && !rows.wait(bar)) st |= PSG_ST_COPY;      // (no block leaves with its copy in flight)
+	if (!rows_here && !rate_bar_wait(bar)) st |= PSG_ST_COPY;      // (no block leaves with its copy in flight)
 	if (st) atomicOr(status, st);
 }
 
@@ -1682,16 +1682,31 @@ __device__ __forceinline__ HeStep load_he_step(const PhysParams &P, const HeSrc 
 // on average on the 2M-particle field: a thread per particle kept half the
 // lanes waiting for the warp's slowest), and the stages' slopes live in
 // shared memory (see HeDp). A particle still unfinished after the explicit
-// steps goes to k_update_he_stiff.
-#define HEQ_THREADS 128
-#define HEQ_BLOCKS 5
+// steps goes to k_update_he_stiff. What bounds it: the latency of a step, 20
+// (16 with REC) warps to a multiprocessor, and at the end the chain of the
+// last 32-step particle. One block fills the multiprocessor, as many threads
+// as the registers allow nearly without spills (REC: 640 threads measured
+// 5.07 ms), and copies the rate rows of log T 3 to 6.9 beside the slopes
+// (HeWindow). Measured, update group per call, rows from device memory ->
+// from shared memory: 2M particles 4.30 -> 4.12 ms (4 ticks; 4.25 with 512
+// threads), 262K with REC 4.97 -> 4.67 ms (8 ticks).
 template <bool REC>
-__global__ void __launch_bounds__(HEQ_THREADS, HEQ_BLOCKS) k_update_he(int t, const int32_t *__restrict__ tick_act,
+struct Heq {
+	static constexpr int threads = REC ? 512 : 640, rows = 975;
+	static constexpr int slopes = 24 * threads * 8, smem = slopes + rows * HE_WIN_F4 * 16 + 16;
+	static_assert(smem <= 227 * 1024, "k_update_he's shared memory");
+};
+template <bool REC>
+__global__ void __launch_bounds__(Heq<REC>::threads, 1) k_update_he(int t, const int32_t *__restrict__ tick_act,
 		const HeSrc src, double *__restrict__ lambdaH, float *__restrict__ ie, int64_t *__restrict__ lasthit,
 		PhysParams P, const PsgBatchDev *__restrict__ B, unsigned *__restrict__ cursor,
 		HeStiffItem *__restrict__ stiff, unsigned *__restrict__ nstiff, uint32_t *__restrict__ status) {
-	__shared__ double slopes[24 * HEQ_THREADS];
-	double *k = slopes + threadIdx.x;
+	extern __shared__ __align__(16) char heq_smem[];
+	double *k = reinterpret_cast<double *>(heq_smem) + threadIdx.x;
+	uint64_t *bar = reinterpret_cast<uint64_t *>(heq_smem + Heq<REC>::smem - 16);
+	HeWindow rows;
+	rows.start(P, reinterpret_cast<float4 *>(heq_smem + Heq<REC>::slopes), Heq<REC>::rows, bar);
+	bool rows_here = false;
 	const int64_t tick = B->tick0 + t;
 	const double tick_time = B->tick_time;
 	const int lo = tick_act[t], n = tick_act[t + 1] - lo;
@@ -1722,8 +1737,15 @@ __global__ void __launch_bounds__(HEQ_THREADS, HEQ_BLOCKS) k_update_he(int t, co
 		}
 		if (!__any_sync(0xffffffffu, have)) break;
 		const bool anyfresh = __any_sync(0xffffffffu, fresh);
+		if (!rows_here) {
+			if (!rate_bar_wait(bar)) {      // (never seen: fall back on device memory, and say so)
+				rows.n = 0;
+				st |= PSG_ST_COPY;
+			}
+			rows_here = true;
+		}
 		if (have) {
-			he_dp_step<REC>(P, cx, S, fresh, anyfresh, k, HEQ_THREADS);
+			he_dp_step<REC>(P, cx, S, fresh, anyfresh, k, Heq<REC>::threads, rows);
 			double rec[3] = {0.0, 0.0, 0.0};
 			if (S.t >= 1.0 || S.steps >= HE_SWITCH) {
 				have = false;
@@ -1753,6 +1775,7 @@ __global__ void __launch_bounds__(HEQ_THREADS, HEQ_BLOCKS) k_update_he(int t, co
 			}
 		}
 	}
+	if (!rows_here && !rate_bar_wait(bar)) st |= PSG_ST_COPY;      // (no block leaves with its copies in flight)
 	if (st) atomicOr(status, st);
 }
 
@@ -2200,8 +2223,12 @@ int plan_batch(psg_context *ctx, size_t R, size_t K, const PsgTraceFill &tf, Bat
 	if (!pl.iso && !pl.euler && !pl.helium)
 		PSG_CUDA(!ctx->flags.on_the_spot ? cudaFuncSetAttribute(k_update_queue<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, UPD_SMEM)
 				: cudaFuncSetAttribute(k_update_queue<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, UPD_SMEM));
-	pl.he_grid = pl.euler ? occ_grid(ctx, k_update_he_euler, 128) : ctx->flags.on_the_spot
-			? occ_grid(ctx, k_update_he<false>, HEQ_THREADS) : occ_grid(ctx, k_update_he<true>, HEQ_THREADS);
+	if (!pl.euler && pl.helium)
+		PSG_CUDA(!ctx->flags.on_the_spot ? cudaFuncSetAttribute(k_update_he<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+				Heq<true>::smem)
+				: cudaFuncSetAttribute(k_update_he<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+				Heq<false>::smem));
+	pl.he_grid = pl.euler ? occ_grid(ctx, k_update_he_euler, 128) : (unsigned)ctx->sms;
 	pl.stiff_grid = pl.helium ? (ctx->flags.on_the_spot ? occ_grid(ctx, k_update_he_stiff<false>, STIFF_THREADS)
 			: occ_grid(ctx, k_update_he_stiff<true>, STIFF_THREADS)) : occ_grid(ctx, k_update_stiff<true>, STIFF_THREADS);
 	pl.euler_grid = occ_grid(ctx, k_update_euler, 128);
@@ -2349,10 +2376,10 @@ int enqueue_batch(psg_context *ctx, const BatchPlan &pl, const PsgBatchDev *B) {
 				continue;
 			}
 			if (P.ygrec)
-				k_update_he<true><<<pl.he_grid, HEQ_THREADS, 0, st>>>((int)t, av.tick_act, hs, ctx->d_lambdaH, ctx->d_ie,
+				k_update_he<true><<<pl.he_grid, Heq<true>::threads, Heq<true>::smem, st>>>((int)t, av.tick_act, hs, ctx->d_lambdaH, ctx->d_ie,
 						ctx->d_lasthit, P, B, uv.cursors + t, hstiff, uv.nstiff + t, ctx->d_status);
 			else
-				k_update_he<false><<<pl.he_grid, HEQ_THREADS, 0, st>>>((int)t, av.tick_act, hs, ctx->d_lambdaH, ctx->d_ie,
+				k_update_he<false><<<pl.he_grid, Heq<false>::threads, Heq<false>::smem, st>>>((int)t, av.tick_act, hs, ctx->d_lambdaH, ctx->d_ie,
 						ctx->d_lasthit, P, B, uv.cursors + t, hstiff, uv.nstiff + t, ctx->d_status);
 			PSG_CHECK_LAUNCH();
 			if (P.ygrec)
