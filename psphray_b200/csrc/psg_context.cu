@@ -129,6 +129,8 @@ extern "C" void psg_destroy(psg_context *ctx) {
 	for (auto &b : ctx->scratch) if (b.p) cudaFree(b.p);
 	for (auto &ev : ctx->ev) if (ev) cudaEventDestroy(ev);
 	for (auto &ev : ctx->kev) if (ev) cudaEventDestroy(ev);
+	for (auto &ev : ctx->copy_event) if (ev) cudaEventDestroy(ev);
+	if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
 	cudaStreamDestroy(ctx->own_stream);
 	delete ctx;
 }
@@ -599,22 +601,30 @@ static int to_caller(psg_context *ctx, T *host, const T *dev) {
 
 // Several arrays at once: one kernel puts them all into the caller's order,
 // their copies follow, one wait ends them (for a small field each launch and
-// wait costs more than its bytes).
+// wait costs more than its bytes). From READ_SPLIT bytes on a kernel per array,
+// whose copy overlaps the next one's, and per READ_PART bytes of it: the
+// stores are scattered, and past L2's size their sectors are written back in
+// pieces. Reading 24 bytes a particle: 16.8M particles 9.6 -> 7.7 ms, 2M 0.96
+// -> 0.93 ms (the copies alone 7.2 and 0.9); 1M (24 MB) 0.48 ms either way.
+#define READ_SPLIT ((size_t)32 << 20)
+#define READ_PART ((size_t)64 << 20)
 struct ReadJob {
 	void *host;
 	const void *dev;
 	int item;          // bytes of an element: 4 or 8
 	size_t off;        // in the staging memory
 };
-#define READ_JOBS 5
 struct ReadJobs {
 	ReadJob j[READ_JOBS];
 	int n;
 };
-__global__ void k_scatter_all(size_t n, const uint32_t *__restrict__ g, ReadJobs jobs, char *__restrict__ out) {
+// (the particles whose caller index is in [c0, c0 + nc))
+__global__ void k_scatter_all(size_t n, const uint32_t *__restrict__ g, ReadJobs jobs, char *__restrict__ out, size_t c0,
+		size_t nc) {
 	const size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
 	if (k >= n) return;
 	const size_t c = g[k];
+	if (c - c0 >= nc) return;
 #pragma unroll
 	for (int i = 0; i < READ_JOBS; i++) {
 		if (i >= jobs.n) break;
@@ -625,7 +635,7 @@ __global__ void k_scatter_all(size_t n, const uint32_t *__restrict__ g, ReadJobs
 }
 static int read_arrays(psg_context *ctx, ReadJobs jobs) {
 	const size_t n = ctx->n;
-	cudaStream_t s = ctx->stream;
+	cudaStream_t s = ctx->stream, cs = s;
 	int m = 0;
 	size_t bytes = 0;
 	for (int i = 0; i < jobs.n; i++) {
@@ -639,12 +649,34 @@ static int read_arrays(psg_context *ctx, ReadJobs jobs) {
 	if (ctx->d_order && m) {
 		stage = (char *)psg_scratch(ctx, S_MAP, bytes);
 		if (!stage) return PSG_E_NOMEM;
-		k_scatter_all<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, ctx->d_order, jobs, stage);
-		PSG_CHECK_LAUNCH();
+		if (bytes < READ_SPLIT) {
+			k_scatter_all<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, ctx->d_order, jobs, stage, 0, n);
+			PSG_CHECK_LAUNCH();
+		} else {
+			if (!ctx->copy_stream) PSG_CUDA(cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking));
+			for (int i = 0; i <= READ_JOBS; i++)
+				if (!ctx->copy_event[i]) PSG_CUDA(cudaEventCreateWithFlags(&ctx->copy_event[i], cudaEventDisableTiming));
+			cs = ctx->copy_stream;
+			for (int i = 0; i < m; i++) {
+				ReadJobs one = {{jobs.j[i]}, 1};
+				const size_t parts = jobs.j[i].item * n / READ_PART + 1, nc = (n + parts - 1) / parts;
+				for (size_t c0 = 0; c0 < n; c0 += nc) {
+					k_scatter_all<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, ctx->d_order, one, stage, c0, nc);
+					PSG_CHECK_LAUNCH();
+				}
+				PSG_CUDA(cudaEventRecord(ctx->copy_event[i], s));
+			}
+		}
 	}
-	for (int i = 0; i < m; i++)
+	for (int i = 0; i < m; i++) {
+		if (cs != s) PSG_CUDA(cudaStreamWaitEvent(cs, ctx->copy_event[i], 0));
 		PSG_CUDA(cudaMemcpyAsync(jobs.j[i].host, stage ? stage + jobs.j[i].off : jobs.j[i].dev, jobs.j[i].item * n,
-				cudaMemcpyDeviceToHost, s));
+				cudaMemcpyDeviceToHost, cs));
+	}
+	if (cs != s) {      // (the staging memory's next use comes after the copies)
+		PSG_CUDA(cudaEventRecord(ctx->copy_event[READ_JOBS], cs));
+		PSG_CUDA(cudaStreamWaitEvent(s, ctx->copy_event[READ_JOBS], 0));
+	}
 	PSG_CUDA(cudaStreamSynchronize(s));
 	return PSG_OK;
 }

@@ -18,6 +18,8 @@
 // take the library segmented sort.
 #define PSG_SORT_MAX 8192
 
+#define READ_JOBS 5      // the most arrays of one state call
+
 // The rate rows the integrator keeps in shared memory: those from this log T
 // on, so many of them (up to log T = 8 with the reference's table; 100 KB).
 #define PSG_WIN_LOGT 3.0
@@ -68,6 +70,8 @@ struct psg_context {
 	int device = 0;
 	cudaStream_t stream = nullptr;       // the stream all work is issued on
 	cudaStream_t own_stream = nullptr;   // created with the context
+	cudaStream_t copy_stream = nullptr;  // large states' way to the host (read_arrays), made at the first
+	cudaEvent_t copy_event[READ_JOBS + 1] = {};
 	char err[512] = {0};
 
 	// physics
