@@ -58,7 +58,7 @@ SIDE_LEGS = ("iliev32", "iliev64", "lognormal128")
 # isothermal (DEPOSIT_HEAT_BYTES); the update reads ~60 B and writes ~40 B
 # of particle state per active (tick, particle) pair.
 BYTES_PER_HIT = 36
-GROUP_BYTES = {"trace_count": (16, "hit"), "trace_fill": (36, "hit"), "sort": (56, "hit"),
+GROUP_BYTES = {"trace_count": (16, "hit"), "trace_fill": (20, "hit"), "sort": (40, "hit"),
                "slots": (24, "hit"), "deposit": (32, "hit"), "update": (100, "active particle")}
 DEPOSIT_HEAT_BYTES = 8
 

@@ -753,7 +753,7 @@ int psg_trace_rec_sort_enqueue(psg_context *ctx, size_t R, size_t nray, unsigned
 }
 
 // Sizes the buffers psg_trace_rec_fill_enqueue uses for nray rays (allocates;
-// before a capture) and its persistent grid.
+// before a capture).
 int psg_trace_fill_prepare(psg_context *ctx, size_t nray) {
 	const size_t scap = ctx->slab_cap;
 	const size_t slots = nray * scap;
