@@ -11,6 +11,7 @@
 // or, with the explicit build, step_evolve_euler() solve.c:225-316.
 #pragma once
 
+#include "psg_div3.h"
 #include "psg_solve.cuh"
 
 // xs_get() atomic-rate.c:126-131 for species s (0 HI, 1 HeI, 2 HeII)
@@ -84,13 +85,6 @@ __device__ __forceinline__ HeCtx make_he_ctx(const HeStep &s) {
 	return c;
 }
 
-// x / 3 correctly rounded (Markstein's theorem: the quotient by the rounded
-// reciprocal, corrected once by its exact remainder).
-__device__ __forceinline__ double div3(double x) {
-	const double y = 1.0 / 3.0, q = x * y;
-	return __fma_rn(__fma_rn(-3.0, q, x), y, q);
-}
-
 // Where rhs_he reads its rate rows (7 float4 of the table's 8 hold columns):
 // in device memory, or those of log T from PSG_WIN_LOGT on in the block's
 // shared memory, the others in device memory.
@@ -148,7 +142,7 @@ __device__ __forceinline__ void rhs_he(const PhysParams &P, const HeCtx &c, cons
 	const double xHeIII = 1.0 - x[2] - x[1];
 	const double ye = (xHII + P.he_f * (xHeII + 2 * xHeIII)) + c.yeMET;
 	const double T = P.isothermal ? c.T
-			: div3(rn_dmul(__ddiv_rn(rn_dmul(P.MPROTON_OVER_BOLTZMANN, x[3]), rn_dadd(P.T_den0, rn_dmul(P.hmf, ye))), 2.0));
+			: psg_div3(rn_dmul(__ddiv_rn(rn_dmul(P.MPROTON_OVER_BOLTZMANN, x[3]), rn_dadd(P.T_den0, rn_dmul(P.hmf, ye))), 2.0));
 	const double logT = log10(T);
 	const double u = (logT - P.ar_min) * P.ar_step_inv;
 	int idx = 0;
