@@ -260,6 +260,14 @@ int psg_get_tune(psg_context *ctx, psg_tune *tune);
 int psg_autotune(psg_context *ctx, const psg_ray *d_rays, size_t R, size_t K, int64_t first_tick,
 		double tick_time, int reps, psg_tune *out, double *best_ms);
 
+/* How long a block of the integrators waits for its copy of the rate rows
+ * into shared memory, in GPU clock cycles (default 4e7, 20 ms; the copy takes
+ * microseconds). A block whose wait runs out reads the rows from device
+ * memory, with the same results, and the call that ran the ticks returns
+ * PSG_E_DEVICE once they are done. 0: every block gives up at once, which
+ * shows a host that error. */
+int psg_set_copy_limit(psg_context *ctx, long long cycles);
+
 /* ---- recombination rays (psphray.onTheSpot = false) ---------------------- */
 /* The recombination half of emit_rays() loop.c:197-232, 273-300, 322-368:
  * from the second tick on, the particles hit in the previous tick by its

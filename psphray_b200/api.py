@@ -231,6 +231,7 @@ def lib() -> C.CDLL:
         "psg_get_sources": ([vp, vp, vp], C.c_int),
         "psg_emit_rays": ([vp, sz, sz, i64, dbl, vp], C.c_int),
         "psg_run_ticks_emit": ([vp, sz, sz, i64, dbl, C.POINTER(TickStats)], C.c_int),
+        "psg_set_copy_limit": ([vp, C.c_longlong], C.c_int),
         "psg_mlp_forward": ([vp, vp, vp, sz, vp], C.c_int),
         "psg_mlp_grad": ([vp, vp, vp, vp, sz, vp, vp], C.c_int),
         "psg_mlp_adam": ([vp, vp, vp, vp, vp, C.c_float, C.c_float, C.c_float, C.c_float, C.c_int], C.c_int),
@@ -582,6 +583,10 @@ class Context:
         for k, v in kw.items():
             setattr(t, k, int(v))
         self._check(lib().psg_set_tune(self.h, C.byref(t)), "psg_set_tune")
+
+    def set_copy_limit(self, cycles: int):
+        """How long the integrators wait for their copies of the rate rows."""
+        self._check(lib().psg_set_copy_limit(self.h, cycles), "psg_set_copy_limit")
 
     def autotune(self, d_rays_ptr: int, nray_per_tick: int, nticks: int, first_tick: int, tick_time: float,
                  reps: int = 2) -> tuple[dict, float]:

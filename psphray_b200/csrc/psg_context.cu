@@ -20,6 +20,18 @@ int psg_fail(psg_context *ctx, int code, const char *fmt, ...) {
 	return code;
 }
 
+// The error of a device status word: every bit that is set, by name.
+int psg_status_fail(psg_context *ctx, uint32_t st) {
+	return psg_fail(ctx, PSG_E_DEVICE, "device status 0x%x:%s%s%s%s%s%s%s", st,
+			(st & PSG_ST_NAN) ? " non-finite state" : "",
+			(st & PSG_ST_SOLVER) ? " integrator step limit" : "",
+			(st & PSG_ST_IE_NEG) ? " negative internal energy" : "",
+			(st & PSG_ST_STACK) ? " traversal stack overflow" : "",
+			(st & PSG_ST_SURR) ? " surrogate tile incomplete" : "",
+			(st & PSG_ST_SLAB) ? " hit list beyond its slab" : "",
+			(st & PSG_ST_COPY) ? " rate rows not copied in time" : "");
+}
+
 int psg_cuda_fail(psg_context *ctx, cudaError_t e, const char *what, const char *file, int line) {
 	const int code = (e == cudaErrorMemoryAllocation) ? PSG_E_NOMEM : PSG_E_CUDA;
 	return psg_fail(ctx, code, "%s: %s (%s:%d)", what, cudaGetErrorString(e), file, line);
@@ -436,6 +448,13 @@ __global__ void k_init_particles(size_t n, const float *pos, const float *sml, c
 	lamHeI[i] = l1;
 	lamHeII[i] = l2;
 	yeMET[i] = (float)yem;
+}
+
+extern "C" int psg_set_copy_limit(psg_context *ctx, long long cycles) {
+	if (!ctx) return PSG_E_INVAL;
+	if (cycles < 0) return psg_fail(ctx, PSG_E_INVAL, "psg_set_copy_limit: negative limit");
+	ctx->copy_cycles = cycles;
+	return PSG_OK;
 }
 
 // The architecture of the device code the runtime loaded for this library

@@ -24,6 +24,9 @@
 // on, so many of them (up to log T = 8 with the reference's table; 100 KB).
 #define PSG_WIN_LOGT 3.0
 #define PSG_WIN_ROWS 1250
+// How long a block waits for them, in GPU clock cycles (20 ms; the copy takes
+// microseconds).
+#define PSG_COPY_CYCLES 40000000ll
 
 // Columns of the helium right-hand side's rate rows, two to a 16-byte load:
 // what case B (on the spot) reads comes first, case A's further ones after it.
@@ -39,7 +42,7 @@ enum {
 #define PSG_ST_IE_NEG 4u       // internal energy would turn negative (solve.c:137-139)
 #define PSG_ST_STACK 8u        // traversal stack overflow
 #define PSG_ST_SURR 16u        // a surrogate tile's tensor-core step did not complete
-#define PSG_ST_COPY 64u        // a block's copy of the rate rows did not end
+#define PSG_ST_COPY 64u        // a block gave up waiting for its copy of the rate rows
 #define PSG_ST_SLAB 32u        // a hit list outgrew its slab in a call without host reads (redone)
 
 // scratch slots
@@ -83,6 +86,7 @@ struct psg_context {
 	                             // right-hand side, values then slopes per log T
 	float4 *d_ar_win = nullptr;  // [ar_win_n][5]: the rows from log T = 3 on that the integrator copies to shared memory
 	int ar_win_lo = 0, ar_win_n = 0;
+	long long copy_cycles = PSG_COPY_CYCLES;      // psg_set_copy_limit
 	double ar_step = 0;
 	double ar_ni_scale[8] = {};  // each d_ar_ni column is stored divided by this
 	float4 *d_ar_he = nullptr;   // [ar_nrows][8]: the helium right-hand side's columns (PSG_HE_*), (value, slope) pairs
@@ -194,6 +198,7 @@ struct psg_context {
 // error helpers ---------------------------------------------------------------
 int psg_fail(psg_context *ctx, int code, const char *fmt, ...);
 int psg_cuda_fail(psg_context *ctx, cudaError_t e, const char *what, const char *file, int line);
+int psg_status_fail(psg_context *ctx, uint32_t st);
 // Address of psg_step_evolve_noalloc's static buffer on the current device
 // (psg_tick.cu); 0 or the cudaError_t of the lookup.
 int psg_noalloc_lookup(unsigned char **base);

@@ -37,6 +37,7 @@ struct PhysParams {
 	double ar_ni_scale[8]; // ... each column divided by its largest magnitude
 	const float4 *ar_win;  // [ar_win_n][5]: rows [ar_win_lo, ar_win_lo + ar_win_n) of ar_ni, spaced for shared memory
 	int ar_win_lo, ar_win_n;
+	long long copy_cycles; // how long a block waits for its copy of them
 	const float4 *ar_he;   // [ar_nrows][8]: the helium right-hand side's columns, (value, slope) pairs
 	double ar_he_scale[PSG_HE_NCOLS];   // ... each column divided by its largest magnitude
 	int ar_nrows;
@@ -207,8 +208,8 @@ struct RateRows {
 	}
 };
 // An mbarrier armed for that many bytes, a bulk copy counted on it, and the
-// wait for all of them (false if they did not come within the limit; it takes
-// microseconds).
+// wait for all of them: false if they did not come within that many clock
+// cycles, and at once with a limit of none.
 __device__ __forceinline__ void rate_bar_arm(uint32_t bar, uint32_t bytes) {
 	asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
 	asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -219,9 +220,11 @@ __device__ __forceinline__ void rate_bar_copy(uint32_t dst, const void *src, uin
 			"r"(bytes), "r"(bar)
 			: "memory");
 }
-__device__ __forceinline__ bool rate_bar_wait(uint64_t *bar) {
+__device__ __forceinline__ bool rate_bar_wait(uint64_t *bar, long long cycles) {
 	const uint32_t b = (uint32_t)__cvta_generic_to_shared(bar);
-	for (int i = 0; i < (1 << 22); i++) {
+	if (!cycles) return false;
+	const long long t0 = clock64();
+	do {
 		uint32_t done;
 		asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n\t"
 					 "selp.u32 %0, 1, 0, p;\n\t}\n"
@@ -229,7 +232,7 @@ __device__ __forceinline__ bool rate_bar_wait(uint64_t *bar) {
 					 : "r"(b)
 					 : "memory");
 		if (done) return true;
-	}
+	} while (clock64() - t0 < cycles);
 	return false;
 }
 struct RateWindow {

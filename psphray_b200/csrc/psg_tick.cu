@@ -37,6 +37,7 @@ PhysParams psg_phys_params(const psg_context *ctx) {
 	P.ar_win = ctx->d_ar_win;
 	P.ar_win_lo = ctx->ar_win_lo;
 	P.ar_win_n = ctx->ar_win_n;
+	P.copy_cycles = ctx->copy_cycles;
 	P.ar_he = ctx->d_ar_he;
 	for (int c = 0; c < PSG_HE_NCOLS; c++) P.ar_he_scale[c] = ctx->ar_he_scale[c];
 	P.ar_step = ctx->ar_step;
@@ -1326,7 +1327,7 @@ __global__ void __launch_bounds__(UPD_THREADS, 1) k_update_queue(int t, const in
 	uint64_t *bar = reinterpret_cast<uint64_t *>(upd_smem + PSG_WIN_ROWS * 5 * 16 + UPD_THREADS);
 	RateWindow rows;
 	rows.start(P, reinterpret_cast<float4 *>(upd_smem), bar);
-	bool rows_here = false;
+	bool rows_here = false, copied = false;
 	const int64_t tick = B->tick0 + t;
 	const double tick_time = B->tick_time;
 	// the tick's particles, or only those listed in alist (the surrogate's rejects)
@@ -1388,12 +1389,12 @@ __global__ void __launch_bounds__(UPD_THREADS, 1) k_update_queue(int t, const in
 		}
 		if (!__any_sync(0xffffffffu, have)) break;
 		if (!rows_here) {
-			rows_here = rate_bar_wait(bar);
-			if (!rows_here) {      // (never seen: fall back on device memory, and say so)
+			copied = rate_bar_wait(bar, P.copy_cycles);
+			if (!copied) {      // (the rows in device memory, and say so)
 				rows.n = 0;
 				st |= PSG_ST_COPY;
-				rows_here = true;
 			}
+			rows_here = true;
 		}
 		if (fresh) dp_start<REC>(P, cx, S, h0, rows);
 		if (have) {
@@ -1421,7 +1422,8 @@ __global__ void __launch_bounds__(UPD_THREADS, 1) k_update_queue(int t, const in
 			}
 		}
 	}
-	if (!rows_here && !rate_bar_wait(bar)) st |= PSG_ST_COPY;      // (no block leaves with its copy in flight)
+	// (a block that did not see its copy end waits for it before it leaves)
+	if (!copied && !rate_bar_wait(bar, PSG_COPY_CYCLES)) st |= PSG_ST_COPY;
 	if (st) atomicOr(status, st);
 }
 
@@ -1706,7 +1708,7 @@ __global__ void __launch_bounds__(Heq<REC>::threads, 1) k_update_he(int t, const
 	uint64_t *bar = reinterpret_cast<uint64_t *>(heq_smem + Heq<REC>::smem - 16);
 	HeWindow rows;
 	rows.start(P, reinterpret_cast<float4 *>(heq_smem + Heq<REC>::slopes), Heq<REC>::rows, bar);
-	bool rows_here = false;
+	bool rows_here = false, copied = false;
 	const int64_t tick = B->tick0 + t;
 	const double tick_time = B->tick_time;
 	const int lo = tick_act[t], n = tick_act[t + 1] - lo;
@@ -1738,7 +1740,8 @@ __global__ void __launch_bounds__(Heq<REC>::threads, 1) k_update_he(int t, const
 		if (!__any_sync(0xffffffffu, have)) break;
 		const bool anyfresh = __any_sync(0xffffffffu, fresh);
 		if (!rows_here) {
-			if (!rate_bar_wait(bar)) {      // (never seen: fall back on device memory, and say so)
+			copied = rate_bar_wait(bar, P.copy_cycles);
+			if (!copied) {      // (the rows in device memory, and say so)
 				rows.n = 0;
 				st |= PSG_ST_COPY;
 			}
@@ -1775,7 +1778,8 @@ __global__ void __launch_bounds__(Heq<REC>::threads, 1) k_update_he(int t, const
 			}
 		}
 	}
-	if (!rows_here && !rate_bar_wait(bar)) st |= PSG_ST_COPY;      // (no block leaves with its copies in flight)
+	// (a block that did not see its copies end waits for them before it leaves)
+	if (!copied && !rate_bar_wait(bar, PSG_COPY_CYCLES)) st |= PSG_ST_COPY;
 	if (st) atomicOr(status, st);
 }
 
@@ -1991,10 +1995,7 @@ static int check_status(psg_context *ctx) {
 	PSG_CUDA(cudaStreamSynchronize(ctx->stream));
 	if (st) {
 		PSG_CUDA(cudaMemsetAsync(ctx->d_status, 0, sizeof(uint32_t), ctx->stream));
-		return psg_fail(ctx, PSG_E_DEVICE, "device status 0x%x:%s%s%s", st,
-				(st & PSG_ST_NAN) ? " non-finite state" : "",
-				(st & PSG_ST_SOLVER) ? " integrator step limit" : "",
-				(st & PSG_ST_IE_NEG) ? " negative internal energy" : "");
+		return psg_status_fail(ctx, st);
 	}
 	return PSG_OK;
 }
@@ -2645,10 +2646,7 @@ int psg_run_ticks_core(psg_context *ctx, const psg_ray *d_rays, size_t R, size_t
 	ctx->host_syncs++;
 	if (stw) {
 		PSG_CUDA(cudaMemsetAsync(ctx->d_status, 0, sizeof(uint32_t), st));
-		return psg_fail(ctx, PSG_E_DEVICE, "device status 0x%x:%s%s%s", stw,
-				(stw & PSG_ST_NAN) ? " non-finite state" : "",
-				(stw & PSG_ST_SOLVER) ? " integrator step limit" : "",
-				(stw & PSG_ST_IE_NEG) ? " negative internal energy" : "");
+		return psg_status_fail(ctx, stw);
 	}
 	const unsigned long long nsat = cnt[1];
 	ctx->sat_frac = tf.nhit ? (double)nsat / (double)tf.nhit : 0.0;
@@ -2786,10 +2784,7 @@ int psg_run_ticks_rec_graph(psg_context *ctx, const psg_ray *d_rays, size_t R, s
 	}
 	if (stw) {
 		PSG_CUDA(cudaMemsetAsync(ctx->d_status, 0, sizeof(uint32_t), st));
-		return psg_fail(ctx, PSG_E_DEVICE, "device status 0x%x:%s%s%s", stw,
-				(stw & PSG_ST_NAN) ? " non-finite state" : "",
-				(stw & PSG_ST_SOLVER) ? " integrator step limit" : "",
-				(stw & PSG_ST_IE_NEG) ? " negative internal energy" : "");
+		return psg_status_fail(ctx, stw);
 	}
 	const unsigned *last = (const unsigned *)&c[11];
 	ctx->rec_last = (size_t)last[0] + last[1] + last[2];
@@ -2990,10 +2985,7 @@ extern "C" int psg_step_evolve_noalloc(psg_context *ctx, psg_step *steps, size_t
 	PSG_CUDA(cudaMemcpyAsync(&status, d_status, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
 	PSG_CUDA(cudaStreamSynchronize(st));
 	if (status)
-		return psg_fail(ctx, PSG_E_DEVICE, "device status 0x%x:%s%s%s", status,
-				(status & PSG_ST_NAN) ? " non-finite state" : "",
-				(status & PSG_ST_SOLVER) ? " integrator step limit" : "",
-				(status & PSG_ST_IE_NEG) ? " negative internal energy" : "");
+		return psg_status_fail(ctx, status);
 	return PSG_OK;
 }
 
