@@ -440,13 +440,21 @@ __device__ __forceinline__ void he_dp_start(HeDp &S, const double k1[4], const d
 
 // One pass over the lanes' next work: for fresh lanes the slope at x first,
 // then for all lanes one attempted step. fresh must be the warp's when other
-// lanes call too: anyfresh says whether any lane's is set.
-template <bool REC, typename ROWS = HeRows>
+// lanes call too: anyfresh says whether any lane's is set. UNROLLED: the
+// stages one after another, so that slopes in an array of the thread's own
+// (stride 1) stay in registers; the same sums.
+template <bool REC, bool UNROLLED = false, typename ROWS = HeRows>
 __device__ __forceinline__ void he_dp_step(const PhysParams &P, const HeCtx &c, HeDp &S, bool fresh, bool anyfresh,
 		double *k, int stride, const ROWS &rows = ROWS()) {
 	double e[4], y[4], q[3], h = 0.0;
-#pragma unroll 1
-	for (int st = anyfresh ? -1 : 0; st < 6; st++) {
+	if (UNROLLED && fresh) {
+		double dx[4], r[3];
+		rhs_he(P, c, S.x, dx, REC ? r : nullptr, rows);
+		he_dp_start<REC>(S, dx, r, k, stride);
+	}
+	constexpr int U = UNROLLED ? 6 : 1;
+#pragma unroll U
+	for (int st = !UNROLLED && anyfresh ? -1 : 0; st < 6; st++) {
 		if (st < 0 && !fresh) continue;
 		if (st <= 0) {
 			if (st == 0) {
@@ -512,7 +520,9 @@ __device__ __forceinline__ void he_dp_step(const PhysParams &P, const HeCtx &c, 
 
 // Up to HE_SWITCH steps from s = 0 on one thread; returns true once s = 1
 // is reached, else leaves the time reached and the next step size in *t_out,
-// *h_out. With rec, rec[3] accumulates the recombination photons.
+// *h_out. With rec, rec[3] accumulates the recombination photons. The slopes
+// stay in registers: psg_step_evolve of 300 records 271 -> 237 us (case A
+// 318 -> 254 us) against the loop over slopes in the thread's stack.
 template <bool REC>
 __device__ inline bool dopri_he_explicit(const PhysParams &P, const HeCtx &c, double x[4], double *rec,
 		double *t_out, double *h_out) {
@@ -522,7 +532,7 @@ __device__ inline bool dopri_he_explicit(const PhysParams &P, const HeCtx &c, do
 	for (int i = 0; i < 4; i++) S.x[i] = x[i];
 	bool fresh = true;
 	do {
-		he_dp_step<REC>(P, c, S, fresh, fresh, k, 1);
+		he_dp_step<REC, true>(P, c, S, fresh, fresh, k, 1);
 		fresh = false;
 	} while (S.t < 1.0 && S.steps < HE_SWITCH);
 #pragma unroll

@@ -1748,7 +1748,7 @@ __global__ void __launch_bounds__(Heq<REC>::threads, 1) k_update_he(int t, const
 			rows_here = true;
 		}
 		if (have) {
-			he_dp_step<REC>(P, cx, S, fresh, anyfresh, k, Heq<REC>::threads, rows);
+			he_dp_step<REC, false>(P, cx, S, fresh, anyfresh, k, Heq<REC>::threads, rows);
 			double rec[3] = {0.0, 0.0, 0.0};
 			if (S.t >= 1.0 || S.steps >= HE_SWITCH) {
 				have = false;
