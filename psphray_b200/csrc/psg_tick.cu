@@ -1678,6 +1678,76 @@ __device__ __forceinline__ HeStep load_he_step(const PhysParams &P, const HeSrc 
 	return s;
 }
 
+// The end of a particle's explicit steps: at s = 1 its new state, else an
+// item for k_update_he_stiff. Returns the status bits raised.
+template <bool REC>
+__device__ __forceinline__ uint32_t he_explicit_end(const PhysParams &P, const HeSrc &src, int a, uint32_t p, HeDp &S,
+		const HeCtx &cx, int64_t tick, double tick_time, double *__restrict__ lambdaH, float *__restrict__ ie,
+		int64_t *__restrict__ lasthit, HeStiffItem *__restrict__ stiff, unsigned *__restrict__ nstiff) {
+	double rec[3] = {0.0, 0.0, 0.0};
+	uint32_t st = 0;
+	if (REC) {
+		rec[0] = (double)P.ygrec[p] + S.gain[0];
+		rec[1] = (double)P.ygrecHe1[p] + S.gain[1];
+		rec[2] = (double)P.ygrecHe2[p] + S.gain[2];
+	}
+	if (S.t >= 1.0) {
+		if (!(S.x[3] >= 0.0)) st |= PSG_ST_IE_NEG;
+		for (int i = 0; i < 4; i++)
+			if (!isfinite(S.x[i])) st |= PSG_ST_NAN;
+		clamp_he(S.x);
+		for (int i = 0; i < 3; i++) rec[i] = fmax(0.0, rec[i]);
+		he_write(P, p, S.x, rec, cx.T, tick, lambdaH, ie, lasthit);
+	} else {
+		double x0[4];
+		HeStiffItem it;
+		it.s = load_he_step(P, src, a, p, tick, tick_time, x0);
+		for (int i = 0; i < 4; i++) it.x[i] = S.x[i];
+		for (int i = 0; i < 3; i++) it.rec[i] = rec[i];
+		it.t = S.t;
+		it.h = S.h;
+		it.p = p;
+		stiff[atomicAdd(nstiff, 1u)] = it;
+	}
+	return st;
+}
+
+// The explicit steps of a tick of up to HE_FEW active particles (k_update_he
+// takes the others; each returns at once from the other's ticks, so a captured
+// tick serves both): a thread per particle, the stages unrolled over slopes in
+// registers. What bounds such a tick is the chain of its longest integrations,
+// which the queue's loop over slopes in shared memory makes longer; past
+// HE_FEW the queue's full warps win. The same sums, so the same bits. Measured,
+// call of 4 ticks, queue -> this: 9261 particles on the spot 1.57 -> 1.09 ms
+// (not on the spot 2.69 -> 2.16), 39e3 1.94 -> 1.44 (3.22 -> 2.71), 125e3 2.43
+// -> 2.00 (3.92 -> 3.55), 262e3 3.12 -> 2.74 (4.86 -> 4.56), 512e3 3.36 -> 3.11
+// (5.14 -> 5.06), 1e6 4.33 -> 4.35 (6.50 -> 6.88), 2.1e6 7.9 -> 8.4 (11.1 -> 12.3).
+#define HE_FEW (1 << 19)
+#define HE_FEW_THREADS 64
+template <bool REC>
+__global__ void __launch_bounds__(HE_FEW_THREADS) k_update_he_few(int t, const int32_t *__restrict__ tick_act,
+		const HeSrc src, double *__restrict__ lambdaH, float *__restrict__ ie, int64_t *__restrict__ lasthit,
+		PhysParams P, const PsgBatchDev *__restrict__ B, HeStiffItem *__restrict__ stiff,
+		unsigned *__restrict__ nstiff, uint32_t *__restrict__ status) {
+	const int lo = tick_act[t], n = tick_act[t + 1] - lo;
+	const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+	if (n > HE_FEW || i >= n) return;
+	const int64_t tick = B->tick0 + t;
+	const double tick_time = B->tick_time;
+	const uint32_t p = src.act_ipar[lo + i];
+	double k[24];
+	HeDp S;
+	const HeCtx cx = make_he_ctx(load_he_step(P, src, lo + i, p, tick, tick_time, S.x));
+	bool fresh = true;
+	do {
+		he_dp_step<REC, true>(P, cx, S, fresh, fresh, k, 1);
+		fresh = false;
+	} while (S.t < 1.0 && S.steps < HE_SWITCH);
+	const uint32_t st = he_explicit_end<REC>(P, src, lo + i, p, S, cx, tick, tick_time, lambdaH, ie, lasthit, stiff,
+			nstiff);
+	if (st) atomicOr(status, st);
+}
+
 // update_pars() with helium: explicit steps, one attempted step per
 // iteration and lane. A lane whose particle is done takes the next one of
 // the tick, so that the warp stays full (particles take 1 to 32 steps, 1.7
@@ -1704,6 +1774,8 @@ __global__ void __launch_bounds__(Heq<REC>::threads, 1) k_update_he(int t, const
 		PhysParams P, const PsgBatchDev *__restrict__ B, unsigned *__restrict__ cursor,
 		HeStiffItem *__restrict__ stiff, unsigned *__restrict__ nstiff, uint32_t *__restrict__ status) {
 	extern __shared__ __align__(16) char heq_smem[];
+	const int lo = tick_act[t], n = tick_act[t + 1] - lo;
+	if (n <= HE_FEW) return;
 	double *k = reinterpret_cast<double *>(heq_smem) + threadIdx.x;
 	uint64_t *bar = reinterpret_cast<uint64_t *>(heq_smem + Heq<REC>::smem - 16);
 	HeWindow rows;
@@ -1711,7 +1783,6 @@ __global__ void __launch_bounds__(Heq<REC>::threads, 1) k_update_he(int t, const
 	bool rows_here = false, copied = false;
 	const int64_t tick = B->tick0 + t;
 	const double tick_time = B->tick_time;
-	const int lo = tick_act[t], n = tick_act[t + 1] - lo;
 	const int lane = threadIdx.x & 31;
 	bool have = false, dry = false;
 	int a = 0;
@@ -1749,32 +1820,9 @@ __global__ void __launch_bounds__(Heq<REC>::threads, 1) k_update_he(int t, const
 		}
 		if (have) {
 			he_dp_step<REC, false>(P, cx, S, fresh, anyfresh, k, Heq<REC>::threads, rows);
-			double rec[3] = {0.0, 0.0, 0.0};
 			if (S.t >= 1.0 || S.steps >= HE_SWITCH) {
 				have = false;
-				if (REC) {
-					rec[0] = (double)P.ygrec[p] + S.gain[0];
-					rec[1] = (double)P.ygrecHe1[p] + S.gain[1];
-					rec[2] = (double)P.ygrecHe2[p] + S.gain[2];
-				}
-				if (S.t >= 1.0) {
-					if (!(S.x[3] >= 0.0)) st |= PSG_ST_IE_NEG;
-					for (int i = 0; i < 4; i++)
-						if (!isfinite(S.x[i])) st |= PSG_ST_NAN;
-					clamp_he(S.x);
-					for (int i = 0; i < 3; i++) rec[i] = fmax(0.0, rec[i]);
-					he_write(P, p, S.x, rec, cx.T, tick, lambdaH, ie, lasthit);
-				} else {
-					double x0[4];
-					HeStiffItem it;
-					it.s = load_he_step(P, src, a, p, tick, tick_time, x0);
-					for (int i = 0; i < 4; i++) it.x[i] = S.x[i];
-					for (int i = 0; i < 3; i++) it.rec[i] = rec[i];
-					it.t = S.t;
-					it.h = S.h;
-					it.p = p;
-					stiff[atomicAdd(nstiff, 1u)] = it;
-				}
+				st |= he_explicit_end<REC>(P, src, a, p, S, cx, tick, tick_time, lambdaH, ie, lasthit, stiff, nstiff);
 			}
 		}
 	}
@@ -2376,13 +2424,21 @@ int enqueue_batch(psg_context *ctx, const BatchPlan &pl, const PsgBatchDev *B) {
 				psg_mark_end(ctx);
 				continue;
 			}
-			if (P.ygrec)
-				k_update_he<true><<<pl.he_grid, Heq<true>::threads, Heq<true>::smem, st>>>((int)t, av.tick_act, hs, ctx->d_lambdaH, ctx->d_ie,
-						ctx->d_lasthit, P, B, uv.cursors + t, hstiff, uv.nstiff + t, ctx->d_status);
-			else
-				k_update_he<false><<<pl.he_grid, Heq<false>::threads, Heq<false>::smem, st>>>((int)t, av.tick_act, hs, ctx->d_lambdaH, ctx->d_ie,
-						ctx->d_lasthit, P, B, uv.cursors + t, hstiff, uv.nstiff + t, ctx->d_status);
+#define PSG_HE(REC_)                                                                                          \
+	do {                                                                                                      \
+		k_update_he_few<REC_><<<blocks(std::min<size_t>(N, HE_FEW), HE_FEW_THREADS), HE_FEW_THREADS, 0, st>>>( \
+				(int)t, av.tick_act, hs, ctx->d_lambdaH, ctx->d_ie, ctx->d_lasthit, P, B, hstiff,             \
+				uv.nstiff + t, ctx->d_status);                                                                \
+		if (N > HE_FEW) /* (a tick's active particles are at most N) */                                      \
+			k_update_he<REC_><<<pl.he_grid, Heq<REC_>::threads, Heq<REC_>::smem, st>>>((int)t, av.tick_act,   \
+					hs, ctx->d_lambdaH, ctx->d_ie, ctx->d_lasthit, P, B, uv.cursors + t, hstiff,              \
+					uv.nstiff + t, ctx->d_status);                                                            \
+	} while (0)
+			if (P.ygrec) PSG_HE(true);
+			else PSG_HE(false);
+#undef PSG_HE
 			PSG_CHECK_LAUNCH();
+			ctx->launches += N > HE_FEW ? 2 : 1;
 			if (P.ygrec)
 				k_update_he_stiff<true><<<pl.stiff_grid, STIFF_THREADS, 0, st>>>(hstiff, uv.nstiff + t, uv.stiff_ctr + t,
 						ctx->d_lambdaH, ctx->d_ie, ctx->d_lasthit, P, B, (int)t, ctx->d_status);
@@ -2390,7 +2446,7 @@ int enqueue_batch(psg_context *ctx, const BatchPlan &pl, const PsgBatchDev *B) {
 				k_update_he_stiff<false><<<pl.stiff_grid, STIFF_THREADS, 0, st>>>(hstiff, uv.nstiff + t, uv.stiff_ctr + t,
 						ctx->d_lambdaH, ctx->d_ie, ctx->d_lasthit, P, B, (int)t, ctx->d_status);
 			PSG_CHECK_LAUNCH();
-			ctx->launches += 2;
+			ctx->launches++;
 		} else {
 			const double *gcarry = pl.euler ? ctx->d_gcarry : nullptr;
 			// not isothermal, every pair's sums first (a thread per short run,
