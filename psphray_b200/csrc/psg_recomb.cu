@@ -343,7 +343,7 @@ int psg_rec_emit_enqueue(psg_context *ctx, const PsgBatchDev *B, psg_ray *out, u
 			k_rec_draw<<<nblocks(kmax, 128), 128, 0, st>>>(n, (int)kmax, s, s == 0 ? 4u : 6u + (uint32_t)s, W.ex + 1,
 					B, ctx->rec_seed, W.leaf_of, items + s * kmax, d_count);
 			PSG_CHECK_LAUNCH();
-			ctx->launches += 5;
+			ctx->launches += 2 + scan_launches(n);
 		}
 		RecItem pad;
 		memset(&pad, 0xff, sizeof(pad));
@@ -359,7 +359,7 @@ int psg_rec_emit_enqueue(psg_context *ctx, const PsgBatchDev *B, psg_ray *out, u
 		PSG_CUDA(scan_enqueue(st, W.flag, n * nspec, W.pos, W.tiles_u, Widen()));
 		k_rec_place<<<nblocks(n * nspec, 256), 256, 0, st>>>(n, nspec, W.flag, W.pos, W.leaf_of, items, d_count);
 		PSG_CHECK_LAUNCH();
-		ctx->launches += 4;
+		ctx->launches += 1 + scan_launches(n * nspec);
 	}
 	const RecItem *sorted = rec_sorted(ctx, ktot, threshold_mode);
 	LteView L;
@@ -464,6 +464,7 @@ int psg_run_ticks_rec(psg_context *ctx, const psg_ray *d_rays, size_t R, size_t 
 		if (ctx->rec_nrec != 0) {      // (no rays at the first tick, loop.c:197: k_rec_draw, k_rec_flag)
 			k_set_batch_rec<<<1, 1, 0, st>>>(ctx->d_batch, tick, tick_time, buf, d_rays, (int64_t)k);
 			PSG_CHECK_LAUNCH();
+			ctx->launches++;
 			const int rc = emit_rec(ctx, ctx->d_batch, cap, buf + R, &M);
 			if (rc) return rc;
 		}

@@ -122,6 +122,10 @@ inline size_t scan_tiles(size_t n) {
 	const size_t t = (n + (size_t)SCAN_T * SCAN_I - 1) / ((size_t)SCAN_T * SCAN_I);
 	return t ? t : 1;
 }
+inline int scan_launches(size_t n) {
+	const size_t t = scan_tiles(n);
+	return t == 1 ? 1 : (t <= SCAN_FEW ? 2 : 3);
+}
 template <typename T, typename Op, typename V>
 cudaError_t scan_enqueue(cudaStream_t st, const T *in, size_t n, V *out, V *tiles, Op op) {
 	const size_t nt = scan_tiles(n);

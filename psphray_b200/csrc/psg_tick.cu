@@ -2328,8 +2328,9 @@ int enqueue_batch(psg_context *ctx, const BatchPlan &pl, const PsgBatchDev *B) {
 	for (uint32_t p0 = 0; p0 < N; p0 += np) {
 		k_slot_place<<<blocks(nray * 32, 256), 256, 0, st>>>(nray, (int)R, N, off64, hit_ipar, kcnt, vals, p0, np);
 		PSG_CHECK_LAUNCH();
+		ctx->launches++;
 	}
-	ctx->launches += 8;
+	ctx->launches += 2 + scan_launches(pl.KN);
 	unsigned long long *d_nsat = ctx->d_counters + 1;      // (zeroed by the caller, per call)
 	psg_mark_end(ctx);
 
@@ -2348,7 +2349,7 @@ int enqueue_batch(psg_context *ctx, const BatchPlan &pl, const PsgBatchDev *B) {
 	PSG_CHECK_LAUNCH();
 	k_tick_rays<<<blocks(K, 128), 128, 0, st>>>((int)K, R, nray, cls, cls_scan, uv.tick_rays);
 	PSG_CHECK_LAUNCH();
-	ctx->launches += 3;
+	ctx->launches += 3 + scan_launches(nray);
 
 	// the long-segment lists and (not isothermal) the integrator's work
 	// cursors, stiff lists and the deposit's unit counters
@@ -2379,14 +2380,16 @@ int enqueue_batch(psg_context *ctx, const BatchPlan &pl, const PsgBatchDev *B) {
 	if (R > SLOT_WARP_MAX) {
 		k_slot_canon_mid<<<(unsigned)(4 * sms), 256, 0, st>>>(ll.mid_list, ll.mid_count, av.act_seg, vals);
 		PSG_CHECK_LAUNCH();
+		ctx->launches++;
 	}
 	if (R > SLOT_MID_MAX) {
 		k_slot_canon_long<<<(unsigned)sms, 1024, sizeof(uint32_t) * std::max(pl.long_cap, 2048), st>>>(ll.vl_list,
 				ll.vl_count, av.act_seg, vals, pl.long_cap, cap);
 		PSG_CHECK_LAUNCH();
+		ctx->launches++;
 	}
 	psg_mark_end(ctx);
-	ctx->launches += 6;
+	ctx->launches += 4;
 
 	// the tick loop
 	double *d_lost = (double *)(ctx->d_counters + 2);
@@ -2489,6 +2492,7 @@ int enqueue_batch(psg_context *ctx, const BatchPlan &pl, const PsgBatchDev *B) {
 					k_log_pre<<<pl.log_grid, 256, 0, st>>>((int)t, av.tick_act, av.act_ipar, uv.act_g, uv.act_heat,
 							ctx->d_lambdaH, ctx->d_ie, ctx->d_lasthit, ctx->d_rho, ctx->d_yeMET, P, B, feat);
 					PSG_CHECK_LAUNCH();
+					ctx->launches++;
 				}
 				if (pl.surr) {
 					// the network first; the integrator takes its rejects
@@ -2518,6 +2522,7 @@ int enqueue_batch(psg_context *ctx, const BatchPlan &pl, const PsgBatchDev *B) {
 					k_log_post<<<pl.log_grid, 256, 0, st>>>((int)t, av.tick_act, av.act_ipar, ctx->d_lambdaH,
 							ctx->d_ie, ctx->d_yeMET, P, feat, ctx->log_buf, ctx->log_cap, ctx->log_count);
 					PSG_CHECK_LAUNCH();
+					ctx->launches++;
 				}
 			}
 		}
@@ -2782,6 +2787,7 @@ int psg_run_ticks_rec_graph(psg_context *ctx, const psg_ray *d_rays, size_t R, s
 	PsgBatchDev *B = ctx->d_batch;
 	k_set_batch<<<1, 1, 0, st>>>(B, first_tick, tick_time, buf, d_rays);
 	PSG_CHECK_LAUNCH();
+	ctx->launches++;
 	unsigned long long *cnt = ctx->d_counters;
 	PSG_CUDA(cudaMemsetAsync(cnt + 1, 0, 3 * sizeof(unsigned long long), st));      // 1-3
 	PSG_CUDA(cudaMemsetAsync(cnt + 6, 0, 2 * sizeof(unsigned long long), st));      // 6, 7
@@ -2803,7 +2809,7 @@ int psg_run_ticks_rec_graph(psg_context *ctx, const psg_ray *d_rays, size_t R, s
 		if (r) return r;
 		k_rec_tick_end<<<1, 1, 0, st>>>(off64, nray, cnt + 7, B);
 		PSG_CHECK_LAUNCH();
-		ctx->launches += 3;
+		ctx->launches += 2;
 		return PSG_OK;
 	};
 	std::vector<unsigned long long> key = batch_key(ctx, pl, B);

@@ -735,7 +735,7 @@ int psg_trace_rec_fill_enqueue(psg_context *ctx, const psg_ray *buf, size_t R, s
 	k_offsets64<<<blocks(nray + 1, 256), 256, 0, st>>>(scan, count, nray, off64, d_max, cap,
 			ctx->d_counters + 24, ctx->d_status);
 	PSG_CHECK_LAUNCH();
-	ctx->launches += 4;
+	ctx->launches += 2 + scan_launches(nray + 1);
 	return PSG_OK;
 }
 
@@ -804,7 +804,7 @@ int psg_trace_fill(psg_context *ctx, const psg_ray *d_rays, size_t nray, PsgTrac
 		k_offsets64<<<blocks(nray + 1, 256), 256, 0, st>>>(scan, count, nray, off64, d_max, 0, nullptr,
 				nullptr);
 		PSG_CHECK_LAUNCH();
-		ctx->launches++;
+		ctx->launches += 1 + scan_launches(nray + 1);
 		PSG_CUDA(cudaMemcpyAsync(hdr, d_max, sizeof(hdr), cudaMemcpyDeviceToHost, st));
 		uint32_t stw = 0;
 		PSG_CUDA(cudaMemcpyAsync(&stw, ctx->d_status, sizeof(stw), cudaMemcpyDeviceToHost, st));
