@@ -154,6 +154,7 @@ struct psg_context {
 	size_t src_nray = 0;         // S_SRCHIT: the call's source rays traced and sorted before its ticks ran
 	size_t src_nhit = 0;         //   (offsets[src_nray + 1], kernel factor[src_nhit], ipar[src_nhit]; src_nhit
 	                             //   a grow-only capacity)
+	size_t src_total = 0;        //   their hits
 
 	// chemistry surrogate (not isothermal): weight blob, residual tolerance
 	void *d_surr = nullptr;

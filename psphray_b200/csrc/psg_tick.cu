@@ -2085,6 +2085,8 @@ struct BatchPlan {
 
 	// grids
 	unsigned dep_grid = 0, red_grid = 0, he_grid = 0, euler_grid = 0, log_grid = 0, stiff_grid = 0;
+	size_t tick_hits = 0;       // hits of a tick on average (0: from the traversal's total)
+	size_t parts = 1;           // launches of the slot placement
 	size_t src_R = 0;           // > 0: a recombination tick whose first src_R rays come traced and sorted (S_SRCHIT)
 };
 
@@ -2212,6 +2214,9 @@ int plan_batch(psg_context *ctx, size_t R, size_t K, const PsgTraceFill &tf, Bat
 		ctx->batch_cap = c;
 	}
 	pl.cap = std::max<size_t>(ctx->batch_cap, 1);
+	// (from this batch's hits: the capacity keeps the largest batch's)
+	if (!pl.tick_hits) pl.tick_hits = tf.nhit / K;
+	pl.parts = std::min<size_t>(sizeof(uint32_t) * pl.tick_hits / SLOT_PART + 1, 16);
 	pl.pcap = std::max<size_t>(std::min(ctx->n, pl.cap), 1);
 	pl.KN = K * ctx->n;
 	if (pl.KN >= (1ull << 31))
@@ -2323,8 +2328,7 @@ int enqueue_batch(psg_context *ctx, const BatchPlan &pl, const PsgBatchDev *B) {
 	k_act_build<<<(unsigned)std::min<size_t>(blocks(pl.KN, 256), (size_t)sms * 16), 256, 0, st>>>(pl.KN, N, (int)K,
 			kbase, av.act_ipar, av.act_seg, av.tick_act, d_nact, kcnt);
 	PSG_CHECK_LAUNCH();
-	const size_t parts = std::min<size_t>(sizeof(uint32_t) * (cap / K) / SLOT_PART + 1, 16);
-	const uint32_t np = (uint32_t)((N + parts - 1) / parts);
+	const uint32_t np = (uint32_t)((N + pl.parts - 1) / pl.parts);
 	for (uint32_t p0 = 0; p0 < N; p0 += np) {
 		k_slot_place<<<blocks(nray * 32, 256), 256, 0, st>>>(nray, (int)R, N, off64, hit_ipar, kcnt, vals, p0, np);
 		PSG_CHECK_LAUNCH();
@@ -2576,6 +2580,7 @@ std::vector<unsigned long long> batch_key(const psg_context *ctx, const BatchPla
 	k.push_back((unsigned long long)ctx->tune.run_short);
 	k.push_back((unsigned long long)ctx->tune.update_order);
 	k.push_back((unsigned long long)psg_sort_classes(pl.maxcount));
+	k.push_back(pl.parts);
 	k.push_back(pl.src_R);
 	k.push_back(ctx->src_nray);
 	k.push_back(ctx->src_nhit);
@@ -2780,6 +2785,7 @@ int psg_run_ticks_rec_graph(psg_context *ctx, const psg_ray *d_rays, size_t R, s
 	PsgTraceFill tf{ctx->batch_cap, ctx->slab_cap, ctx->slab_cap};
 	BatchPlan pl;
 	pl.src_R = R;
+	pl.tick_hits = (size_t)((double)ctx->src_total / K * ((double)nray / R));      // (the emitted rays' as the sources')
 	rc = plan_batch(ctx, nray, 1, tf, pl);
 	if (rc) return rc;
 	rc = psg_state_save(ctx);      // (the undo if a tick outgrows the buffers)

@@ -692,6 +692,7 @@ int psg_trace_src_batch(psg_context *ctx, const psg_ray *d_rays, size_t nray) {
 			ctx->src_nhit);
 	if (!m) return PSG_E_NOMEM;
 	ctx->src_nray = nray;
+	ctx->src_total = tf.nhit;
 	const SrcHits h = src_hits(ctx);
 	cudaStream_t st = ctx->stream;
 	PSG_CUDA(cudaMemcpyAsync((void *)h.off, ctx->scratch[S_OFFSETS].p, sizeof(int64_t) * (nray + 1),

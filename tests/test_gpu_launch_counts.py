@@ -1,4 +1,7 @@
-"""The launches a call reports are the library's kernels it launched."""
+"""The launches a call reports are the library's kernels it launched, and a
+batch's launches follow its own hits: the slots of a tick past L2's size are
+placed in parts (80 MB of slots, 21M hits, to a part), which a small batch on
+the same context does not inherit."""
 import numpy as np
 import pytest
 import torch
@@ -18,6 +21,23 @@ def _kernels(call):
         torch.cuda.synchronize()
     names = [e.name for e in p.events() if e.device_type == torch.autograd.DeviceType.CUDA]
     return r, [n for n in names if not n.startswith(("Memcpy", "Memset"))]
+
+
+def test_parts_follow_the_batch(phys):
+    w = fields.make_workload("iliev32", n_side=19, nray=12000, seed=5)
+    f = w.field
+    f.sml[:] = np.float32(0.9 * f.boxsize)      # every ray hits every particle
+    rays = w.schedule.rays_for_tick(1)
+    ctx = api.Context(0)
+    ctx.set_physics(phys)
+    ctx.load(f)
+    ctx.build_tree(8)
+    for tick, (n, parts) in enumerate(((2500, 1), (12000, 3), (2500, 1), (5000, 2)), 1):
+        st, names = _kernels(lambda: ctx.run_ticks(rays[:n], n, 1, tick, w.tick_time))
+        assert int(4 * st["hits"]) // (80 << 20) + 1 == parts
+        assert sum("k_slot_place" in k for k in names) == parts
+        assert st["launches"] == len(names)
+    ctx.close()
 
 
 @pytest.mark.parametrize("helium,on_the_spot,iso,nray,nticks,nrec", [
