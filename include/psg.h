@@ -233,10 +233,13 @@ int psg_run_ticks_device(psg_context *ctx, const psg_ray *d_rays, size_t nray_pe
  * chosen per device by timing. */
 typedef struct {
 	int trace_warps;        /* warps per traversal block, 1-16 (default 4) */
-	int deposit_long;       /* rays with more hits than this take a 128-thread group (default 96) ... */
-	int deposit_mid;        /* ... more than this a 512-thread block (default 384); fewer take a warp */
-	int update_minblocks;   /* 1 (default), 3 or 4, accepted and kept; the integrator has one register
-	                         * budget (a block per multiprocessor) and runs the same for each */
+	int deposit_long;       /* the deposit scans a ray's hits in steps of 32; of 128 from more hits than
+	                         * this on (default 96) ... */
+	int deposit_mid;        /* ... of 512 from more than this on (default 384). The steps fix the order
+	                         * of the sums. A step is taken by a group of at most its width: a warp, 128
+	                         * or 512 threads, narrower where the tick has many rays */
+	int update_minblocks;   /* 1 (default), 3 or 4: accepted and reported, selects nothing (the
+	                         * integrator has one register budget, a block per multiprocessor) */
 	int leaf_size;          /* particles per octree leaf: the reference's CFG_OCTTREE_PPC, 8; the hit
 	                         * lists are bit-exact only with the reference's leaves, so it is reported,
 	                         * never searched */

@@ -15,7 +15,7 @@
 #define PSG_KEY_OUTSIDE 0xFFFFFFFFFFFFFFFFull
 #define PSG_INVALID_BIT 0x80000000u
 // Longest hit list sorted in shared memory (16 bytes per hit); longer lists
-// take the library segmented sort.
+// are sorted between two global halves (k_sort_long).
 #define PSG_SORT_MAX 8192
 
 #define READ_JOBS 5      // the most arrays of one state call

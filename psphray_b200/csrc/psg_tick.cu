@@ -1289,7 +1289,7 @@ struct UpdSrc {
 
 // A warp claims chunks of 32 particles from the tick's cursor; a lane whose
 // particle is done takes the next one of the chunk, and each iteration is
-// one attempted step of every lane (dp_pass).
+// one attempted step of every lane (dp_step).
 //
 // What bounds it: the latency of a right-hand side (an FP64 chain with a
 // logarithm, a division and a rate row in it) at 16 warps per
@@ -1543,12 +1543,12 @@ __global__ void __launch_bounds__(128) k_update_euler(int t, const int32_t *__re
 	}
 }
 
-// update_pars() loop.c:647-776 with helium: one thread per active particle
-// of the tick sums its deposits (yGdepHI, heat, yGdepHeI, yGdepHeII, in slot
-// order) and integrates the four variables; isothermal, ie follows T at the
-// new ye (loop.c:764-766). A particle still unfinished after the explicit
-// steps goes to k_update_he_stiff (the Rosenbrock finish), which keeps the
-// W-method's registers out of this kernel.
+// update_pars() loop.c:647-776 with helium: k_sum_he sums each active
+// particle's deposits (yGdepHI, heat, yGdepHeI, yGdepHeII, in slot order), then
+// k_update_he_few or k_update_he, by the number of particles, integrates the
+// four variables; isothermal, ie follows T at the new ye (loop.c:764-766). A
+// particle still unfinished after the explicit steps goes to k_update_he_stiff
+// (the Rosenbrock finish), which keeps the W-method's registers out of them.
 struct HeStiffItem {
 	HeStep s;
 	double x[4], rec[3], t, h;
@@ -2931,7 +2931,8 @@ extern "C" int psg_autotune(psg_context *ctx, const psg_ray *d_rays, size_t R, s
 		t.trace_warps = w;
 		rc = consider(t);
 	}
-	// deposit groups: which rays take a warp, a 128-thread group, a block
+	// the deposit's scan steps (32, 128 or 512 hits) by a ray's length, which
+	// also are the least that its groups are narrowed to
 	const int thr[][2] = {{64, 256}, {96, 384}, {128, 512}, {192, 768}, {256, 1024}, {384, 1536}, {512, 2048},
 			{768, 3072}};
 	for (auto &th : thr) {
