@@ -264,11 +264,11 @@ int psg_autotune(psg_context *ctx, const psg_ray *d_rays, size_t R, size_t K, in
 		double tick_time, int reps, psg_tune *out, double *best_ms);
 
 /* How long a block of the integrators waits for its copy of the rate rows
- * into shared memory, in GPU clock cycles (default 4e7, 20 ms; the copy takes
- * microseconds). A block whose wait runs out reads the rows from device
- * memory, with the same results, and the call that ran the ticks returns
- * PSG_E_DEVICE once they are done. 0: every block gives up at once, which
- * shows a host that error. */
+ * into shared memory after its first 1024 attempts, in GPU clock cycles
+ * (default 4e7, 20 ms; the copy takes microseconds). A block whose wait runs
+ * out reads the rows from device memory, with the same results, and the call
+ * that ran the ticks returns PSG_E_DEVICE once they are done. 0: every block
+ * takes the wait as run out, which shows a host that error. */
 int psg_set_copy_limit(psg_context *ctx, long long cycles);
 
 /* ---- recombination rays (psphray.onTheSpot = false) ---------------------- */

@@ -1327,7 +1327,7 @@ __global__ void __launch_bounds__(UPD_THREADS, 1) k_update_queue(int t, const in
 	uint64_t *bar = reinterpret_cast<uint64_t *>(upd_smem + PSG_WIN_ROWS * 5 * 16 + UPD_THREADS);
 	RateWindow rows;
 	rows.start(P, reinterpret_cast<float4 *>(upd_smem), bar);
-	bool rows_here = false, copied = false;
+	bool rows_here = false;
 	const int64_t tick = B->tick0 + t;
 	const double tick_time = B->tick_time;
 	// the tick's particles, or only those listed in alist (the surrogate's rejects)
@@ -1389,8 +1389,7 @@ __global__ void __launch_bounds__(UPD_THREADS, 1) k_update_queue(int t, const in
 		}
 		if (!__any_sync(0xffffffffu, have)) break;
 		if (!rows_here) {
-			copied = rate_bar_wait(bar, P.copy_cycles);
-			if (!copied) {      // (the rows in device memory, and say so)
+			if (!rate_bar_wait(bar, P.copy_cycles)) {      // (the rows in device memory, and say so)
 				rows.n = 0;
 				st |= PSG_ST_COPY;
 			}
@@ -1423,7 +1422,7 @@ __global__ void __launch_bounds__(UPD_THREADS, 1) k_update_queue(int t, const in
 		}
 	}
 	// (a block that did not see its copy end waits for it before it leaves)
-	if (!copied && !rate_bar_wait(bar, PSG_COPY_CYCLES)) st |= PSG_ST_COPY;
+	if ((!rows_here || (st & PSG_ST_COPY)) && !rate_bar_wait(bar, PSG_COPY_CYCLES)) st |= PSG_ST_COPY;
 	if (st) atomicOr(status, st);
 }
 
@@ -1780,7 +1779,7 @@ __global__ void __launch_bounds__(Heq<REC>::threads, 1) k_update_he(int t, const
 	uint64_t *bar = reinterpret_cast<uint64_t *>(heq_smem + Heq<REC>::smem - 16);
 	HeWindow rows;
 	rows.start(P, reinterpret_cast<float4 *>(heq_smem + Heq<REC>::slopes), Heq<REC>::rows, bar);
-	bool rows_here = false, copied = false;
+	bool rows_here = false;
 	const int64_t tick = B->tick0 + t;
 	const double tick_time = B->tick_time;
 	const int lane = threadIdx.x & 31;
@@ -1811,8 +1810,7 @@ __global__ void __launch_bounds__(Heq<REC>::threads, 1) k_update_he(int t, const
 		if (!__any_sync(0xffffffffu, have)) break;
 		const bool anyfresh = __any_sync(0xffffffffu, fresh);
 		if (!rows_here) {
-			copied = rate_bar_wait(bar, P.copy_cycles);
-			if (!copied) {      // (the rows in device memory, and say so)
+			if (!rate_bar_wait(bar, P.copy_cycles)) {      // (the rows in device memory, and say so)
 				rows.n = 0;
 				st |= PSG_ST_COPY;
 			}
@@ -1827,7 +1825,7 @@ __global__ void __launch_bounds__(Heq<REC>::threads, 1) k_update_he(int t, const
 		}
 	}
 	// (a block that did not see its copies end waits for them before it leaves)
-	if (!copied && !rate_bar_wait(bar, PSG_COPY_CYCLES)) st |= PSG_ST_COPY;
+	if ((!rows_here || (st & PSG_ST_COPY)) && !rate_bar_wait(bar, PSG_COPY_CYCLES)) st |= PSG_ST_COPY;
 	if (st) atomicOr(status, st);
 }
 
