@@ -1714,7 +1714,8 @@ __device__ __forceinline__ uint32_t he_explicit_end(const PhysParams &P, const H
 // The explicit steps of a tick of up to HE_FEW active particles (k_update_he
 // takes the others; each returns at once from the other's ticks, so a captured
 // tick serves both): a thread per particle, the stages unrolled over slopes in
-// registers. What bounds such a tick is the chain of its longest integrations,
+// registers; the grid is what fits the machine, a warp that is done takes the
+// next 32 particles. What bounds such a tick is the chain of its longest integrations,
 // which the queue's loop over slopes in shared memory makes longer; past
 // HE_FEW the queue's full warps win. The same sums, so the same bits. Measured,
 // call of 4 ticks, queue -> this: 9261 particles on the spot 1.57 -> 1.09 ms
@@ -1726,24 +1727,34 @@ __device__ __forceinline__ uint32_t he_explicit_end(const PhysParams &P, const H
 template <bool REC>
 __global__ void __launch_bounds__(HE_FEW_THREADS) k_update_he_few(int t, const int32_t *__restrict__ tick_act,
 		const HeSrc src, double *__restrict__ lambdaH, float *__restrict__ ie, int64_t *__restrict__ lasthit,
-		PhysParams P, const PsgBatchDev *__restrict__ B, HeStiffItem *__restrict__ stiff,
+		PhysParams P, const PsgBatchDev *__restrict__ B, unsigned *__restrict__ cursor, HeStiffItem *__restrict__ stiff,
 		unsigned *__restrict__ nstiff, uint32_t *__restrict__ status) {
 	const int lo = tick_act[t], n = tick_act[t + 1] - lo;
-	const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-	if (n > HE_FEW || i >= n) return;
+	const int lane = threadIdx.x & 31, nwarp = (int)(gridDim.x * (HE_FEW_THREADS / 32));
+	int c = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);      // the warp's 32 particles
+	if (n > HE_FEW || 32 * c >= n) return;
 	const int64_t tick = B->tick0 + t;
 	const double tick_time = B->tick_time;
-	const uint32_t p = src.act_ipar[lo + i];
-	double k[24];
-	HeDp S;
-	const HeCtx cx = make_he_ctx(load_he_step(P, src, lo + i, p, tick, tick_time, S.x));
-	bool fresh = true;
+	uint32_t st = 0;
 	do {
-		he_dp_step<REC, true>(P, cx, S, fresh, fresh, k, 1);
-		fresh = false;
-	} while (S.t < 1.0 && S.steps < HE_SWITCH);
-	const uint32_t st = he_explicit_end<REC>(P, src, lo + i, p, S, cx, tick, tick_time, lambdaH, ie, lasthit, stiff,
-			nstiff);
+		const int a = lo + 32 * c + lane;
+		if (a < lo + n) {
+			const uint32_t p = src.act_ipar[a];
+			double k[24];
+			HeDp S;
+			const HeCtx cx = make_he_ctx(load_he_step(P, src, a, p, tick, tick_time, S.x));
+			bool fresh = true;
+			do {
+				he_dp_step<REC, true>(P, cx, S, fresh, fresh, k, 1);
+				fresh = false;
+			} while (S.t < 1.0 && S.steps < HE_SWITCH);
+			st |= he_explicit_end<REC>(P, src, a, p, S, cx, tick, tick_time, lambdaH, ie, lasthit, stiff, nstiff);
+		}
+		__syncwarp();
+		if (32 * nwarp >= n) break;
+		if (lane == 0) c = nwarp + (int)atomicAdd(cursor, 1u);
+		c = __shfl_sync(0xffffffffu, c, 0);
+	} while (32 * c < n);
 	if (st) atomicOr(status, st);
 }
 
@@ -2082,7 +2093,7 @@ struct BatchPlan {
 	bool gen = false, helium = false, iso = false, euler = false, surr = false, aff = false, feat_on = false;
 
 	// grids
-	unsigned dep_grid = 0, red_grid = 0, he_grid = 0, euler_grid = 0, log_grid = 0, stiff_grid = 0;
+	unsigned dep_grid = 0, red_grid = 0, he_grid = 0, he_few_grid = 0, euler_grid = 0, log_grid = 0, stiff_grid = 0;
 	size_t tick_hits = 0;       // hits of a tick on average (0: from the traversal's total)
 	size_t parts = 1;           // launches of the slot placement
 	size_t src_R = 0;           // > 0: a recombination tick whose first src_R rays come traced and sorted (S_SRCHIT)
@@ -2280,6 +2291,9 @@ int plan_batch(psg_context *ctx, size_t R, size_t K, const PsgTraceFill &tf, Bat
 				Heq<true>::smem)
 				: cudaFuncSetAttribute(k_update_he<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
 				Heq<false>::smem));
+	if (!pl.euler && pl.helium)
+		pl.he_few_grid = std::min(blocks(ctx->n, HE_FEW_THREADS), ctx->flags.on_the_spot
+				? occ_grid(ctx, k_update_he_few<false>, HE_FEW_THREADS) : occ_grid(ctx, k_update_he_few<true>, HE_FEW_THREADS));
 	pl.he_grid = pl.euler ? occ_grid(ctx, k_update_he_euler, 128) : (unsigned)ctx->sms;
 	pl.stiff_grid = pl.helium ? (ctx->flags.on_the_spot ? occ_grid(ctx, k_update_he_stiff<false>, STIFF_THREADS)
 			: occ_grid(ctx, k_update_he_stiff<true>, STIFF_THREADS)) : occ_grid(ctx, k_update_stiff<true>, STIFF_THREADS);
@@ -2431,9 +2445,9 @@ int enqueue_batch(psg_context *ctx, const BatchPlan &pl, const PsgBatchDev *B) {
 			}
 #define PSG_HE(REC_)                                                                                          \
 	do {                                                                                                      \
-		k_update_he_few<REC_><<<blocks(std::min<size_t>(N, HE_FEW), HE_FEW_THREADS), HE_FEW_THREADS, 0, st>>>( \
-				(int)t, av.tick_act, hs, ctx->d_lambdaH, ctx->d_ie, ctx->d_lasthit, P, B, hstiff,             \
-				uv.nstiff + t, ctx->d_status);                                                                \
+		k_update_he_few<REC_><<<pl.he_few_grid, HE_FEW_THREADS, 0, st>>>((int)t, av.tick_act, hs,            \
+				ctx->d_lambdaH, ctx->d_ie, ctx->d_lasthit, P, B, uv.cursors + t, hstiff, uv.nstiff + t,       \
+				ctx->d_status);                                                                               \
 		if (N > HE_FEW) /* (a tick's active particles are at most N) */                                      \
 			k_update_he<REC_><<<pl.he_grid, Heq<REC_>::threads, Heq<REC_>::smem, st>>>((int)t, av.tick_act,   \
 					hs, ctx->d_lambdaH, ctx->d_ie, ctx->d_lasthit, P, B, uv.cursors + t, hstiff,              \
