@@ -208,10 +208,12 @@ struct RateRows {
 	}
 };
 // An mbarrier armed for that many bytes, a bulk copy counted on it, and the
-// wait for all of them: false if they did not come within 1024 attempts and then
-// that many clock cycles, and with a limit of none. (Neither the clock nor the
-// limit is read before the first attempt: that cost a launch 1.2 us, the update
-// of 91 thousand particles 90.2 instead of 89.0 us a tick.)
+// wait for all of them: false if they did not come within 1024 attempts and
+// that many clock cycles, and with a limit of none. Whether the limit and the
+// clock are looked at before the first attempt decides how the compiler lays
+// out the loop around it: the hydrogen queue is faster without (91 thousand
+// particles 89.0 against 90.2 us a tick), the helium queue with (2M particles,
+// 4 ticks 7.89 against 7.99 ms).
 __device__ __forceinline__ void rate_bar_arm(uint32_t bar, uint32_t bytes) {
 	asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
 	asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -222,26 +224,30 @@ __device__ __forceinline__ void rate_bar_copy(uint32_t dst, const void *src, uin
 			"r"(bytes), "r"(bar)
 			: "memory");
 }
+__device__ __forceinline__ bool rate_bar_try(uint32_t bar) {
+	uint32_t done;
+	asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n\t"
+				 "selp.u32 %0, 1, 0, p;\n\t}\n"
+				 : "=r"(done)
+				 : "r"(bar)
+				 : "memory");
+	return done != 0;
+}
+template <bool CLOCK_FIRST>
 __device__ __forceinline__ bool rate_bar_wait(uint64_t *bar, long long cycles) {
 	const uint32_t b = (uint32_t)__cvta_generic_to_shared(bar);
-	for (int i = 0; i < 1024; i++) {
-		uint32_t done;
-		asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n\t"
-					 "selp.u32 %0, 1, 0, p;\n\t}\n"
-					 : "=r"(done)
-					 : "r"(b)
-					 : "memory");
-		if (done) return cycles != 0;
+	if (CLOCK_FIRST) {
+		if (!cycles) return false;
+		const long long t0 = clock64();
+		for (int tries = 1;; tries++) {
+			if (rate_bar_try(b)) return true;
+			if (tries >= 1024 && clock64() - t0 >= cycles) return false;
+		}
 	}
-	for (const long long t0 = clock64(); clock64() - t0 < cycles;) {
-		uint32_t done;
-		asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n\t"
-					 "selp.u32 %0, 1, 0, p;\n\t}\n"
-					 : "=r"(done)
-					 : "r"(b)
-					 : "memory");
-		if (done) return true;
-	}
+	for (int i = 0; i < 1024; i++)
+		if (rate_bar_try(b)) return cycles != 0;
+	for (const long long t0 = clock64(); clock64() - t0 < cycles;)
+		if (rate_bar_try(b)) return true;
 	return false;
 }
 struct RateWindow {

@@ -1389,7 +1389,7 @@ __global__ void __launch_bounds__(UPD_THREADS, 1) k_update_queue(int t, const in
 		}
 		if (!__any_sync(0xffffffffu, have)) break;
 		if (!rows_here) {
-			if (!rate_bar_wait(bar, P.copy_cycles)) {      // (the rows in device memory, and say so)
+			if (!rate_bar_wait<false>(bar, P.copy_cycles)) {      // (the rows in device memory, and say so)
 				rows.n = 0;
 				st |= PSG_ST_COPY;
 			}
@@ -1422,7 +1422,7 @@ __global__ void __launch_bounds__(UPD_THREADS, 1) k_update_queue(int t, const in
 		}
 	}
 	// (a block that did not see its copy end waits for it before it leaves)
-	if ((!rows_here || (st & PSG_ST_COPY)) && !rate_bar_wait(bar, PSG_COPY_CYCLES)) st |= PSG_ST_COPY;
+	if ((!rows_here || (st & PSG_ST_COPY)) && !rate_bar_wait<false>(bar, PSG_COPY_CYCLES)) st |= PSG_ST_COPY;
 	if (st) atomicOr(status, st);
 }
 
@@ -1821,7 +1821,7 @@ __global__ void __launch_bounds__(Heq<REC>::threads, 1) k_update_he(int t, const
 		if (!__any_sync(0xffffffffu, have)) break;
 		const bool anyfresh = __any_sync(0xffffffffu, fresh);
 		if (!rows_here) {
-			if (!rate_bar_wait(bar, P.copy_cycles)) {      // (the rows in device memory, and say so)
+			if (!rate_bar_wait<true>(bar, P.copy_cycles)) {      // (the rows in device memory, and say so)
 				rows.n = 0;
 				st |= PSG_ST_COPY;
 			}
@@ -1836,7 +1836,7 @@ __global__ void __launch_bounds__(Heq<REC>::threads, 1) k_update_he(int t, const
 		}
 	}
 	// (a block that did not see its copies end waits for them before it leaves)
-	if ((!rows_here || (st & PSG_ST_COPY)) && !rate_bar_wait(bar, PSG_COPY_CYCLES)) st |= PSG_ST_COPY;
+	if ((!rows_here || (st & PSG_ST_COPY)) && !rate_bar_wait<true>(bar, PSG_COPY_CYCLES)) st |= PSG_ST_COPY;
 	if (st) atomicOr(status, st);
 }
 

@@ -3,7 +3,8 @@ the rate rows that they keep in shared memory (from log T = 3; up to 8 for
 hydrogen, 6.9 with helium) to above the table's end (log T = 9), against
 psg_step_evolve, which reads device memory throughout: the same bits. With
 helium a tick of up to 524,288 active particles takes the integrator without
-these rows, so the field has more, hit by many rays or by few."""
+these rows, so the field has more, hit by many rays, by few (a particle or
+less to each of its threads) or by some (several)."""
 import numpy as np
 import pytest
 
@@ -18,7 +19,8 @@ HE_FEW = 1 << 19
 
 @pytest.mark.parametrize("helium,on_the_spot,side,nray", [
     (False, True, 30, 3000), (False, False, 30, 3000),
-    (True, True, 90, 6000), (True, False, 90, 6000), (True, True, 90, 60), (True, False, 90, 60)])
+    (True, True, 90, 6000), (True, False, 90, 6000), (True, True, 90, 60), (True, False, 90, 60),
+    (True, True, 90, 400), (True, False, 90, 400)])
 def test_all_temperatures(helium, on_the_spot, side, nray):
     units = Units(hmf=0.76 if helium else 1.0)
     f = _field(side, units, 11)
