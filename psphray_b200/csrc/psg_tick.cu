@@ -1295,7 +1295,7 @@ struct UpdSrc {
 // logarithm, a division and a rate row in it) at 16 warps per
 // multiprocessor, and before the rate rows came from shared memory L1's line
 // lookups of them (66% of its peak). So one block fills the multiprocessor,
-// at 104 registers (128 with REC), and copies the rate rows of log T 3 to 8
+// at 108 registers (128 with REC), and copies the rate rows of log T 3 to 8
 // beside it once per launch (RateWindow, 100 KB from L2, one bulk copy that
 // the first particles' gathers overlap); a temperature outside reads device
 // memory. Measured, update group per call, rows from device memory -> from
@@ -1718,10 +1718,11 @@ __device__ __forceinline__ uint32_t he_explicit_end(const PhysParams &P, const H
 // next 32 particles. What bounds such a tick is the chain of its longest integrations,
 // which the queue's loop over slopes in shared memory makes longer; past
 // HE_FEW the queue's full warps win. The same sums, so the same bits. Measured,
-// call of 4 ticks, queue -> this: 9261 particles on the spot 1.57 -> 1.09 ms
-// (not on the spot 2.69 -> 2.16), 39e3 1.94 -> 1.44 (3.22 -> 2.71), 125e3 2.43
-// -> 2.00 (3.92 -> 3.55), 262e3 3.12 -> 2.74 (4.86 -> 4.56), 512e3 3.36 -> 3.11
-// (5.14 -> 5.06), 1e6 4.33 -> 4.35 (6.50 -> 6.88), 2.1e6 7.9 -> 8.4 (11.1 -> 12.3).
+// call of 4 ticks, queue -> this: 9261 particles on the spot 1.60 -> 1.12 ms
+// (not on the spot 2.71 -> 2.22), 91e3 2.27 -> 1.80 (3.66 -> 3.25), 125e3 2.43
+// -> 2.00 (3.94 -> 3.50), 262e3 3.10 -> 2.72 (4.88 -> 4.53), 512e3 3.36 -> 3.06
+// (5.16 -> 4.96); with a thread for each particle of the launch 1e6 took 4.33 ->
+// 4.35 (6.50 -> 6.88), 2.1e6 7.9 -> 8.4 (11.1 -> 12.3).
 #define HE_FEW (1 << 19)
 #define HE_FEW_THREADS 64
 template <bool REC>
